@@ -255,58 +255,287 @@ __global__ void __launch_bounds__(512)
     }
 }
 
-// weight and bias gradients, stage 1: per chunk of voxels, per output channel o,
-// partial[chunk][o][c][t] = sum_v gy[o][v] * u[c][v + t]; partial bias in slot
-// [chunk][o][cin * 27].  blockIdx.x = chunk, blockIdx.y = o, blockIdx.z = sample.
-constexpr int kChunk = 2048;
-__global__ void k_conv_wgrad_partial(const float *__restrict__ in, const float *__restrict__ gy,
-                                     float *__restrict__ partial, ConvGeom g, size_t in_stride, size_t g_stride,
-                                     int nchunks) {
-    __shared__ float gs[kChunk];
-    const size_t nv = (size_t)g.X * g.Y * g.Z;
-    const int o     = blockIdx.y;
-    const size_t v0 = (size_t)blockIdx.x * kChunk;
-    const int cnt   = (int)min((size_t)kChunk, nv - v0);
-    const float *gyo = gy + blockIdx.z * g_stride + (size_t)o * nv + v0;
-    for (int e = threadIdx.x; e < cnt; e += blockDim.x)
-        gs[e] = gyo[e];
-    __syncthreads();
-    const float *inb = in + blockIdx.z * in_stride;
-    const int nk     = g.cin * 27 + 1;
-    float *dst = partial + (((size_t)blockIdx.z * nchunks + blockIdx.x) * g.cout + o) * nk;
-    for (int k = threadIdx.x; k < nk; k += blockDim.x) {
-        float acc = 0.f;
-        if (k == nk - 1) {
-            for (int e = 0; e < cnt; ++e)
-                acc += gs[e];
-        } else {
-            const int c = k / 27, t = k % 27;
-            const int dx = t / 9 - 1, dy = (t / 3) % 3 - 1, dz = t % 3 - 1;
-            for (int e = 0; e < cnt; ++e) {
-                const size_t v = v0 + e;
-                const int z = (int)(v % g.Z), y = (int)((v / g.Z) % g.Y), x = (int)(v / ((size_t)g.Z * g.Y));
-                acc = fmaf(gs[e], conv_in(inb, g, c, x + dx, y + dy, z + dz), acc);
+// Weight and bias gradients of an upsampling convolution, folded taps.
+//
+// Of the 27 fine taps an output voxel reads, the nearest upsampling makes
+// several read the same coarse voxel: per axis an output of parity p sees two
+// coarse voxels (p = 0: v-1, v; p = 1: v, v+1), so the gradient is gathered for
+// the 4 x 4 x 4 products of (parity, coarse tap) pairs,
+//   dK[o][c][kx ky kz] = sum_v gy[o][2v + p] u[c][v + p - 1 + t],
+// k = 3, 1 (p = 0, t = 0, 1) and 2, 0 (p = 1, t = 0, 1), and the 27 tap
+// gradients are sums of 8 of them (k_up_wgrad_reduce): 8 multiply-adds per fine
+// voxel and channel pair instead of 27.
+//
+// Bound by FP32 issue (FMA pipe) in the inner loop.  A CTA takes 8 input
+// channels x OT output channels (blockIdx.y) and strides over tiles of at most
+// 128 coarse voxels.  A warp holds one (x, y) parity (warp & 3) and its lanes 8
+// input channels x the 4 (x, y) taps, so gy comes as warp-uniform 16-byte loads
+// and a new u as one load per z step: 32 multiply-adds per 5 shared-memory
+// wavefronts, with the 4 x OT sums in registers.  The pitches put the 32 lanes'
+// u values in 32 banks.  Two halves of the warps split a tile's rows and are
+// added in shared memory at the end.
+//   8 -> 8 channels at 128 x 128 x 32, 8 samples: 30.8 ms -> see k_up_wgrad_reduce
+constexpr int kWgVox = 128; // coarse voxels per tile, at most
+
+struct WgTile {
+    int tx, ty, tz;        // tile edges (coarse voxels)
+    int ys, xs, cs;        // u pitches: row, x plane, channel
+    int nx, ny, nz, ntile; // tiles per axis, tiles over all samples
+    int ncg;               // groups of 8 input channels
+};
+
+// position of the (parity, coarse tap) pair among the four folded taps of an axis
+__device__ __forceinline__ int fold_k(int p, int t) { return p == 0 ? (t == 0 ? 3 : 1) : (t == 0 ? 2 : 0); }
+
+template <int OT>
+__global__ void __launch_bounds__(256)
+    k_up_wgrad(const float *__restrict__ in, const float *__restrict__ gy, float *__restrict__ partial,
+               float *__restrict__ bpartial, ConvGeom g, WgTile w, size_t in_stride, size_t g_stride) {
+    extern __shared__ __align__(16) float wg_smem[];
+    float *us = wg_smem;                                   // 8 channels of u with halo
+    const int un = (8 * w.cs + 3) & ~3;
+    float *gs = wg_smem + un;                              // [pxy][voxel][pz][OT]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cg = blockIdx.y % w.ncg, og = blockIdx.y / w.ncg;
+    const int c0 = cg * 8, o0 = og * OT;
+    const int Xi = g.X >> 1, Yi = g.Y >> 1, Zi = g.Z >> 1;
+    const int nvox = w.tx * w.ty * w.tz;
+    const int pxy = warp & 3, half = warp >> 2, px = pxy >> 1, py = pxy & 1;
+    const int cl = lane & 7, tx = lane >> 4, ty = (lane >> 3) & 1;
+    float acc[4][OT]; // (pz, tz), output channel
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int o = 0; o < OT; ++o)
+            acc[k][o] = 0.f;
+    float bsum = 0.f; // of this thread's staged gy (channel lane % OT)
+    for (int tile = blockIdx.x; tile < w.ntile; tile += gridDim.x) {
+        int r         = tile;
+        const int bz = r % w.nz;
+        r /= w.nz;
+        const int by = r % w.ny;
+        r /= w.ny;
+        const int bx = r % w.nx, smp = r / w.nx;
+        const int x0 = bx * w.tx, y0 = by * w.ty, z0 = bz * w.tz;
+        const float *inb = in + smp * in_stride, *gyb = gy + smp * g_stride;
+        __syncthreads(); // the previous tile's reads
+        // u: one row of z per warp and step
+        const int hy = w.ty + 2, hx = w.tx + 2;
+        for (int row = warp; row < 8 * hx * hy; row += 8) {
+            const int c = row / (hx * hy), q = row - c * hx * hy, xl = q / hy, yl = q - xl * hy;
+            const int x = x0 + xl - 1, y = y0 + yl - 1;
+            const bool ok = c0 + c < g.cin && x >= 0 && x < Xi && y >= 0 && y < Yi;
+            const float *src = inb + ((size_t)(c0 + c) * Xi + x) * Yi * Zi + (size_t)y * Zi;
+            for (int zl = lane; zl < w.tz + 2; zl += 32) {
+                const int z = z0 + zl - 1;
+                us[c * w.cs + xl * w.xs + yl * w.ys + zl] = ok && z >= 0 && z < Zi ? __ldg(&src[z]) : 0.f;
             }
         }
-        dst[k] = acc;
+        // gy: lanes take the output channels first (conflict-free stores)
+        for (int row = warp; row < 4 * w.tx * w.ty; row += 8) {
+            const int p = row & 3, q = row >> 2, xl = q / w.ty, yl = q - xl * w.ty;
+            const int x = 2 * (x0 + xl) + (p >> 1), y = 2 * (y0 + yl) + (p & 1);
+            const bool ok = x < g.X && y < g.Y;
+            const float *src = gyb + ((size_t)(o0 + lane % OT) * g.X + x) * g.Y * g.Z + (size_t)y * g.Z + 2 * z0;
+            float *dst = gs + (size_t)(p * nvox + q * w.tz) * 2 * OT;
+            for (int fz = lane / OT; fz < 2 * w.tz; fz += 32 / OT) {
+                const float v = ok && 2 * z0 + fz < g.Z ? __ldg(&src[fz]) : 0.f;
+                dst[fz * OT + lane % OT] = v;
+                bsum += v;
+            }
+        }
+        __syncthreads();
+        for (int row = half; row < w.tx * w.ty; row += 2) {
+            const int xl = row / w.ty, yl = row - xl * w.ty;
+            const float *u = us + cl * w.cs + (xl + px + tx) * w.xs + (yl + py + ty) * w.ys;
+            const float *gr = gs + (size_t)(pxy * nvox + row * w.tz) * 2 * OT;
+            float u0 = u[0], u1 = u[1];
+#pragma unroll 4
+            for (int z = 0; z < w.tz; ++z) {
+                const float u2 = u[z + 2];
+                alignas(16) float ga[2 * OT];
+                if constexpr (OT % 2 == 0) {
+#pragma unroll
+                    for (int k = 0; k < 2 * OT; k += 4)
+                        *reinterpret_cast<float4 *>(ga + k) = *reinterpret_cast<const float4 *>(gr + z * 2 * OT + k);
+                } else {
+                    ga[0] = gr[z * 2], ga[1] = gr[z * 2 + 1];
+                }
+#pragma unroll
+                for (int o = 0; o < OT; ++o) {
+                    acc[0][o] = fmaf(ga[o], u0, acc[0][o]);
+                    acc[1][o] = fmaf(ga[o], u1, acc[1][o]);
+                    acc[2][o] = fmaf(ga[OT + o], u1, acc[2][o]);
+                    acc[3][o] = fmaf(ga[OT + o], u2, acc[3][o]);
+                }
+                u0 = u1;
+                u1 = u2;
+            }
+        }
+    }
+    // the two halves, then this CTA's part: [c][kx ky][kz][o]
+    __syncthreads();
+    if (half == 1)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int o = 0; o < OT; ++o)
+                gs[(k * OT + o) * 128 + (tid & 127)] = acc[k][o];
+    __syncthreads();
+    float *dst = partial + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * (8 * 64 * OT);
+    if (half == 0) {
+        const int kxy = fold_k(px, tx) * 4 + fold_k(py, ty);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+            for (int o = 0; o < OT; ++o)
+                dst[(cl * 64 + kxy * 4 + fold_k(k >> 1, k & 1)) * OT + o] = acc[k][o] + gs[(k * OT + o) * 128 + tid];
+    }
+    if (cg == 0) {
+        __syncthreads();
+        gs[tid] = bsum;
+        __syncthreads();
+        if (tid < OT) {
+            float s = 0.f;
+            for (int t = tid; t < 256; t += OT)
+                s += gs[t];
+            bpartial[(size_t)blockIdx.x * g.cout + o0 + tid] = s;
+        }
     }
 }
 
-// stage 2: dW[o][c][t] = sum over samples and chunks (fixed order); db[o] likewise
-__global__ void k_conv_wgrad_reduce(const float *__restrict__ partial, float *__restrict__ dW,
-                                    float *__restrict__ db, int cout, int cin, int nparts) {
-    const int nk = cin * 27 + 1;
-    const int e  = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= cout * nk)
+// Sums the CTAs' parts of one input channel (blockIdx.x) and output-channel
+// group (blockIdx.y), then unfolds the 64 products into the 27 tap gradients:
+// tap -1 of an axis collects k = 2, 3, tap 0 k = 1, 2, tap 1 k = 0, 1.
+// 64 x OT threads per slice of the parts, 1024 / (64 OT) slices (at most 4).
+template <int OT> constexpr int up_reduce_slices() { return 1024 / (64 * OT) > 4 ? 4 : 1024 / (64 * OT); }
+template <int OT>
+__global__ void __launch_bounds__(64 * OT * up_reduce_slices<OT>())
+    k_up_wgrad_reduce(const float *__restrict__ partial, const float *__restrict__ bpartial, float *__restrict__ dW,
+                      float *__restrict__ db, int cout, int cin, int ncg, int nparts) {
+    constexpr int SL = up_reduce_slices<OT>();
+    __shared__ float red[SL][64 * OT];
+    const int c = blockIdx.x, og = blockIdx.y, tid = threadIdx.x;
+    const int sl = tid / (64 * OT), e = tid % (64 * OT);
+    const int pair      = og * ncg + c / 8, npair = gridDim.y * ncg;
+    const float *src    = partial + (size_t)pair * (8 * 64 * OT) + (c % 8) * 64 * OT + e;
+    const size_t stride = (size_t)npair * (8 * 64 * OT);
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    int p      = sl;
+    for (; p + 3 * SL < nparts; p += 4 * SL)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            s[k] += src[(size_t)(p + k * SL) * stride];
+    for (; p < nparts; p += SL)
+        s[0] += src[(size_t)p * stride];
+    red[sl][e] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    for (int q = tid; q < 27 * OT; q += blockDim.x) {
+        const int o = q % OT, t = q / OT;
+        float v = 0.f;
+#pragma unroll
+        for (int m = 0; m < 8; ++m) {
+            const int k = ((2 - t / 9 + (m >> 2)) * 4 + (2 - (t / 3) % 3 + ((m >> 1) & 1))) * 4 + (2 - t % 3 + (m & 1));
+#pragma unroll
+            for (int l = 0; l < SL; ++l)
+                v += red[l][k * OT + o];
+        }
+        dW[((size_t)(og * OT + o) * cin + c) * 27 + t] = v;
+    }
+    if (c == 0 && tid < 32)
+        for (int o = 0; o < OT; ++o) {
+            float b = 0.f;
+            for (int q = tid; q < nparts; q += 32)
+                b += bpartial[(size_t)q * cout + og * OT + o];
+            for (int off = 16; off > 0; off >>= 1)
+                b += __shfl_down_sync(0xffffffffu, b, off);
+            if (tid == 0)
+                db[og * OT + o] = b;
+        }
+}
+
+// Weight and bias gradients of the last convolution (cin -> 1, no upsampling).
+// Lanes take neighbouring (y, z) columns and walk along x over a segment of sx
+// planes, holding the 3 x 9 window of one input channel (blockIdx.y) and the 27
+// sums in registers: 9 loads (L1) and 27 multiply-adds per voxel.  The block's
+// sums meet in shared memory.  blockIdx.x = column block x segment, z = sample.
+__global__ void __launch_bounds__(256)
+    k_last_wgrad(const float *__restrict__ in, const float *__restrict__ gy, float *__restrict__ partial,
+                 ConvGeom g, int sx, int nseg, size_t in_stride, size_t g_stride) {
+    __shared__ float red[28][257];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int cols = g.Y * g.Z;
+    const int cb = blockIdx.x / nseg, seg = blockIdx.x - cb * nseg;
+    const int col = cb * 256 + tid, y = col / g.Z, z = col - y * g.Z;
+    const float *u   = in + blockIdx.z * in_stride + (size_t)blockIdx.y * g.X * cols;
+    const float *gyb = gy + blockIdx.z * g_stride;
+    const int x0 = seg * sx, x1 = min(x0 + sx, g.X);
+    float acc[3][9], w[3][9], gsum = 0.f;
+    bool ok[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int yy = y + k / 3 - 1, zz = z + k % 3 - 1;
+        ok[k] = col < cols && yy >= 0 && yy < g.Y && zz >= 0 && zz < g.Z;
+        acc[0][k] = acc[1][k] = acc[2][k] = 0.f;
+        const int off = (k / 3 - 1) * g.Z + k % 3 - 1;
+        w[0][k] = ok[k] && x0 > 0 ? __ldg(&u[(size_t)(x0 - 1) * cols + col + off]) : 0.f;
+        w[1][k] = ok[k] && x0 < g.X ? __ldg(&u[(size_t)x0 * cols + col + off]) : 0.f;
+    }
+    // sx is a multiple of 3: the window's planes rotate by renaming
+#pragma unroll 1
+    for (int xb = x0; xb < x1; xb += 3) {
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+            const int x = xb + s;
+            const float gv = col < cols && x < x1 ? __ldg(&gyb[(size_t)x * cols + col]) : 0.f;
+            gsum += gv;
+#pragma unroll
+            for (int k = 0; k < 9; ++k) {
+                const int off = (k / 3 - 1) * g.Z + k % 3 - 1;
+                w[(s + 2) % 3][k] = ok[k] && x + 1 < g.X ? __ldg(&u[(size_t)(x + 1) * cols + col + off]) : 0.f;
+#pragma unroll
+                for (int d = 0; d < 3; ++d)
+                    acc[d][k] = fmaf(gv, w[(s + d) % 3][k], acc[d][k]);
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < 27; ++t)
+        red[t][tid] = acc[t / 9][t % 9];
+    red[27][tid] = gsum;
+    __syncthreads();
+    float *dst = partial + (((size_t)blockIdx.z * gridDim.x + blockIdx.x) * g.cin + blockIdx.y) * 28;
+    for (int t = warp; t < 28; t += 8) {
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            v += red[t][lane + 32 * k];
+        for (int off = 16; off > 0; off >>= 1)
+            v += __shfl_down_sync(0xffffffffu, v, off);
+        if (lane == 0)
+            dst[t] = v;
+    }
+}
+
+// dW[c][t] and db of the last convolution: one warp per (c, t), lanes over the parts
+__global__ void __launch_bounds__(256)
+    k_last_wgrad_reduce(const float *__restrict__ partial, float *__restrict__ dW, float *__restrict__ db, int cin,
+                        int nparts) {
+    const int lane = threadIdx.x & 31, e = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (e >= cin * 28)
         return;
-    const int o = e / nk, k = e % nk;
-    float acc = 0.f;
-    for (int p = 0; p < nparts; ++p)
-        acc += partial[((size_t)p * cout + o) * nk + k];
-    if (k == nk - 1)
-        db[o] = acc;
-    else
-        dW[(size_t)o * cin * 27 + k] = acc;
+    const int c = e / 28, t = e - c * 28;
+    float v = 0.f;
+    for (int p = lane; p < nparts; p += 32)
+        v += partial[(size_t)p * cin * 28 + e];
+    for (int off = 16; off > 0; off >>= 1)
+        v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) {
+        if (t < 27)
+            dW[c * 27 + t] = v;
+        else if (c == 0)
+            db[0] = v;
+    }
 }
 
 // input gradient: dU[c][v] = sum_o sum_t W[o][c][t] gy[o][v - t] on the fine
@@ -402,6 +631,15 @@ int grid_for(size_t n, int bs = 256) { return (int)std::min<size_t>((n + bs - 1)
 // channel counts the kernels are compiled for
 bool channels_ok(int c) { return c == 1 || c == 2 || c == 4 || c == 8 || c == 16 || c == 32; }
 
+// output channels per thread of the folded kernels (channel counts are powers of two)
+template <class F> void by_ot(int ot, F &&f) {
+    switch (ot) {
+    case 1: f(std::integral_constant<int, 1>{}); break;
+    case 2: f(std::integral_constant<int, 2>{}); break;
+    case 4: f(std::integral_constant<int, 4>{}); break;
+    default: f(std::integral_constant<int, 8>{}); break;
+    }
+}
 template <class F> void by_channels(int c, F &&f) {
     switch (c) {
     case 1: f(std::integral_constant<int, 1>{}); break;
@@ -528,6 +766,78 @@ void forward(gpe_warm *W, int B) {
     WS_CUDA(cudaGetLastError());
 }
 
+// tile of the folded weight gradient for a coarse volume, and its shared memory
+gpe::WgTile wg_tile(const gpe_warm::Layer &L, int B) {
+    gpe::WgTile w{};
+    const int Xi = L.g.X / 2, Yi = L.g.Y / 2, Zi = L.g.Z / 2;
+    auto pow2 = [](int n, int most) {
+        int p = 1;
+        while (2 * p <= most && p < n)
+            p *= 2;
+        return p;
+    };
+    w.tz = pow2(Zi, 16);
+    w.ty = pow2(Yi, std::min(gpe::kWgVox / w.tz, 4));
+    w.tx = pow2(Xi, gpe::kWgVox / (w.tz * w.ty));
+    auto up = [](int v, int rem, int mod) { // smallest value >= v that is rem modulo mod
+        return v + ((rem - v) % mod + mod) % mod;
+    };
+    w.ys = up(w.tz + 2, 8, 16);
+    w.xs = up((w.ty + 2) * w.ys, 16, 32);
+    w.cs = up((w.tx + 2) * w.xs, 1, 32);
+    w.nx = (Xi + w.tx - 1) / w.tx;
+    w.ny = (Yi + w.ty - 1) / w.ty;
+    w.nz = (Zi + w.tz - 1) / w.tz;
+    w.ntile = w.nx * w.ny * w.nz * B;
+    w.ncg   = (L.cin + 7) / 8;
+    return w;
+}
+size_t wg_smem(const gpe::WgTile &w, int ot) {
+    const size_t gs = (size_t)8 * w.tx * w.ty * w.tz * ot;
+    return sizeof(float) * (((size_t)8 * w.cs + 3) / 4 * 4 + std::max<size_t>(gs, (size_t)512 * ot));
+}
+int wg_ot(const gpe_warm::Layer &L) { return std::min(L.cout, 8); }
+// CTAs along the tiles: up to four per SM over all channel groups
+int wg_parts(const gpe::WgTile &w, int pairs) { return std::min(w.ntile, std::max(1, 148 * 4 / pairs)); }
+// planes per segment of the last layer's gradient (a multiple of 3) and segments
+int last_segments(const gpe_warm::Layer &L) { return (L.g.X + 32) / 33; }
+int last_segment(const gpe_warm::Layer &L) {
+    const int n = last_segments(L);
+    return ((L.g.X + n - 1) / n + 2) / 3 * 3;
+}
+// floats of partial sums that layer l's weight gradient needs
+size_t wg_partial(const gpe_warm::Layer &L, int B) {
+    if (!L.g.up)
+        return (size_t)B * last_segments(L) * (((size_t)L.g.Y * L.g.Z + 255) / 256) * L.cin * 28;
+    const gpe::WgTile w = wg_tile(L, B);
+    const int ot = wg_ot(L), pairs = w.ncg * (L.cout / ot);
+    return (size_t)wg_parts(w, pairs) * ((size_t)pairs * 512 * ot + L.cout);
+}
+
+// weight and bias gradients of layer l from its input and dL/d(pre-activation)
+void conv_wgrad(gpe_warm *W, int l, int B, const float *in, size_t in_stride, const float *gy, size_t g_stride) {
+    const auto &L  = W->conv[l];
+    cudaStream_t s = W->stream;
+    if (!L.g.up) {
+        const int nseg = last_segments(L), nb = (L.g.Y * L.g.Z + 255) / 256 * nseg;
+        gpe::k_last_wgrad<<<dim3(nb, L.cin, B), 256, 0, s>>>(in, gy, W->partial.p, L.g, last_segment(L), nseg,
+                                                             in_stride, g_stride);
+        gpe::k_last_wgrad_reduce<<<(L.cin * 28 + 7) / 8, 256, 0, s>>>(W->partial.p, W->grad.p + L.w,
+                                                                      W->grad.p + L.b, L.cin, nb * B);
+        return;
+    }
+    const gpe::WgTile w = wg_tile(L, B);
+    gpe::by_ot(wg_ot(L), [&](auto O) {
+        constexpr int OT = decltype(O)::value;
+        const int nog = L.cout / OT, pairs = w.ncg * nog, parts = wg_parts(w, pairs);
+        float *bp = W->partial.p + (size_t)parts * pairs * 512 * OT;
+        gpe::k_up_wgrad<OT><<<dim3(parts, pairs), 256, wg_smem(w, OT), s>>>(in, gy, W->partial.p, bp, L.g, w,
+                                                                            in_stride, g_stride);
+        gpe::k_up_wgrad_reduce<OT><<<dim3(L.cin, nog), 64 * OT * gpe::up_reduce_slices<OT>(), 0, s>>>(
+            W->partial.p, bp, W->grad.p + L.w, W->grad.p + L.b, L.cout, L.cin, w.ncg, parts);
+    });
+}
+
 // gradients of the mean squared amplitude error against `targets` (device,
 // B x N floats); returns the loss (host)
 double backward(gpe_warm *W, int B, const float *targets) {
@@ -548,12 +858,7 @@ double backward(gpe_warm *W, int B, const float *targets) {
             k_silu_back<<<gpe::grid_for((size_t)B * n), 256, 0, s>>>(gy, W->pre[l].p, (size_t)B * n);
         const float *in  = l == 0 ? W->h2.p : W->act[l - 1].p;
         const size_t ins = l == 0 ? (size_t)W->latent : W->vox(l - 1) * W->conv[l - 1].cout;
-        const int nchunks = (int)((W->vox(l) + kChunk - 1) / kChunk);
-        k_conv_wgrad_partial<<<dim3(nchunks, L.cout, B), 256, 0, s>>>(in, gy, W->partial.p, L.g, ins, n, nchunks);
-        const int nk = L.cin * 27 + 1;
-        k_conv_wgrad_reduce<<<(L.cout * nk + 255) / 256, 256, 0, s>>>(W->partial.p, W->grad.p + L.w,
-                                                                       W->grad.p + L.b, L.cout, L.cin,
-                                                                       nchunks * B);
+        conv_wgrad(W, l, B, in, ins, gy, n);
         float *dx = l == 0 ? W->gh2.p : W->gact[l - 1].p;
         const size_t ni = l == 0 ? (size_t)W->latent / L.cin : W->vox(l - 1);
         const size_t sm = sizeof(float) * L.cin * L.cout * 27;
@@ -655,8 +960,7 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
             W->pre[l].alloc(n);
             W->act[l].alloc(n);
             W->gact[l].alloc(n);
-            const size_t nch = (W->vox((int)l) + gpe::kChunk - 1) / gpe::kChunk;
-            maxpart = std::max(maxpart, nch * B * W->conv[l].cout * (W->conv[l].cin * 27 + 1));
+            maxpart = std::max(maxpart, wg_partial(W->conv[l], B));
         }
         W->partial.alloc(maxpart);
         W->lpart.alloc(148 * 4);
@@ -668,6 +972,11 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
                 WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_conv_xgrad<decltype(C)::value>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
+            });
+        for (int ot : {1, 2, 4, 8})
+            gpe::by_ot(ot, [&](auto O) {
+                WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_up_wgrad<decltype(O)::value>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
             });
         *out = W.release();
     });
