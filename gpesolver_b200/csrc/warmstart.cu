@@ -86,12 +86,6 @@ __global__ void k_dense_fwd(const float *__restrict__ X, const __nv_bfloat16 *__
     Y[(size_t)b * O + o]    = silu(acc);
 }
 
-// G[b][o] = dL/dY[b][o] * silu'(Ypre)  (in place)
-__global__ void k_silu_back(float *__restrict__ G, const float *__restrict__ Ypre, size_t n) {
-    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
-        G[e] *= silu_grad(Ypre[e]);
-}
-
 // dW[o][i] = sum_b G[b][o] X[b][i];  db[o] = sum_b G[b][o]
 __global__ void k_dense_wgrad(const float *__restrict__ G, const float *__restrict__ X, float *__restrict__ dW,
                               float *__restrict__ db, int B, int I, int O) {
@@ -111,17 +105,46 @@ __global__ void k_dense_wgrad(const float *__restrict__ G, const float *__restri
     }
 }
 
-// dX[b][i] = sum_o W[o][i] G[b][o]
-__global__ void k_dense_xgrad(const float *__restrict__ G, const __nv_bfloat16 *__restrict__ W,
-                              float *__restrict__ dX, int B, int I, int O) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y;
-    if (i >= I || b >= B)
+// dX[b][i] = sum_o W[o][i] G[b][o], times SiLU'(pre[b][i]): the rows o in chunks
+// (blockIdx.y), eight samples at a time, coalesced along i; then the chunks'
+// sums.  (One thread per (b, i) over all rows: 381 us at 4096 x 256, 8 samples,
+// 16 CTAs with one serial chain each.)
+constexpr int kXgRows = 32;
+__global__ void __launch_bounds__(128)
+    k_dense_xgrad_part(const float *__restrict__ G, const __nv_bfloat16 *__restrict__ W, float *__restrict__ part,
+                       int B, int I, int O) {
+    const int i = blockIdx.x * 128 + threadIdx.x;
+    if (i >= I)
         return;
-    float acc = 0.f;
-    for (int o = 0; o < O; ++o)
-        acc = fmaf(__bfloat162float(W[(size_t)o * I + i]), G[(size_t)b * O + o], acc);
-    dX[(size_t)b * I + i] = acc;
+    const int o0 = blockIdx.y * kXgRows, o1 = min(o0 + kXgRows, O);
+    for (int b0 = 0; b0 < B; b0 += 8) {
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int o = o0; o < o1; ++o) {
+            const float w = __bfloat162float(W[(size_t)o * I + i]);
+#pragma unroll
+            for (int b = 0; b < 8; ++b)
+                if (b0 + b < B)
+                    acc[b] = fmaf(w, __ldg(&G[(size_t)(b0 + b) * O + o]), acc[b]);
+        }
+        for (int b = 0; b < 8 && b0 + b < B; ++b)
+            part[((size_t)blockIdx.y * B + b0 + b) * I + i] = acc[b];
+    }
+}
+__global__ void k_dense_xgrad_sum(const float *__restrict__ part, const float *__restrict__ pre,
+                                  float *__restrict__ dX, int n, int nparts) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= n)
+        return;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    int p      = 0;
+    for (; p + 3 < nparts; p += 4)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            s[k] += part[(size_t)(p + k) * n + e];
+    for (; p < nparts; ++p)
+        s[0] += part[(size_t)p * n + e];
+    dX[e] = ((s[0] + s[1]) + (s[2] + s[3])) * silu_grad(pre[e]);
 }
 
 // ---------------------------------------------------------------------------
@@ -538,49 +561,167 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// input gradient: dU[c][v] = sum_o sum_t W[o][c][t] gy[o][v - t] on the fine
-// grid, summed over the 8 fine children of each coarse voxel when the input was
-// upsampled.  One thread per input voxel, all input channels (<= 32).
-template <int CIN>
-__global__ void k_conv_xgrad(const float *__restrict__ gy, const __nv_bfloat16 *__restrict__ W,
-                             float *__restrict__ dx, ConvGeom g, size_t g_stride, size_t dx_stride) {
-    extern __shared__ float ws[];
-    const int nw = g.cout * g.cin * 27;
-    for (int e = threadIdx.x; e < nw; e += blockDim.x)
-        ws[e] = __bfloat162float(W[e]);
+// Folded weights of the upsampling convolutions, refreshed whenever the BF16
+// weights change: FP32 sums of the 1, 2, 4 or 8 taps that meet in one coarse
+// voxel (k as in fold_k: 0 the tap +1, 1 taps 0 and +1, 2 taps -1 and 0, 3 the
+// tap -1, per axis).  bwd[o][kx ky kz][c] for the input gradient.
+struct FoldArgs {
+    int n;
+    struct {
+        int cin, cout;
+        size_t w, f; // offsets of the layer's weights and of its folded weights
+    } L[8];
+};
+__global__ void k_fold(const __nv_bfloat16 *__restrict__ wb, float *__restrict__ bwd, FoldArgs a) {
+    const auto L = a.L[blockIdx.y];
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < L.cin * L.cout * 64; e += gridDim.x * blockDim.x) {
+        const int c = e % L.cin, k = (e / L.cin) & 63, o = e / (L.cin * 64);
+        // first tap and number of taps per axis
+        auto lo = [](int q) { return q == 0 ? 2 : (q == 1 ? 1 : 0); };
+        auto nt = [](int q) { return q == 0 || q == 3 ? 1 : 2; };
+        const int kx = k >> 4, ky = (k >> 2) & 3, kz = k & 3;
+        const __nv_bfloat16 *w = wb + L.w + ((size_t)o * L.cin + c) * 27;
+        float v = 0.f;
+        for (int i = lo(kx); i < lo(kx) + nt(kx); ++i)
+            for (int j = lo(ky); j < lo(ky) + nt(ky); ++j)
+                for (int l = lo(kz); l < lo(kz) + nt(kz); ++l)
+                    v += __bfloat162float(w[(i * 3 + j) * 3 + l]);
+        bwd[L.f + e] = v;
+    }
+}
+
+// Input gradient of an upsampling convolution, on the coarse grid, times
+// SiLU'(pre) of the layer below (its dL/d(pre-activation)).  A coarse voxel v
+// collects from the fine voxels 2v - 1 .. 2v + 2 per axis with the folded
+// weights: 64 multiply-adds per channel pair instead of 8 x 27.  One thread: VX
+// coarse voxels along x and CT input channels (blockIdx.y: channel group), the
+// weights of a step shared by its voxels; lanes run along z (8-byte loads).
+// Bound by FP32 issue and the shared-memory weight reads (VX = 2 halves them);
+// small volumes take CT = 2, VX = 1 so that the layer fills the SMs.
+template <int CT, int VX>
+__global__ void __launch_bounds__(128)
+    k_up_xgrad(const float *__restrict__ gy, const float *__restrict__ bwd, const float *__restrict__ pre_in,
+               float *__restrict__ dx, ConvGeom g, size_t g_stride, size_t dx_stride) {
+    extern __shared__ __align__(16) float xg_ws[]; // [o][64][CT]
+    const int c0 = blockIdx.y * CT;
+    for (int e = threadIdx.x; e < g.cout * 64 * CT; e += 128)
+        xg_ws[e] = bwd[(size_t)(e / CT) * g.cin + c0 + e % CT];
     __syncthreads();
-    const int Xi = g.up ? g.X >> 1 : g.X, Yi = g.up ? g.Y >> 1 : g.Y, Zi = g.up ? g.Z >> 1 : g.Z;
-    const size_t ni = (size_t)Xi * Yi * Zi, nv = (size_t)g.X * g.Y * g.Z;
-    const float *gyb = gy + blockIdx.y * g_stride;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < ni; q += (size_t)gridDim.x * blockDim.x) {
-        const int zi = (int)(q % Zi), yi = (int)((q / Zi) % Yi), xi = (int)(q / ((size_t)Zi * Yi));
-        float acc[CIN];
+    const int Xi = g.X >> 1, Yi = g.Y >> 1, Zi = g.Z >> 1;
+    const int idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= Xi / VX * Yi * Zi)
+        return;
+    const int zi = idx % Zi, yi = idx / Zi % Yi, xi = idx / Zi / Yi * VX;
+    const size_t nv = (size_t)g.X * g.Y * g.Z;
+    const float *gyb = gy + blockIdx.z * g_stride + 2 * zi;
+    float acc[VX][CT];
 #pragma unroll
-        for (int c = 0; c < CIN; ++c)
-            acc[c] = 0.f;
-        const int nch = g.up ? 8 : 1;
-        for (int ch = 0; ch < nch; ++ch) {
-            const int x = g.up ? 2 * xi + (ch >> 2) : xi;
-            const int y = g.up ? 2 * yi + ((ch >> 1) & 1) : yi;
-            const int z = g.up ? 2 * zi + (ch & 1) : zi;
-            for (int t = 0; t < 27; ++t) {
-                // output voxel w = v - tap reads u[v] through tap t
-                const int ox = x - (t / 9 - 1), oy = y - ((t / 3) % 3 - 1), oz = z - (t % 3 - 1);
-                if (ox < 0 || oy < 0 || oz < 0 || ox >= g.X || oy >= g.Y || oz >= g.Z)
-                    continue;
-                const size_t w = ((size_t)ox * g.Y + oy) * g.Z + oz;
-                for (int o = 0; o < g.cout; ++o) {
-                    const float gv = __ldg(&gyb[(size_t)o * nv + w]);
+    for (int v = 0; v < VX; ++v)
 #pragma unroll
-                    for (int c = 0; c < CIN; ++c)
-                        acc[c] = fmaf(ws[(o * CIN + c) * 27 + t], gv, acc[c]);
+        for (int c = 0; c < CT; ++c)
+            acc[v][c] = 0.f;
+    const bool zl = zi > 0, zr = zi + 1 < Zi;
+    for (int o = 0; o < g.cout; ++o) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const int y = 2 * yi - 1 + b;
+            if (y < 0 || y >= g.Y)
+                continue;
+            float gv[2 * VX + 2][4];
+#pragma unroll
+            for (int a = 0; a < 2 * VX + 2; ++a) {
+                const int x = 2 * xi - 1 + a;
+                gv[a][0] = gv[a][1] = gv[a][2] = gv[a][3] = 0.f;
+                if (x >= 0 && x < g.X) {
+                    const float *r = gyb + o * nv + ((size_t)x * g.Y + y) * g.Z;
+                    const float2 m = __ldg(reinterpret_cast<const float2 *>(r));
+                    gv[a][1]       = m.x;
+                    gv[a][2]       = m.y;
+                    if (zl)
+                        gv[a][0] = __ldg(r - 1);
+                    if (zr)
+                        gv[a][3] = __ldg(r + 2);
                 }
             }
+#pragma unroll
+            for (int kx = 0; kx < 4; ++kx)
+#pragma unroll
+                for (int d = 0; d < 4; ++d) {
+                    const float *w = xg_ws + (size_t)(o * 64 + (kx * 4 + b) * 4 + d) * CT;
+#pragma unroll
+                    for (int c = 0; c < CT; ++c) {
+                        const float wc = w[c];
+#pragma unroll
+                        for (int v = 0; v < VX; ++v)
+                            acc[v][c] = fmaf(wc, gv[2 * v + kx][d], acc[v][c]);
+                    }
+                }
+        }
+    }
+#pragma unroll
+    for (int v = 0; v < VX; ++v)
+#pragma unroll
+        for (int c = 0; c < CT; ++c) {
+            const size_t q = blockIdx.z * dx_stride + (((size_t)(c0 + c) * Xi + xi + v) * Yi + yi) * Zi + zi;
+            dx[q]          = acc[v][c] * silu_grad(pre_in[q]);
+        }
+}
+
+// Input gradient of the last convolution (cin -> 1), times SiLU'(pre) of the
+// layer below.  One thread: 4 voxels along x and CT input channels; lanes take
+// neighbouring (y, z) columns.  A step's window of gy and its weights serve
+// 4 x CT sums.  Bound by the stores and the reads of `pre` (DRAM) at CT = 8.
+template <int CT>
+__global__ void __launch_bounds__(128)
+    k_last_xgrad(const float *__restrict__ gy, const __nv_bfloat16 *__restrict__ W, const float *__restrict__ pre_in,
+                 float *__restrict__ dx, ConvGeom g, size_t g_stride, size_t dx_stride) {
+    constexpr int RX = 4;
+    __shared__ __align__(16) float ws[27 * CT]; // [tap, mirrored][CT]
+    const int ngrp = g.cin / CT, c0 = (blockIdx.y % ngrp) * CT;
+    for (int e = threadIdx.x; e < 27 * CT; e += 128)
+        ws[e] = __bfloat162float(W[(size_t)(c0 + e % CT) * 27 + 26 - e / CT]);
+    __syncthreads();
+    const int cols = g.Y * g.Z, col = blockIdx.x * 128 + threadIdx.x;
+    if (col >= cols)
+        return;
+    const int y = col / g.Z, z = col - y * g.Z, x0 = blockIdx.y / ngrp * RX;
+    const float *gyb = gy + blockIdx.z * g_stride + col;
+    float acc[RX][CT];
+#pragma unroll
+    for (int r = 0; r < RX; ++r)
+#pragma unroll
+        for (int c = 0; c < CT; ++c)
+            acc[r][c] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int yy = y + k / 3 - 1, zz = z + k % 3 - 1;
+        if (yy < 0 || yy >= g.Y || zz < 0 || zz >= g.Z)
+            continue;
+        float gv[RX + 2];
+#pragma unroll
+        for (int r = 0; r < RX + 2; ++r) {
+            const int x = x0 + r - 1;
+            gv[r] = x >= 0 && x < g.X ? __ldg(gyb + (size_t)x * cols + (k / 3 - 1) * g.Z + k % 3 - 1) : 0.f;
         }
 #pragma unroll
-        for (int c = 0; c < CIN; ++c)
-            dx[blockIdx.y * dx_stride + (size_t)c * ni + q] = acc[c];
+        for (int d = 0; d < 3; ++d)
+#pragma unroll
+            for (int c = 0; c < CT; ++c) {
+                const float wc = ws[(d * 9 + k) * CT + c];
+#pragma unroll
+                for (int r = 0; r < RX; ++r)
+                    acc[r][c] = fmaf(wc, gv[r + d], acc[r][c]);
+            }
     }
+#pragma unroll
+    for (int c = 0; c < CT; ++c)
+#pragma unroll
+        for (int r = 0; r < RX; ++r) {
+            if (x0 + r >= g.X)
+                break;
+            const size_t q = blockIdx.z * dx_stride + ((size_t)(c0 + c) * g.X + x0 + r) * cols + col;
+            dx[q]          = acc[r][c] * silu_grad(pre_in[q]);
+        }
 }
 
 // loss partials of (u - target)^2 per block and gu = dL/du = 2 (u - t) / (B n)
@@ -663,6 +804,7 @@ struct gpe_warm {
     // parameter layout (offsets into the flat weight vector)
     struct Layer {
         size_t w = 0, b = 0; // offsets
+        size_t f = 0;        // offset of the folded weights (upsampling layers)
         int cin = 0, cout = 0;
         gpe::ConvGeom g{};
     };
@@ -671,6 +813,7 @@ struct gpe_warm {
     std::vector<Layer> conv; // levels upsampling stages + the last one
     Buf<float> w, m, v, grad;
     Buf<__nv_bfloat16> wb;
+    Buf<float> fold; // folded weights of the upsampling layers, as wb
     // activations (max_batch samples)
     Buf<float> x, h1pre, h1, h2pre, h2, gh1, gh2;
     std::vector<Buf<float>> pre, act, gact; // per conv layer output
@@ -702,6 +845,21 @@ template <class F> int wguard(F &&f) {
 }
 
 using gpe::Error;
+
+// the folded weights follow every change of the BF16 weights
+void refold(gpe_warm *W) {
+    gpe::FoldArgs a{};
+    for (const auto &L : W->conv)
+        if (L.g.up) {
+            a.L[a.n].cin  = L.cin;
+            a.L[a.n].cout = L.cout;
+            a.L[a.n].w    = L.w;
+            a.L[a.n++].f  = L.f;
+        }
+    if (a.n)
+        gpe::k_fold<<<dim3(64, a.n), 256, 0, W->stream>>>(W->wb.p, W->fold.p, a);
+    WS_CUDA(cudaGetLastError());
+}
 
 void forward(gpe_warm *W, int B) {
     using namespace gpe;
@@ -838,6 +996,37 @@ void conv_wgrad(gpe_warm *W, int l, int B, const float *in, size_t in_stride, co
     });
 }
 
+// dL/d(pre-activation) of the layer below l, from layer l's
+void conv_xgrad(gpe_warm *W, int l, int B, const float *gy, size_t g_stride, const float *pre_in, float *dx,
+                size_t dx_stride) {
+    const auto &L  = W->conv[l];
+    cudaStream_t s = W->stream;
+    if (!L.g.up) {
+        gpe::by_ot(std::min(L.cin, 8), [&](auto C) {
+            constexpr int CT = decltype(C)::value;
+            gpe::k_last_xgrad<CT><<<dim3((L.g.Y * L.g.Z + 127) / 128, (L.g.X + 3) / 4 * (L.cin / CT), B), 128, 0, s>>>(
+                gy, W->wb.p + L.w, pre_in, dx, L.g, g_stride, dx_stride);
+        });
+        return;
+    }
+    const int Xi = L.g.X / 2, nvox = Xi * (L.g.Y / 2) * (L.g.Z / 2);
+    auto go = [&](auto C, auto V) {
+        constexpr int CT = decltype(C)::value, VX = decltype(V)::value;
+        gpe::k_up_xgrad<CT, VX><<<dim3((nvox / VX + 127) / 128, L.cin / CT, B), 128, sizeof(float) * L.cout * 64 * CT,
+                                  s>>>(gy, W->fold.p + L.f, pre_in, dx, L.g, g_stride, dx_stride);
+    };
+    using I1 = std::integral_constant<int, 1>;
+    using I2 = std::integral_constant<int, 2>;
+    // two voxels and eight channels a thread where that still leaves 512 threads
+    // per SM, else one voxel and two channels (or one)
+    if (Xi % 2 == 0 && L.cin >= 8 && (size_t)nvox / 2 * (L.cin / 8) * B >= 148 * 512)
+        go(std::integral_constant<int, 8>{}, I2{});
+    else if (L.cin >= 2)
+        go(I2{}, I1{});
+    else
+        go(I1{}, I1{});
+}
+
 // gradients of the mean squared amplitude error against `targets` (device,
 // B x N floats); returns the loss (host)
 double backward(gpe_warm *W, int B, const float *targets) {
@@ -852,28 +1041,20 @@ double backward(gpe_warm *W, int B, const float *targets) {
                               1.f / (float)((size_t)B * N));
     for (int l = nl - 1; l >= 0; --l) {
         const auto &L  = W->conv[l];
-        const size_t n = W->vox(l) * L.cout;
-        float *gy      = W->gact[l].p; // dL/d(pre-activation) after the line below
-        if (l != nl - 1)
-            k_silu_back<<<gpe::grid_for((size_t)B * n), 256, 0, s>>>(gy, W->pre[l].p, (size_t)B * n);
+        const size_t n   = W->vox(l) * L.cout;
+        const float *gy  = W->gact[l].p; // dL/d(pre-activation)
         const float *in  = l == 0 ? W->h2.p : W->act[l - 1].p;
         const size_t ins = l == 0 ? (size_t)W->latent : W->vox(l - 1) * W->conv[l - 1].cout;
         conv_wgrad(W, l, B, in, ins, gy, n);
-        float *dx = l == 0 ? W->gh2.p : W->gact[l - 1].p;
-        const size_t ni = l == 0 ? (size_t)W->latent / L.cin : W->vox(l - 1);
-        const size_t sm = sizeof(float) * L.cin * L.cout * 27;
-        gpe::by_channels(L.cin, [&](auto CI) {
-            k_conv_xgrad<decltype(CI)::value><<<dim3(gpe::grid_for(ni), B), 256, sm, s>>>(gy, wb + L.w, dx, L.g, n,
-                                                                                       ni * L.cin);
-        });
+        conv_xgrad(W, l, B, gy, n, l == 0 ? W->h2pre.p : W->pre[l - 1].p, l == 0 ? W->gh2.p : W->gact[l - 1].p, ins);
     }
-    // dense 2 and dense 1
-    k_silu_back<<<gpe::grid_for((size_t)B * W->latent), 256, 0, s>>>(W->gh2.p, W->h2pre.p, (size_t)B * W->latent);
+    // dense 2 and dense 1 (gh2 and gh1 are gradients of the pre-activations)
     k_dense_wgrad<<<(int)(((size_t)W->latent * c.hidden + 255) / 256), 256, 0, s>>>(
         W->gh2.p, W->h1.p, W->grad.p + W->d2w, W->grad.p + W->d2b, B, c.hidden, W->latent);
-    k_dense_xgrad<<<dim3((c.hidden + 127) / 128, B), 128, 0, s>>>(W->gh2.p, wb + W->d2w, W->gh1.p, B, c.hidden,
-                                                                   W->latent);
-    k_silu_back<<<gpe::grid_for((size_t)B * c.hidden), 256, 0, s>>>(W->gh1.p, W->h1pre.p, (size_t)B * c.hidden);
+    const int rows = (W->latent + kXgRows - 1) / kXgRows;
+    k_dense_xgrad_part<<<dim3((c.hidden + 127) / 128, rows), 128, 0, s>>>(W->gh2.p, wb + W->d2w, W->partial.p, B,
+                                                                          c.hidden, W->latent);
+    k_dense_xgrad_sum<<<(B * c.hidden + 63) / 64, 64, 0, s>>>(W->partial.p, W->h1pre.p, W->gh1.p, B * c.hidden, rows);
     k_dense_wgrad<<<(int)(((size_t)c.hidden * c.n_inputs + 255) / 256), 256, 0, s>>>(
         W->gh1.p, W->x.p, W->grad.p + W->d1w, W->grad.p + W->d1b, B, c.n_inputs, c.hidden);
     WS_CUDA(cudaGetLastError());
@@ -935,6 +1116,11 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
             W->conv.push_back(L);
         }
         W->nweights = off;
+        size_t foff = 0;
+        for (auto &L : W->conv)
+            if (L.g.up)
+                L.f = foff, foff += (size_t)L.cin * L.cout * 64;
+        W->fold.alloc(foff);
         W->w.alloc(off);
         W->m.alloc(off);
         W->v.alloc(off);
@@ -951,7 +1137,8 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
         W->h2pre.alloc((size_t)B * W->latent);
         W->h2.alloc((size_t)B * W->latent);
         W->gh2.alloc((size_t)B * W->latent);
-        size_t maxpart = 0;
+        // partial sums: the weight gradients' and dense 2's input gradient's
+        size_t maxpart = (size_t)((W->latent + gpe::kXgRows - 1) / gpe::kXgRows) * B * c.hidden;
         W->pre.resize(W->conv.size());
         W->act.resize(W->conv.size());
         W->gact.resize(W->conv.size());
@@ -970,9 +1157,10 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
             gpe::by_channels(ch, [&](auto C) {
                 WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_conv_fwd<decltype(C)::value>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
-                WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_conv_xgrad<decltype(C)::value>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
             });
+        WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_up_xgrad<8, 2>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(float) * gpe::kMaxCout * 64 * 8));
         for (int ot : {1, 2, 4, 8})
             gpe::by_ot(ot, [&](auto O) {
                 WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_up_wgrad<decltype(O)::value>,
@@ -1007,6 +1195,7 @@ int gpe_warm_set_weights(gpe_warm *W, const float *host, size_t n) {
         WS_CUDA(cudaSetDevice(W->device));
         WS_CUDA(cudaMemcpyAsync(W->w.p, host, sizeof(float) * n, cudaMemcpyHostToDevice, W->stream));
         gpe::k_to_bf16<<<gpe::grid_for(n), 256, 0, W->stream>>>(W->w.p, W->wb.p, n);
+        refold(W);
         WS_CUDA(cudaMemsetAsync(W->m.p, 0, sizeof(float) * n, W->stream));
         WS_CUDA(cudaMemsetAsync(W->v.p, 0, sizeof(float) * n, W->stream));
         WS_CUDA(cudaStreamSynchronize(W->stream));
@@ -1095,6 +1284,7 @@ int gpe_warm_train_step(gpe_warm *W, const float *params_host, const float *targ
         gpe::k_adam<<<gpe::grid_for(W->nweights), 256, 0, W->stream>>>(W->w.p, W->m.p, W->v.p, W->grad.p, W->wb.p,
                                                                         W->nweights, lr, b1, b2, 1e-8f, c1, c2);
         WS_CUDA(cudaGetLastError());
+        refold(W);
     });
 }
 
