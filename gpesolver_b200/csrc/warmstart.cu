@@ -70,20 +70,39 @@ __device__ __forceinline__ float silu_grad(float y) {
 // ---------------------------------------------------------------------------
 // dense layers: Y[b][o] = sum_i W[o][i] X[b][i] + bias[o]
 // ---------------------------------------------------------------------------
-__global__ void k_dense_fwd(const float *__restrict__ X, const __nv_bfloat16 *__restrict__ W,
-                            const __nv_bfloat16 *__restrict__ bias, float *__restrict__ Ypre,
-                            float *__restrict__ Y, int B, int I, int O) {
-    const int o = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y;
-    if (o >= O || b >= B)
+// One warp per output row: the row is read once, coalesced, for up to eight
+// samples at a time (one thread per output walked its row alone: 25 us for 4096 x
+// 256, now bound by the 2 MB of weights and the launch).
+__global__ void __launch_bounds__(128)
+    k_dense_fwd(const float *__restrict__ X, const __nv_bfloat16 *__restrict__ W,
+                const __nv_bfloat16 *__restrict__ bias, float *__restrict__ Ypre, float *__restrict__ Y, int B, int I,
+                int O) {
+    const int o = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (o >= O)
         return;
-    float acc = __bfloat162float(bias[o]);
     const __nv_bfloat16 *w = W + (size_t)o * I;
-    const float *x         = X + (size_t)b * I;
-    for (int i = 0; i < I; ++i)
-        acc = fmaf(__bfloat162float(w[i]), x[i], acc);
-    Ypre[(size_t)b * O + o] = acc;
-    Y[(size_t)b * O + o]    = silu(acc);
+    for (int b0 = 0; b0 < B; b0 += 8) {
+        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int i = lane; i < I; i += 32) {
+            const float wi = __bfloat162float(w[i]);
+#pragma unroll
+            for (int b = 0; b < 8; ++b)
+                if (b0 + b < B)
+                    acc[b] = fmaf(wi, __ldg(&X[(size_t)(b0 + b) * I + i]), acc[b]);
+        }
+#pragma unroll
+        for (int b = 0; b < 8; ++b) {
+            float v = acc[b];
+            for (int off = 16; off > 0; off >>= 1)
+                v += __shfl_xor_sync(0xffffffffu, v, off);
+            if (lane == b && b0 + b < B) {
+                v += __bfloat162float(bias[o]);
+                Ypre[(size_t)(b0 + b) * O + o] = v;
+                Y[(size_t)(b0 + b) * O + o]    = silu(v);
+            }
+        }
+    }
 }
 
 // dW[o][i] = sum_b G[b][o] X[b][i];  db[o] = sum_b G[b][o]
@@ -156,138 +175,185 @@ struct ConvGeom {
     int up;         // 1: input is (X/2, Y/2, Z/2), read through nearest upsampling
 };
 
-// input value of channel c at fine position (x, y, z), zero outside
-__device__ __forceinline__ float conv_in(const float *__restrict__ in, const ConvGeom &g, int c, int x, int y,
-                                         int z) {
-    if (x < 0 || y < 0 || z < 0 || x >= g.X || y >= g.Y || z >= g.Z)
-        return 0.f;
-    if (g.up) {
-        const int Xc = g.X >> 1, Yc = g.Y >> 1, Zc = g.Z >> 1;
-        return __ldg(&in[(((size_t)c * Xc + (x >> 1)) * Yc + (y >> 1)) * Zc + (z >> 1)]);
-    }
-    return __ldg(&in[(((size_t)c * g.X + x) * g.Y + y) * g.Z + z]);
-}
-
 constexpr int kMaxCout = 32;
 
-// one thread per output voxel and group of COUT output channels (blockIdx.y =
-// sample * groups + group: small volumes spread their channels over more
-// threads); weights [o][c][27] BF16 staged in shared memory as FP32.  pre =
-// the pre-activation, out = SiLU(pre) (act = 0: out = pre).
-template <int COUT>
-__global__ void k_conv_fwd(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ W,
-                           const __nv_bfloat16 *__restrict__ bias, float *__restrict__ pre,
-                           float *__restrict__ out, ConvGeom g, int act, size_t in_stride, size_t out_stride) {
-    const int groups = g.cout / COUT;
-    const int smp = blockIdx.y / groups, o0 = (blockIdx.y % groups) * COUT;
-    extern __shared__ float ws[];
-    const int nw = g.cout * g.cin * 27;
-    for (int e = threadIdx.x; e < nw; e += blockDim.x)
-        ws[e] = __bfloat162float(W[e]);
-    __syncthreads();
-    const size_t nv = (size_t)g.X * g.Y * g.Z;
-    const float *inb = in + smp * in_stride;
-    for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < nv; v += (size_t)gridDim.x * blockDim.x) {
-        const int z = (int)(v % g.Z), y = (int)((v / g.Z) % g.Y), x = (int)(v / ((size_t)g.Z * g.Y));
-        float acc[COUT];
-#pragma unroll
-        for (int o = 0; o < COUT; ++o)
-            acc[o] = __bfloat162float(bias[o0 + o]);
-        for (int c = 0; c < g.cin; ++c)
-            for (int t = 0; t < 27; ++t) {
-                const int dx = t / 9 - 1, dy = (t / 3) % 3 - 1, dz = t % 3 - 1;
-                const float u = conv_in(inb, g, c, x + dx, y + dy, z + dz);
-#pragma unroll
-                for (int o = 0; o < COUT; ++o)
-                    acc[o] = fmaf(ws[((o0 + o) * g.cin + c) * 27 + t], u, acc[o]);
-            }
-#pragma unroll
-        for (int o = 0; o < COUT; ++o) {
-            const size_t q = smp * out_stride + (size_t)(o0 + o) * nv + v;
-            pre[q]         = acc[o];
-            out[q]         = act ? silu(acc[o]) : acc[o];
-        }
+// Folded weights of the upsampling convolutions, refreshed whenever the BF16
+// weights change.  Of the 27 fine taps an output voxel reads, the nearest
+// upsampling makes 1, 2, 4 or 8 meet in one coarse voxel: per axis an output of
+// parity p sees the coarse voxels v + p - 1 + t, t = 0, 1, with the FP32 sums
+//   k = fold_k(p, t):  0 the tap +1;  1 taps 0 and +1;  2 taps -1 and 0;  3 the tap -1
+// fwd[px py][c][tx ty pz tz][o] for the forward pass, bwd[o][kx ky kz][c] for the
+// input gradient.
+struct FoldArgs {
+    int n;
+    struct {
+        int cin, cout;
+        size_t w, f; // offsets of the layer's weights and of its folded weights
+    } L[8];
+};
+
+// position of the (parity, coarse tap) pair among the four folded taps of an axis
+__host__ __device__ __forceinline__ int fold_k(int p, int t) { return p == 0 ? (t == 0 ? 3 : 1) : (t == 0 ? 2 : 0); }
+
+__global__ void k_fold(const __nv_bfloat16 *__restrict__ wb, float *__restrict__ fwd, float *__restrict__ bwd,
+                       FoldArgs a) {
+    const auto L = a.L[blockIdx.y];
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < L.cin * L.cout * 64; e += gridDim.x * blockDim.x) {
+        const int c = e % L.cin, k = (e / L.cin) & 63, o = e / (L.cin * 64);
+        // first tap and number of taps per axis
+        auto lo = [](int q) { return q == 0 ? 2 : (q == 1 ? 1 : 0); };
+        auto nt = [](int q) { return q == 0 || q == 3 ? 1 : 2; };
+        const int kx = k >> 4, ky = (k >> 2) & 3, kz = k & 3;
+        const __nv_bfloat16 *w = wb + L.w + ((size_t)o * L.cin + c) * 27;
+        float v = 0.f;
+        for (int i = lo(kx); i < lo(kx) + nt(kx); ++i)
+            for (int j = lo(ky); j < lo(ky) + nt(ky); ++j)
+                for (int l = lo(kz); l < lo(kz) + nt(kz); ++l)
+                    v += __bfloat162float(w[(i * 3 + j) * 3 + l]);
+        bwd[L.f + e] = v;
+        // k -> (parity, tap): 3 (0, 0), 1 (0, 1), 2 (1, 0), 0 (1, 1)
+        auto par = [](int q) { return q == 0 || q == 2; };
+        auto tap = [](int q) { return q == 0 || q == 1; };
+        const int pxy = par(kx) * 2 + par(ky), t = tap(kx) * 8 + tap(ky) * 4 + par(kz) * 2 + tap(kz);
+        fwd[L.f + (((size_t)pxy * L.cin + c) * 16 + t) * L.cout + o] = v;
     }
 }
 
-// The same convolution on 8x8x8 output tiles, one voxel per thread (512
-// threads): the input tile with its halo is staged in shared memory once
-// (zeros outside the volume), the 27 taps and CIN channels unroll, so a voxel
-// costs CIN x 27 shared loads and CIN x 27 x COUT FMAs without per-tap index
-// arithmetic.  For volumes with all sizes multiples of 8 and the channel
-// counts instantiated below.  blockIdx.y = sample.
-template <int CIN, int COUT, int UP>
-__global__ void __launch_bounds__(512)
-    k_conv_fwd_tile(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ W,
-                    const __nv_bfloat16 *__restrict__ bias, float *__restrict__ pre, float *__restrict__ out,
-                    ConvGeom g, int act, size_t in_stride, size_t out_stride) {
-    constexpr int T = UP ? 6 : 10; // staged input tile edge
-    __shared__ float ws[COUT * CIN * 27];
-    __shared__ float ts[CIN * T * T * T];
-    const int tid = threadIdx.x;
-    for (int e = tid; e < COUT * CIN * 27; e += 512)
-        ws[e] = __bfloat162float(W[e]);
-    const int tx = g.X / 8, ty = g.Y / 8;
-    const int bx = blockIdx.x / (ty * (g.Z / 8)), rem = blockIdx.x % (ty * (g.Z / 8));
-    const int by = rem / (g.Z / 8), bz = rem % (g.Z / 8);
-    (void)tx;
-    const int x0 = bx * 8, y0 = by * 8, z0 = bz * 8;
-    const float *inb = in + blockIdx.y * in_stride;
-    // input origin of the tile (coarse grid when UP)
-    const int Xi = UP ? g.X / 2 : g.X, Yi = UP ? g.Y / 2 : g.Y, Zi = UP ? g.Z / 2 : g.Z;
-    const int ox = UP ? x0 / 2 - 1 : x0 - 1, oy = UP ? y0 / 2 - 1 : y0 - 1, oz = UP ? z0 / 2 - 1 : z0 - 1;
-    for (int e = tid; e < CIN * T * T * T; e += 512) {
-        const int c = e / (T * T * T), r = e % (T * T * T);
-        const int ix = ox + r / (T * T), iy = oy + (r / T) % T, iz = oz + r % T;
-        float v = 0.f;
-        if (ix >= 0 && iy >= 0 && iz >= 0 && ix < Xi && iy < Yi && iz < Zi)
-            v = __ldg(&inb[(((size_t)c * Xi + ix) * Yi + iy) * Zi + iz]);
-        ts[e] = v;
-    }
+// Forward upsampling convolution with the folded weights: 8 multiply-adds per
+// fine voxel and channel pair instead of 27.  A block has one (x, y) parity and
+// one group of OT output channels (blockIdx.y); a thread makes both z parities
+// of VX coarse voxels along x, so that a step's weights (shared memory, warp-uniform
+// 16-byte reads) serve 2 VX x OT sums and its u (L1) all of them; lanes run along z and
+// store 8 bytes each.  Bound by FP32 issue at <8, 2>; small volumes take fewer
+// channels a thread, so that the layer fills the SMs.  pre may be null (prediction).
+// Measured: 32 -> 32 channels to 16 x 16 x 4, 1 sample, 190 -> 18 us; 8 -> 8 to
+// 128 x 128 x 32, 8 samples, 747 -> 195 us.
+template <int OT, int VX>
+__global__ void __launch_bounds__(128)
+    k_up_fwd(const float *__restrict__ in, const float *__restrict__ fwd, const __nv_bfloat16 *__restrict__ bias,
+             float *__restrict__ pre, float *__restrict__ out, ConvGeom g, size_t in_stride, size_t out_stride) {
+    extern __shared__ __align__(16) float uf_ws[]; // [c][16][OT]
+    const int pxy = blockIdx.y & 3, px = pxy >> 1, py = pxy & 1, o0 = (blockIdx.y >> 2) * OT;
+    for (int e = threadIdx.x; e < g.cin * 16 * OT; e += 128)
+        uf_ws[e] = fwd[((size_t)pxy * g.cin * 16 + e / OT) * g.cout + o0 + e % OT];
     __syncthreads();
-    const int lx = tid / 64, ly = (tid / 8) % 8, lz = tid % 8;
-    // tile offsets of the three neighbours along each axis
-    int ax[3], ay[3], az[3];
+    const int Xi = g.X >> 1, Yi = g.Y >> 1, Zi = g.Z >> 1;
+    const int idx = blockIdx.x * 128 + threadIdx.x;
+    if (idx >= Xi / VX * Yi * Zi)
+        return;
+    const int zi = idx % Zi, yi = idx / Zi % Yi, xi = idx / Zi / Yi * VX;
+    const size_t ni  = (size_t)Xi * Yi * Zi;
+    const float *inb = in + blockIdx.z * in_stride + zi;
+    float acc[VX][2][OT];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        ax[d] = UP ? ((lx + d - 1) >> 1) + 1 : lx + d;
-        ay[d] = UP ? ((ly + d - 1) >> 1) + 1 : ly + d;
-        az[d] = UP ? ((lz + d - 1) >> 1) + 1 : lz + d;
-    }
-    float acc[COUT];
+    for (int v = 0; v < VX; ++v)
 #pragma unroll
-    for (int o = 0; o < COUT; ++o)
-        acc[o] = __bfloat162float(bias[o]);
+        for (int o = 0; o < OT; ++o)
+            acc[v][0][o] = acc[v][1][o] = __bfloat162float(bias[o0 + o]);
+    const bool zl = zi > 0, zr = zi + 1 < Zi;
+#pragma unroll 2
+    for (int c = 0; c < g.cin; ++c) {
+        float u[VX + 1][2][3];
 #pragma unroll
-    for (int c = 0; c < CIN; ++c) {
+        for (int a = 0; a <= VX; ++a)
 #pragma unroll
-        for (int t = 0; t < 27; ++t) {
-            const float u = ts[c * T * T * T + (ax[t / 9] * T + ay[(t / 3) % 3]) * T + az[t % 3]];
+            for (int b = 0; b < 2; ++b) {
+                const int x = xi + px - 1 + a, y = yi + py - 1 + b;
+                u[a][b][0] = u[a][b][1] = u[a][b][2] = 0.f;
+                if (x >= 0 && x < Xi && y >= 0 && y < Yi) {
+                    const float *r = inb + c * ni + ((size_t)x * Yi + y) * Zi;
+                    u[a][b][1]     = __ldg(r);
+                    if (zl)
+                        u[a][b][0] = __ldg(r - 1);
+                    if (zr)
+                        u[a][b][2] = __ldg(r + 1);
+                }
+            }
 #pragma unroll
-            for (int o = 0; o < COUT; ++o)
-                acc[o] = fmaf(ws[(o * CIN + c) * 27 + t], u, acc[o]);
+        for (int k = 0; k < 16; ++k) {
+            const int tx = k >> 3, ty = (k >> 2) & 1, pz = (k >> 1) & 1, tz = k & 1;
+            const float *w = uf_ws + (size_t)(c * 16 + k) * OT;
+#pragma unroll
+            for (int o = 0; o < OT; ++o) {
+                const float wo = w[o];
+#pragma unroll
+                for (int v = 0; v < VX; ++v)
+                    acc[v][pz][o] = fmaf(wo, u[v + tx][ty][pz + tz], acc[v][pz][o]);
+            }
         }
     }
-    const size_t nv = (size_t)g.X * g.Y * g.Z;
-    const size_t v  = ((size_t)(x0 + lx) * g.Y + (y0 + ly)) * g.Z + (z0 + lz);
 #pragma unroll
-    for (int o = 0; o < COUT; ++o) {
-        const size_t q = blockIdx.y * out_stride + (size_t)o * nv + v;
-        pre[q]         = acc[o];
-        out[q]         = act ? silu(acc[o]) : acc[o];
+    for (int v = 0; v < VX; ++v)
+#pragma unroll
+        for (int o = 0; o < OT; ++o) {
+            const size_t q = blockIdx.z * out_stride +
+                             (((size_t)(o0 + o) * g.X + 2 * (xi + v) + px) * g.Y + 2 * yi + py) * g.Z + 2 * zi;
+            const float2 y = make_float2(acc[v][0][o], acc[v][1][o]);
+            if (pre)
+                *reinterpret_cast<float2 *>(pre + q) = y;
+            *reinterpret_cast<float2 *>(out + q) = make_float2(silu(y.x), silu(y.y));
+        }
+}
+
+// The last convolution (cin -> 1, no upsampling, linear).  One thread: 4 voxels
+// along x, whose windows share their loads (L1); lanes take neighbouring (y, z)
+// columns.  Bound by the L1 reads (54 per 108 multiply-adds): 448 -> 182 us at 8
+// channels, 128 x 128 x 32, 8 samples (one voxel a thread, staged tiles, before).
+__global__ void __launch_bounds__(128)
+    k_last_fwd(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ W,
+               const __nv_bfloat16 *__restrict__ bias, float *__restrict__ out, ConvGeom g, size_t in_stride) {
+    constexpr int RX = 4;
+    __shared__ float ws[kMaxCout * 27];
+    for (int e = threadIdx.x; e < g.cin * 27; e += 128)
+        ws[e] = __bfloat162float(W[e]);
+    __syncthreads();
+    const int cols = g.Y * g.Z, col = blockIdx.x * 128 + threadIdx.x;
+    if (col >= cols)
+        return;
+    const int y = col / g.Z, z = col - y * g.Z, x0 = blockIdx.y * RX;
+    const float *inb = in + blockIdx.z * in_stride + col;
+    float acc[RX];
+#pragma unroll
+    for (int r = 0; r < RX; ++r)
+        acc[r] = __bfloat162float(bias[0]);
+    bool ok[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        const int yy = y + k / 3 - 1, zz = z + k % 3 - 1;
+        ok[k] = yy >= 0 && yy < g.Y && zz >= 0 && zz < g.Z;
     }
+    for (int c = 0; c < g.cin; ++c) {
+        const float *u = inb + (size_t)c * g.X * cols;
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            float uv[RX + 2];
+#pragma unroll
+            for (int r = 0; r < RX + 2; ++r) {
+                const int x = x0 + r - 1;
+                uv[r] = ok[k] && x >= 0 && x < g.X ? __ldg(u + (size_t)x * cols + (k / 3 - 1) * g.Z + k % 3 - 1) : 0.f;
+            }
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const float w = ws[c * 27 + d * 9 + k];
+#pragma unroll
+                for (int r = 0; r < RX; ++r)
+                    acc[r] = fmaf(w, uv[r + d], acc[r]);
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RX; ++r)
+        if (x0 + r < g.X)
+            out[(blockIdx.z * (size_t)g.X + x0 + r) * cols + col] = acc[r];
 }
 
 // Weight and bias gradients of an upsampling convolution, folded taps.
 //
-// Of the 27 fine taps an output voxel reads, the nearest upsampling makes
-// several read the same coarse voxel: per axis an output of parity p sees two
-// coarse voxels (p = 0: v-1, v; p = 1: v, v+1), so the gradient is gathered for
-// the 4 x 4 x 4 products of (parity, coarse tap) pairs,
+// The gradient is gathered for the 4 x 4 x 4 products of (parity, coarse tap)
+// pairs of fold_k,
 //   dK[o][c][kx ky kz] = sum_v gy[o][2v + p] u[c][v + p - 1 + t],
-// k = 3, 1 (p = 0, t = 0, 1) and 2, 0 (p = 1, t = 0, 1), and the 27 tap
-// gradients are sums of 8 of them (k_up_wgrad_reduce): 8 multiply-adds per fine
-// voxel and channel pair instead of 27.
+// and the 27 tap gradients are sums of 8 of them (k_up_wgrad_reduce): 8
+// multiply-adds per fine voxel and channel pair instead of 27.
 //
 // Bound by FP32 issue (FMA pipe) in the inner loop.  A CTA takes 8 input
 // channels x OT output channels (blockIdx.y) and strides over tiles of at most
@@ -297,7 +363,8 @@ __global__ void __launch_bounds__(512)
 // wavefronts, with the 4 x OT sums in registers.  The pitches put the 32 lanes'
 // u values in 32 banks.  Two halves of the warps split a tile's rows and are
 // added in shared memory at the end.
-//   8 -> 8 channels at 128 x 128 x 32, 8 samples: 30.8 ms -> see k_up_wgrad_reduce
+// Measured at 8 -> 8 channels, 128 x 128 x 32, 8 samples: 30.8 ms (one thread per
+// tap over 2048 voxels) -> 390 us.
 constexpr int kWgVox = 128; // coarse voxels per tile, at most
 
 struct WgTile {
@@ -306,9 +373,6 @@ struct WgTile {
     int nx, ny, nz, ntile; // tiles per axis, tiles over all samples
     int ncg;               // groups of 8 input channels
 };
-
-// position of the (parity, coarse tap) pair among the four folded taps of an axis
-__device__ __forceinline__ int fold_k(int p, int t) { return p == 0 ? (t == 0 ? 3 : 1) : (t == 0 ? 2 : 0); }
 
 template <int OT>
 __global__ void __launch_bounds__(256)
@@ -481,7 +545,8 @@ __global__ void __launch_bounds__(64 * OT * up_reduce_slices<OT>())
 // Lanes take neighbouring (y, z) columns and walk along x over a segment of sx
 // planes, holding the 3 x 9 window of one input channel (blockIdx.y) and the 27
 // sums in registers: 9 loads (L1) and 27 multiply-adds per voxel.  The block's
-// sums meet in shared memory.  blockIdx.x = column block x segment, z = sample.
+// sums meet in shared memory.  8 channels, 128 x 128 x 32, 8 samples: 4.2 ms -> 250 us.
+//  blockIdx.x = column block x segment, z = sample.
 __global__ void __launch_bounds__(256)
     k_last_wgrad(const float *__restrict__ in, const float *__restrict__ gy, float *__restrict__ partial,
                  ConvGeom g, int sx, int nseg, size_t in_stride, size_t g_stride) {
@@ -561,35 +626,6 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// Folded weights of the upsampling convolutions, refreshed whenever the BF16
-// weights change: FP32 sums of the 1, 2, 4 or 8 taps that meet in one coarse
-// voxel (k as in fold_k: 0 the tap +1, 1 taps 0 and +1, 2 taps -1 and 0, 3 the
-// tap -1, per axis).  bwd[o][kx ky kz][c] for the input gradient.
-struct FoldArgs {
-    int n;
-    struct {
-        int cin, cout;
-        size_t w, f; // offsets of the layer's weights and of its folded weights
-    } L[8];
-};
-__global__ void k_fold(const __nv_bfloat16 *__restrict__ wb, float *__restrict__ bwd, FoldArgs a) {
-    const auto L = a.L[blockIdx.y];
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < L.cin * L.cout * 64; e += gridDim.x * blockDim.x) {
-        const int c = e % L.cin, k = (e / L.cin) & 63, o = e / (L.cin * 64);
-        // first tap and number of taps per axis
-        auto lo = [](int q) { return q == 0 ? 2 : (q == 1 ? 1 : 0); };
-        auto nt = [](int q) { return q == 0 || q == 3 ? 1 : 2; };
-        const int kx = k >> 4, ky = (k >> 2) & 3, kz = k & 3;
-        const __nv_bfloat16 *w = wb + L.w + ((size_t)o * L.cin + c) * 27;
-        float v = 0.f;
-        for (int i = lo(kx); i < lo(kx) + nt(kx); ++i)
-            for (int j = lo(ky); j < lo(ky) + nt(ky); ++j)
-                for (int l = lo(kz); l < lo(kz) + nt(kz); ++l)
-                    v += __bfloat162float(w[(i * 3 + j) * 3 + l]);
-        bwd[L.f + e] = v;
-    }
-}
-
 // Input gradient of an upsampling convolution, on the coarse grid, times
 // SiLU'(pre) of the layer below (its dL/d(pre-activation)).  A coarse voxel v
 // collects from the fine voxels 2v - 1 .. 2v + 2 per axis with the folded
@@ -597,7 +633,8 @@ __global__ void k_fold(const __nv_bfloat16 *__restrict__ wb, float *__restrict__
 // coarse voxels along x and CT input channels (blockIdx.y: channel group), the
 // weights of a step shared by its voxels; lanes run along z (8-byte loads).
 // Bound by FP32 issue and the shared-memory weight reads (VX = 2 halves them);
-// small volumes take CT = 2, VX = 1 so that the layer fills the SMs.
+// small volumes take CT = 2, VX = 1 so that the layer fills the SMs.  8 -> 8
+// channels at 128 x 128 x 32, 8 samples: 1086 + 2 x 70 (SiLU' pass) -> 200 us.
 template <int CT, int VX>
 __global__ void __launch_bounds__(128)
     k_up_xgrad(const float *__restrict__ gy, const float *__restrict__ bwd, const float *__restrict__ pre_in,
@@ -781,17 +818,6 @@ template <class F> void by_ot(int ot, F &&f) {
     default: f(std::integral_constant<int, 8>{}); break;
     }
 }
-template <class F> void by_channels(int c, F &&f) {
-    switch (c) {
-    case 1: f(std::integral_constant<int, 1>{}); break;
-    case 2: f(std::integral_constant<int, 2>{}); break;
-    case 4: f(std::integral_constant<int, 4>{}); break;
-    case 8: f(std::integral_constant<int, 8>{}); break;
-    case 16: f(std::integral_constant<int, 16>{}); break;
-    default: f(std::integral_constant<int, 32>{}); break;
-    }
-}
-
 } // namespace
 } // namespace gpe
 
@@ -857,67 +883,48 @@ void refold(gpe_warm *W) {
             a.L[a.n++].f  = L.f;
         }
     if (a.n)
-        gpe::k_fold<<<dim3(64, a.n), 256, 0, W->stream>>>(W->wb.p, W->fold.p, a);
+        gpe::k_fold<<<dim3(64, a.n), 256, 0, W->stream>>>(W->wb.p, W->fold.p, W->fold.p + W->fold.n / 2, a);
     WS_CUDA(cudaGetLastError());
 }
 
-void forward(gpe_warm *W, int B) {
+// the amplitudes of W->x into amp; the backward pass's values are kept when training
+void forward(gpe_warm *W, int B, float *amp, bool training) {
     using namespace gpe;
     const auto &c = W->cfg;
     cudaStream_t s = W->stream;
     const __nv_bfloat16 *wb = W->wb.p;
-    k_dense_fwd<<<dim3((c.hidden + 127) / 128, B), 128, 0, s>>>(W->x.p, wb + W->d1w, wb + W->d1b, W->h1pre.p,
-                                                                 W->h1.p, B, c.n_inputs, c.hidden);
-    k_dense_fwd<<<dim3((W->latent + 127) / 128, B), 128, 0, s>>>(W->h1.p, wb + W->d2w, wb + W->d2b, W->h2pre.p,
-                                                                  W->h2.p, B, c.hidden, W->latent);
-    const float *in = W->h2.p;
+    k_dense_fwd<<<(c.hidden + 3) / 4, 128, 0, s>>>(W->x.p, wb + W->d1w, wb + W->d1b, W->h1pre.p, W->h1.p, B,
+                                                   c.n_inputs, c.hidden);
+    k_dense_fwd<<<(W->latent + 3) / 4, 128, 0, s>>>(W->h1.p, wb + W->d2w, wb + W->d2b, W->h2pre.p, W->h2.p, B,
+                                                    c.hidden, W->latent);
+    const float *in  = W->h2.p;
     size_t in_stride = W->latent;
-    for (size_t l = 0; l < W->conv.size(); ++l) {
-        const auto &L  = W->conv[l];
-        const size_t n = W->vox((int)l) * L.cout;
-        const size_t sm = sizeof(float) * L.cin * L.cout * 27;
-        const int last  = l + 1 == W->conv.size();
-        const size_t nvox = W->vox((int)l);
-        if (L.g.X % 8 == 0 && L.g.Y % 8 == 0 && L.g.Z % 8 == 0 && nvox >= 32768) {
-            const int tiles = (L.g.X / 8) * (L.g.Y / 8) * (L.g.Z / 8);
-            bool done = false;
-            auto go = [&](auto CI, auto CO, auto UPc) {
-                constexpr int ci = decltype(CI)::value, co = decltype(CO)::value, up = decltype(UPc)::value;
-                if (L.cin == ci && L.cout == co && L.g.up == up) {
-                    gpe::k_conv_fwd_tile<ci, co, up><<<dim3(tiles, B), 512, 0, s>>>(
-                        in, wb + L.w, wb + L.b, W->pre[l].p, W->act[l].p, L.g, last ? 0 : 1, in_stride, n);
-                    done = true;
-                }
-            };
-            using I4 = std::integral_constant<int, 4>;
-            using I8 = std::integral_constant<int, 8>;
-            using I16 = std::integral_constant<int, 16>;
-            using I1 = std::integral_constant<int, 1>;
-            using U0 = std::integral_constant<int, 0>;
-            using U1 = std::integral_constant<int, 1>;
-            go(I16{}, I8{}, U1{});
-            go(I8{}, I8{}, U1{});
-            go(I8{}, I4{}, U1{});
-            go(I4{}, I4{}, U1{});
-            go(I8{}, I1{}, U0{});
-            go(I4{}, I1{}, U0{});
-            go(I8{}, I8{}, U0{});
-            if (done) {
-                in        = W->act[l].p;
-                in_stride = n;
-                continue;
-            }
+    for (const auto &L : W->conv) {
+        const size_t l = &L - W->conv.data();
+        if (!L.g.up) {
+            k_last_fwd<<<dim3((L.g.Y * L.g.Z + 127) / 128, (L.g.X + 3) / 4, B), 128, 0, s>>>(
+                in, wb + L.w, wb + L.b, amp, L.g, in_stride);
+            break;
         }
-        // output channels per thread: all of them on large volumes, fewer on
-        // small ones, so that a layer runs at least ~64 k threads
-        int per = L.cout;
-        while (per > 1 && nvox * B * (L.cout / per) < 65536)
-            per >>= 1;
-        const int groups = L.cout / per;
-        gpe::by_channels(per, [&](auto CO) {
-            k_conv_fwd<decltype(CO)::value><<<dim3(gpe::grid_for(nvox), B * groups), 256, sm, s>>>(
-                in, wb + L.w, wb + L.b, W->pre[l].p, W->act[l].p, L.g, last ? 0 : 1, in_stride, n);
-        });
+        const int Xi = L.g.X / 2, nvox = Xi * (L.g.Y / 2) * (L.g.Z / 2);
+        const size_t n = W->vox((int)l) * L.cout;
+        auto go = [&](auto O, auto V) {
+            constexpr int OT = decltype(O)::value, VX = decltype(V)::value;
+            k_up_fwd<OT, VX><<<dim3((nvox / VX + 127) / 128, 4 * (L.cout / OT), B), 128,
+                               sizeof(float) * L.cin * 16 * OT, s>>>(in, W->fold.p + L.f, wb + L.b,
+                                                                     training ? W->pre[l].p : nullptr, W->act[l].p,
+                                                                     L.g, in_stride, n);
+        };
+        using I1 = std::integral_constant<int, 1>;
+        using I2 = std::integral_constant<int, 2>;
+        // two voxels and eight channels a thread where that still leaves 512
+        // threads per SM, else one voxel and two channels (or one)
+        if (Xi % 2 == 0 && L.cout >= 8 && (size_t)nvox / 2 * 4 * (L.cout / 8) * B >= 148 * 512)
+            go(std::integral_constant<int, 8>{}, I2{});
+        else if (L.cout >= 2)
+            go(I2{}, I1{});
+        else
+            go(I1{}, I1{});
         in        = W->act[l].p;
         in_stride = n;
     }
@@ -1013,7 +1020,7 @@ void conv_xgrad(gpe_warm *W, int l, int B, const float *gy, size_t g_stride, con
     auto go = [&](auto C, auto V) {
         constexpr int CT = decltype(C)::value, VX = decltype(V)::value;
         gpe::k_up_xgrad<CT, VX><<<dim3((nvox / VX + 127) / 128, L.cin / CT, B), 128, sizeof(float) * L.cout * 64 * CT,
-                                  s>>>(gy, W->fold.p + L.f, pre_in, dx, L.g, g_stride, dx_stride);
+                                  s>>>(gy, W->fold.p + W->fold.n / 2 + L.f, pre_in, dx, L.g, g_stride, dx_stride);
     };
     using I1 = std::integral_constant<int, 1>;
     using I2 = std::integral_constant<int, 2>;
@@ -1120,7 +1127,7 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
         for (auto &L : W->conv)
             if (L.g.up)
                 L.f = foff, foff += (size_t)L.cin * L.cout * 64;
-        W->fold.alloc(foff);
+        W->fold.alloc(2 * foff); // forward, then backward
         W->w.alloc(off);
         W->m.alloc(off);
         W->v.alloc(off);
@@ -1151,13 +1158,7 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
         }
         W->partial.alloc(maxpart);
         W->lpart.alloc(148 * 4);
-        // weights staged in shared memory: up to 32 x 32 x 27 floats
-        const int smax = (int)(sizeof(float) * gpe::kMaxCout * gpe::kMaxCout * 27);
-        for (int ch : {1, 2, 4, 8, 16, 32})
-            gpe::by_channels(ch, [&](auto C) {
-                WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_conv_fwd<decltype(C)::value>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smax));
-            });
+        // folded weights staged in shared memory, up to 32 channels
         WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_up_xgrad<8, 2>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(float) * gpe::kMaxCout * 64 * 8));
@@ -1239,11 +1240,7 @@ int gpe_warm_forward(gpe_warm *W, const float *params_host, int B, float *amp_de
     return wguard([&] {
         WS_CUDA(cudaSetDevice(W->device));
         upload_inputs(W, params_host, B);
-        forward(W, B);
-        const int nl   = (int)W->conv.size();
-        const size_t n = (size_t)B * W->vox(nl - 1);
-        WS_CUDA(cudaMemcpyAsync(amp_dev, W->pre[nl - 1].p, sizeof(float) * n, cudaMemcpyDeviceToDevice,
-                                W->stream));
+        forward(W, B, amp_dev, false);
         WS_CUDA(cudaStreamSynchronize(W->stream));
     });
 }
@@ -1255,7 +1252,7 @@ int gpe_warm_gradients(gpe_warm *W, const float *params_host, const float *targe
     return wguard([&] {
         WS_CUDA(cudaSetDevice(W->device));
         upload_inputs(W, params_host, B);
-        forward(W, B);
+        forward(W, B, W->pre.back().p, true);
         const double l = backward(W, B, targets_dev);
         if (loss)
             *loss = l;
@@ -1274,7 +1271,7 @@ int gpe_warm_train_step(gpe_warm *W, const float *params_host, const float *targ
     return wguard([&] {
         WS_CUDA(cudaSetDevice(W->device));
         upload_inputs(W, params_host, B);
-        forward(W, B);
+        forward(W, B, W->pre.back().p, true);
         const double l = backward(W, B, targets_dev);
         if (loss)
             *loss = l;
