@@ -2,8 +2,8 @@
 //
 // A CTA transforms a tile of `count` independent lines of length L held in
 // shared memory: element t of line b sits at s[b*bs + t*ts].  Each stage of the
-// mixed-radix Stockham auto-sort algorithm (radix r in {2,3,4,5,7,8,16}) maps
-// one thread to one r-point butterfly held in registers:
+// mixed-radix Stockham auto-sort algorithm (radix r <= 16 with factors 2, 3, 5, 7)
+// maps one thread to one r-point butterfly held in registers:
 //
 //   a_k = src[j + k L/r] * W_{Ns r}^{(j mod Ns) k}            k < r
 //   b   = DFT_r(a)                                            (in registers)
@@ -108,6 +108,10 @@ template <int SIGN, class C, class R, bool CMP> __device__ __forceinline__ C mul
     else
         return mul_w<SIGN>(a, (R)c, (R)s);
 }
+
+template <int SIGN, class R, bool CMP> struct DFT<1, SIGN, R, CMP> {
+    static __device__ __forceinline__ void run(cplx<R> *) {}
+};
 
 template <int SIGN, class R, bool CMP> struct DFT<2, SIGN, R, CMP> {
     using C = cplx<R>;
@@ -216,73 +220,75 @@ template <int SIGN, class R, bool CMP> struct DFTZ<16, SIGN, R, CMP, 8> {
     static __device__ __forceinline__ void run(cplx<R> *a) { DFTSplit<4, 4, SIGN, R, CMP, 2>::run(a); }
 };
 
-// Odd prime radices: direct r-point sums with the constant table cos/sin(2 pi m / r).
+// Odd prime radices, with the inputs paired as sums and differences (x_k +- x_{P-k}):
+// (P-1)^2 / 2 real products per component instead of 2 (P-1)^2.
 template <int P> struct OddTab;
 template <> struct OddTab<3> {
-    static __device__ __forceinline__ double c(int m) { return m == 0 ? 1.0 : -0.5; }
+    static __device__ __forceinline__ double c(int) { return -0.5; }
     static __device__ __forceinline__ double s(int m) {
-        return m == 0 ? 0.0 : (m == 1 ? 0.86602540378443864676 : -0.86602540378443864676);
+        return m == 1 ? 0.86602540378443864676 : -0.86602540378443864676;
     }
 };
 template <> struct OddTab<5> {
     static __device__ __forceinline__ double c(int m) {
         constexpr double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;
-        return m == 0 ? 1.0 : (m == 1 || m == 4) ? c1 : c2;
+        return (m == 1 || m == 4) ? c1 : c2;
     }
     static __device__ __forceinline__ double s(int m) {
         constexpr double s1 = 0.95105651629515357212, s2 = 0.58778525229247312917;
-        switch (m) {
-        case 1: return s1;
-        case 2: return s2;
-        case 3: return -s2;
-        case 4: return -s1;
-        default: return 0.0;
-        }
+        return m == 1 ? s1 : (m == 2 ? s2 : (m == 3 ? -s2 : -s1));
     }
 };
 template <> struct OddTab<7> {
     static __device__ __forceinline__ double c(int m) {
         constexpr double c1 = 0.62348980185873353053, c2 = -0.22252093395631440429,
                          c3 = -0.90096886790241912624;
-        switch (m) {
-        case 0: return 1.0;
-        case 1: case 6: return c1;
-        case 2: case 5: return c2;
-        default: return c3;
-        }
+        return (m == 1 || m == 6) ? c1 : ((m == 2 || m == 5) ? c2 : c3);
     }
     static __device__ __forceinline__ double s(int m) {
         constexpr double s1 = 0.78183148246802980871, s2 = 0.97492791218182360702,
                          s3 = 0.43388373911755812048;
-        switch (m) {
-        case 1: return s1;
-        case 2: return s2;
-        case 3: return s3;
-        case 4: return -s3;
-        case 5: return -s2;
-        case 6: return -s1;
-        default: return 0.0;
-        }
+        return m == 1 ? s1 : (m == 2 ? s2 : (m == 3 ? s3 : (m == 4 ? -s3 : (m == 5 ? -s2 : -s1))));
     }
 };
 
 template <int P, int SIGN, class R, bool CMP = true> struct DFTOdd {
     using C = cplx<R>;
+    static __device__ __forceinline__ R mulc(R x, double c) {
+        if constexpr (CMP)
+            return cmulk<R>(x, c);
+        else
+            return x * (R)c;
+    }
     static __device__ __forceinline__ void run(C *a) {
-        C out[P];
+        constexpr int H = P / 2;
+        C t[H], d[H];
 #pragma unroll
-        for (int q = 0; q < P; ++q) {
-            C acc = a[0];
-#pragma unroll
-            for (int k = 1; k < P; ++k) {
-                const int m = (k * q) % P;
-                acc         = cadd(acc, mul_wc<SIGN, C, R, CMP>(a[k], OddTab<P>::c(m), OddTab<P>::s(m)));
-            }
-            out[q] = acc;
+        for (int k = 0; k < H; ++k) {
+            t[k] = cadd(a[k + 1], a[P - 1 - k]);
+            d[k] = csub(a[k + 1], a[P - 1 - k]);
         }
+        const C x0 = a[0];
+        C sum      = x0;
 #pragma unroll
-        for (int q = 0; q < P; ++q)
-            a[q] = out[q];
+        for (int k = 0; k < H; ++k)
+            sum = cadd(sum, t[k]);
+        a[0] = sum;
+#pragma unroll
+        for (int q = 1; q <= H; ++q) {
+            C re = x0, im{(R)0, (R)0}; // X_q = re + SIGN i im, X_{P-q} = re - SIGN i im
+#pragma unroll
+            for (int k = 0; k < H; ++k) {
+                const int m = ((k + 1) * q) % P;
+                re.x += mulc(t[k].x, OddTab<P>::c(m));
+                re.y += mulc(t[k].y, OddTab<P>::c(m));
+                im.x += mulc(d[k].x, OddTab<P>::s(m));
+                im.y += mulc(d[k].y, OddTab<P>::s(m));
+            }
+            const C j = mul_si<SIGN>(im);
+            a[q]      = cadd(re, j);
+            a[P - q]  = csub(re, j);
+        }
     }
 };
 template <int SIGN, class R, bool CMP> struct DFT<3, SIGN, R, CMP> {
@@ -295,13 +301,75 @@ template <int SIGN, class R, bool CMP> struct DFT<7, SIGN, R, CMP> {
     static __device__ __forceinline__ void run(cplx<R> *a) { DFTOdd<7, SIGN, R, CMP>::run(a); }
 };
 
-// Plan of one line transform of length L (host-built; passed by value).
-struct LinePlan {
-    int L;
-    int nstages;
-    int radix[8];
-    const void *tw;   // cplx<R>[L]: exp(-2 pi i m / L), rounded to R
-    const void *twlo; // FP32 only: cplx<R>[L], the rounding remainder of tw
+// N = N1 * N2 with coprime factors (Good-Thomas): inputs at N2 n1 + N1 n2, output
+// k from (k mod N1, k mod N2); no twiddles between the two.
+template <int N1, int N2, int SIGN, class R, bool CMP> struct DFTCoprime {
+    using C = cplx<R>;
+    static __device__ __forceinline__ void run(C *a) {
+        constexpr int N = N1 * N2;
+        C y[N2][N1];
+#pragma unroll
+        for (int n2 = 0; n2 < N2; ++n2) {
+#pragma unroll
+            for (int n1 = 0; n1 < N1; ++n1)
+                y[n2][n1] = a[(N2 * n1 + N1 * n2) % N];
+            DFT<N1, SIGN, R, CMP>::run(y[n2]);
+        }
+#pragma unroll
+        for (int k1 = 0; k1 < N1; ++k1) {
+            C z[N2];
+#pragma unroll
+            for (int n2 = 0; n2 < N2; ++n2)
+                z[n2] = y[n2][k1];
+            DFT<N2, SIGN, R, CMP>::run(z);
+#pragma unroll
+            for (int n2 = 0; n2 < N2; ++n2)
+                y[n2][k1] = z[n2];
+        }
+#pragma unroll
+        for (int k = 0; k < N; ++k)
+            a[k] = y[k % N2][k % N1];
+    }
+};
+#define GPE_DFT_COPRIME(N, A, B)                                                                   \
+    template <int SIGN, class R, bool CMP> struct DFT<N, SIGN, R, CMP> {                           \
+        static __device__ __forceinline__ void run(cplx<R> *a) { DFTCoprime<A, B, SIGN, R, CMP>::run(a); } \
+    };
+GPE_DFT_COPRIME(6, 3, 2)
+GPE_DFT_COPRIME(10, 5, 2)
+GPE_DFT_COPRIME(12, 3, 4)
+GPE_DFT_COPRIME(14, 7, 2)
+GPE_DFT_COPRIME(15, 3, 5)
+#undef GPE_DFT_COPRIME
+
+// 9 = 3 x 3 with the twiddles exp(SIGN 2 pi i m / 9), m = 1, 2, 4
+template <int SIGN, class R, bool CMP> struct DFT<9, SIGN, R, CMP> {
+    using C = cplx<R>;
+    static __device__ __forceinline__ void run(C *a) {
+        constexpr double c1 = 0.76604444311897803520, s1 = 0.64278760968653932632;
+        constexpr double c2 = 0.17364817766693034885, s2 = 0.98480775301220805937;
+        constexpr double c4 = -0.93969262078590838405, s4 = 0.34202014332566873304;
+        C y[3][3];
+#pragma unroll
+        for (int n2 = 0; n2 < 3; ++n2) {
+#pragma unroll
+            for (int n1 = 0; n1 < 3; ++n1)
+                y[n2][n1] = a[3 * n1 + n2];
+            DFT<3, SIGN, R, CMP>::run(y[n2]);
+        }
+        y[1][1] = mul_wc<SIGN, C, R, CMP>(y[1][1], c1, s1);
+        y[1][2] = mul_wc<SIGN, C, R, CMP>(y[1][2], c2, s2);
+        y[2][1] = mul_wc<SIGN, C, R, CMP>(y[2][1], c2, s2);
+        y[2][2] = mul_wc<SIGN, C, R, CMP>(y[2][2], c4, s4);
+#pragma unroll
+        for (int k1 = 0; k1 < 3; ++k1) {
+            C z[3] = {y[0][k1], y[1][k1], y[2][k1]};
+            DFT<3, SIGN, R, CMP>::run(z);
+#pragma unroll
+            for (int k2 = 0; k2 < 3; ++k2)
+                a[k1 + 3 * k2] = z[k2];
+        }
+    }
 };
 
 // v * w (SIGN < 0) or v * conj(w) (SIGN > 0) with w = hi + lo (compensated).
@@ -310,77 +378,6 @@ template <int SIGN, class C> __device__ __forceinline__ C twmul(C v, C hi, C lo)
     const float cre = v.x * lo.x - v.y * sl;
     const float cim = v.x * sl + v.y * lo.x;
     return C{fmaf(v.x, hi.x, fmaf(-v.y, sh, cre)), fmaf(v.x, sh, fmaf(v.y, hi.x, cim))};
-}
-
-template <int RADIX, int SIGN, class R>
-__device__ __forceinline__ void fft_stage(const cplx<R> *__restrict__ src, cplx<R> *__restrict__ dst,
-                                          int L, int Ns, int count, int bs, int ts,
-                                          const cplx<R> *__restrict__ tw,
-                                          const cplx<R> *__restrict__ twlo, int tid, int nthreads) {
-    using C         = cplx<R>;
-    const int nr    = L / RADIX;
-    const int step  = L / (Ns * RADIX);
-    const int items = count * nr;
-    // consecutive threads take consecutive lines b: with the tile layouts used
-    // here (bs = 1) their shared-memory accesses fall in distinct banks.
-    for (int it = tid; it < items; it += nthreads) {
-        const int j  = it / count;
-        const int b  = it - j * count;
-        const int jm = j % Ns;
-        C a[RADIX];
-        const C *s = src + (size_t)b * bs + (size_t)j * ts;
-#pragma unroll
-        for (int k = 0; k < RADIX; ++k) {
-            C v = s[(size_t)k * nr * ts];
-            if (k > 0 && jm > 0) {
-                const int t = jm * k * step; // < Ns * RADIX * step = L
-                const C w   = __ldg(&tw[t]);
-                if constexpr (sizeof(R) == 4)
-                    v = twmul<SIGN>(v, w, __ldg(&twlo[t]));
-                else
-                    v = SIGN < 0 ? cmul(v, w) : cmulc(v, w);
-            }
-            a[k] = v;
-        }
-        DFT<RADIX, SIGN, R>::run(a);
-        const int idxD = (j / Ns) * Ns * RADIX + jm;
-        C *d           = dst + (size_t)b * bs + (size_t)idxD * ts;
-#pragma unroll
-        for (int q = 0; q < RADIX; ++q)
-            d[(size_t)q * Ns * ts] = a[q];
-    }
-}
-
-// Transforms the tile in buf0 (using buf1 as the second Stockham buffer).
-// Requires the tile to be complete in shared memory (caller syncs before);
-// syncs after every stage.  Returns the buffer that holds the result.
-template <int SIGN, class R>
-__device__ cplx<R> *block_fft(cplx<R> *buf0, cplx<R> *buf1, const LinePlan &ln, int count, int bs,
-                              int ts, int tid, int nthreads) {
-    using C     = cplx<R>;
-    C *src      = buf0;
-    C *dst      = buf1;
-    int Ns      = 1;
-    const C *tw = reinterpret_cast<const C *>(ln.tw);
-    const C *tl = reinterpret_cast<const C *>(ln.twlo);
-    for (int s = 0; s < ln.nstages; ++s) {
-        const int r = ln.radix[s];
-        switch (r) {
-        case 2: fft_stage<2, SIGN, R>(src, dst, ln.L, Ns, count, bs, ts, tw, tl, tid, nthreads); break;
-        case 3: fft_stage<3, SIGN, R>(src, dst, ln.L, Ns, count, bs, ts, tw, tl, tid, nthreads); break;
-        case 4: fft_stage<4, SIGN, R>(src, dst, ln.L, Ns, count, bs, ts, tw, tl, tid, nthreads); break;
-        case 5: fft_stage<5, SIGN, R>(src, dst, ln.L, Ns, count, bs, ts, tw, tl, tid, nthreads); break;
-        case 7: fft_stage<7, SIGN, R>(src, dst, ln.L, Ns, count, bs, ts, tw, tl, tid, nthreads); break;
-        case 8: fft_stage<8, SIGN, R>(src, dst, ln.L, Ns, count, bs, ts, tw, tl, tid, nthreads); break;
-        default: fft_stage<16, SIGN, R>(src, dst, ln.L, Ns, count, bs, ts, tw, tl, tid, nthreads); break;
-        }
-        __syncthreads();
-        C *t = src;
-        src  = dst;
-        dst  = t;
-        Ns *= r;
-    }
-    return src;
 }
 
 } // namespace gpe

@@ -45,12 +45,6 @@ struct Twid {
     const void *lo;
 };
 
-struct StepIdx {
-    const StepCoef *coef; // per-iteration coefficients of this call
-    const int *base;      // device counter: index of the chunk's first iteration
-    int local;            // iteration within the chunk
-};
-
 enum { ZM_RT_PRO = 0, ZM_RT_MID, ZM_RT_EPI, ZM_IT_PRO, ZM_IT_MID };
 
 // Asynchronous global -> shared copies (cp.async, completion per thread; a
@@ -312,28 +306,6 @@ template <class R, int N, int CNT> struct YShape {
 // ---------------------------------------------------------------------------
 // Z rows
 // ---------------------------------------------------------------------------
-struct ZArgs {
-    // fields
-    void *psi_in;        // RT: the kinetic increment's yz spectrum (psi in RT_PRO); IT: psi
-    void *psi_out;       // RT: same as psi_in; IT: the next psi buffer
-    void *psi_r;         // RT: psi in real space after the last phase step (read, then rewritten)
-    const void *bnd;     // IT: boundary values (last loaded psi)
-    void *S;             // dipolar spectrum
-    const void *V;
-    void *phi;
-    // norms (IT)
-    double *norm_state;  // [0] xnorma, [1] divisor of psi_in (read), both written by the last CTA
-    double *partial;     // per-CTA partial sums of |psi_out|^2
-    unsigned *ticket;    // CTA completion counter (reset by the last CTA)
-    int *status;
-    double dV;
-    // coefficients
-    StepIdx step;
-    double half_dt, cdd, w_atoms;
-    double cx, cy, cz, dtau; // IT stencil
-    int nx, ny;
-};
-
 template <class R, int NZ, int MODE>
 __global__ void __launch_bounds__(256, 4) k2_z(ZArgs a, Twid tk, Twid td) {
     using C          = cplx<R>;

@@ -1,0 +1,630 @@
+// The iteration for every grid and both precisions: line lengths at run time.
+//
+// The grids that fused.cuh has compiled line lengths for take its kernels; all
+// others, complex128, and the interface's single steps take these.  One iteration is four
+// kernels, each a batch of 1D lines with the elementwise physics in its loads
+// and stores, the kinetic and the dipolar lines of a pass in one launch:
+//
+//   g_x  lines along x, forward, factor, inverse: kinetic FFT(nx), exp(i(-dt/2m)k^2) / N;
+//        dipolar FFT(2nx) of nx non-zero planes, V_dd(k) * scale, nx planes kept
+//   g_y  lines along y, inverse: kinetic FFT(ny); dipolar FFT(2ny), ny rows kept
+//   g_z  rows along z: dipolar C2R (row pairs) -> phi; kinetic inverse; the last half
+//        step of one iteration and the first of the next, or the imaginary-time
+//        Euler step with its norm; rho; kinetic forward; dipolar R2C (row pairs)
+//   g_y  forward
+//
+// (Before: one kernel per axis pass, 12 launches a real-time iteration, one real
+// row per complex line along z, a division per index.)
+//
+// Spectrum of the dipolar convolution: S[i][ky][kz - 1], 1 <= kz <= nz: V_dd is
+// kz^2/k^2, zero on the kz = 0 plane, which is not stored
+// (fftw_poisson_solver.cpp:39-45).
+//
+// A line transform is two (up to 256 points), three or more Stockham stages of
+// radix <= 16 between two shared-memory buffers; the first stage of a line along x or y
+// reads global memory and the last one stores there, so a two-stage transform crosses shared
+// memory once.  All transforms run forward: an inverse one swaps re and im at both ends.
+// Twiddles are those of plan.hpp, in complex64 hi + lo (compensated).
+#pragma once
+
+#include "kernels.cuh"
+
+namespace gpe {
+
+template <class R> struct GTwid;
+template <> struct GTwid<float> { using T = float4; };   // hi.re, hi.im, lo.re, lo.im
+template <> struct GTwid<double> { using T = double2; };
+__device__ __forceinline__ float2 g_twmul(float2 v, float4 w) {
+    return twmul<-1>(v, float2{w.x, w.y}, float2{w.z, w.w});
+}
+__device__ __forceinline__ double2 g_twmul(double2 v, double2 w) { return cmul(v, w); }
+template <class C> __device__ __forceinline__ C g_swap(C v, bool s) { return s ? C{v.y, v.x} : v; }
+
+constexpr int kGStages = 6;
+struct GStage {
+    int r, ns, nr, step; // radix, product of the radices before, L / r, L / (ns r)
+    unsigned m;          // ceil(2^32 / ns): j / ns = umulhi(j, m) for ns > 1
+};
+struct GPlan {
+    int L, n;
+    GStage f[kGStages]; // radices in order
+    GStage v[kGStages]; // in reverse order (the inverse along x)
+    const void *tw;     // GTwid<R>::T[L], exp(-2 pi i m / L)
+};
+
+__device__ __forceinline__ int g_div(int x, int d, unsigned m) { return d == 1 ? x : (int)__umulhi((unsigned)x, m); }
+
+#define GPE_RADICES(M) M(1) M(2) M(3) M(4) M(5) M(6) M(7) M(8) M(9) M(10) M(12) M(14) M(15) M(16)
+
+// Inputs of item j (line b) of a stage, twiddled, from the tile: element t of line
+// b at s[t TS + b]; elements from nin on are zero and not read.
+template <int RAD, class R>
+__device__ __forceinline__ void g_load(cplx<R> (&a)[RAD], const cplx<R> *s, const GStage &st, int jm, int j, int b,
+                                       int TS, int nin, const void *tw) {
+    using T     = typename GTwid<R>::T;
+    const T *tb = reinterpret_cast<const T *>(tw);
+#pragma unroll
+    for (int k = 0; k < RAD; ++k) {
+        const int t = j + k * st.nr;
+        a[k]        = t < nin ? s[t * TS + b] : cplx<R>{(R)0, (R)0};
+    }
+    if (st.ns > 1) {
+        const int t0 = jm * st.step;
+#pragma unroll
+        for (int k = 1; k < RAD; ++k)
+            a[k] = g_twmul(a[k], __ldg(&tb[t0 * k]));
+    }
+}
+
+// One stage from tile src to tile dst (offsets in g_smem, complex elements) of
+// 2^lb lines of stride 1 and element stride TS.
+template <int RAD, class R>
+__device__ __forceinline__ void g_mid_r(const GStage &st, const void *tw, unsigned src, unsigned dst, int lb, int TS,
+                                        int nin, int tid, int nt) {
+    using C         = cplx<R>;
+    C *sm           = reinterpret_cast<C *>(g_smem);
+    const int items = st.nr << lb;
+    for (int it = tid; it < items; it += nt) {
+        const int b = it & ((1 << lb) - 1), j = it >> lb;
+        const int d = g_div(j, st.ns, st.m), jm = j - d * st.ns;
+        C a[RAD];
+        g_load<RAD, R>(a, sm + src, st, jm, j, b, TS, nin, tw);
+        DFT<RAD, -1, R>::run(a);
+        C *o = sm + dst + (d * st.ns * RAD + jm) * TS + b;
+#pragma unroll
+        for (int q = 0; q < RAD; ++q)
+            o[q * st.ns * TS] = a[q];
+    }
+}
+template <class R>
+__device__ __noinline__ void g_mid(GStage st, const void *tw, unsigned src, unsigned dst, int lb, int TS, int nin,
+                                   int tid, int nt) {
+    switch (st.r) {
+#define GPE_M(N)                                                                                   \
+    case N: g_mid_r<N, R>(st, tw, src, dst, lb, TS, nin, tid, nt); break;
+        GPE_RADICES(GPE_M)
+#undef GPE_M
+    }
+}
+
+// First stage: the lines' columns from global memory (element t of line b at
+// p[t rs + b], t < nin, b < cnt; the rest is zero) into the tile at dst.
+template <int RAD, class R>
+__device__ __forceinline__ void g_first_r(const GStage &st, const cplx<R> *__restrict__ p, size_t rs, int nin, int cnt,
+                                          bool swap, unsigned dst, int lb, int TS, int tid, int nt) {
+    using C         = cplx<R>;
+    C *sm           = reinterpret_cast<C *>(g_smem) + dst;
+    const int items = st.nr << lb;
+    for (int it = tid; it < items; it += nt) {
+        const int b = it & ((1 << lb) - 1), j = it >> lb;
+        C a[RAD];
+#pragma unroll
+        for (int k = 0; k < RAD; ++k) {
+            const int t = j + k * st.nr;
+            a[k]        = t < nin && b < cnt ? p[(size_t)t * rs + b] : C{(R)0, (R)0};
+        }
+#pragma unroll
+        for (int k = 0; k < RAD; ++k)
+            a[k] = g_swap(a[k], swap);
+        DFT<RAD, -1, R>::run(a);
+#pragma unroll
+        for (int q = 0; q < RAD; ++q)
+            sm[(j * RAD + q) * TS + b] = a[q];
+    }
+}
+// Last stage: from the tile at src to global memory, elements t < nout.
+template <int RAD, class R>
+__device__ __forceinline__ void g_last_r(const GStage &st, const void *tw, cplx<R> *__restrict__ p, size_t rs, int nout,
+                                         int cnt, bool swap, unsigned src, int lb, int TS, int tid, int nt) {
+    using C         = cplx<R>;
+    const C *sm     = reinterpret_cast<const C *>(g_smem) + src;
+    const int items = st.nr << lb;
+    for (int it = tid; it < items; it += nt) {
+        const int b = it & ((1 << lb) - 1), j = it >> lb;
+        C a[RAD];
+        g_load<RAD, R>(a, sm, st, j, j, b, TS, st.nr * RAD, tw);
+        DFT<RAD, -1, R>::run(a);
+#pragma unroll
+        for (int q = 0; q < RAD; ++q) {
+            const int t = j + q * st.nr;
+            if (t < nout && b < cnt)
+                p[(size_t)t * rs + b] = g_swap(a[q], swap);
+        }
+    }
+}
+
+// Whole transform of the columns p -> p.  buf: two tiles of `ts` elements each at
+// 0 and ts; the second one only for three stages and more.
+template <class R>
+__device__ __forceinline__ void g_lines(const GPlan &pl, cplx<R> *p, size_t rs, int nin, int nout, int cnt, bool swap,
+                                        int lb, int tid, int nt) {
+    using C       = cplx<R>;
+    const int TS  = 1 << lb;
+    unsigned cur  = 0, oth = (unsigned)(pl.L * TS);
+    switch (pl.f[0].r) {
+#define GPE_M(N)                                                                                   \
+    case N: g_first_r<N, R>(pl.f[0], p, rs, nin, cnt, swap, cur, lb, TS, tid, nt); break;
+        GPE_RADICES(GPE_M)
+#undef GPE_M
+    }
+    __syncthreads();
+    for (int s = 1; s < pl.n - 1; ++s) {
+        g_mid<R>(pl.f[s], pl.tw, cur, oth, lb, TS, pl.L, tid, nt);
+        __syncthreads();
+        const unsigned t = cur;
+        cur = oth, oth = t;
+    }
+    if (pl.n == 1) { // the first stage was the whole line
+        const C *sm = reinterpret_cast<const C *>(g_smem);
+        for (int e = tid; e < nout << lb; e += nt) {
+            const int b = e & (TS - 1), t = e >> lb;
+            if (b < cnt)
+                p[(size_t)t * rs + b] = g_swap(sm[e], swap);
+        }
+        return;
+    }
+    switch (pl.f[pl.n - 1].r) {
+#define GPE_M(N)                                                                                   \
+    case N: g_last_r<N, R>(pl.f[pl.n - 1], pl.tw, p, rs, nout, cnt, swap, cur, lb, TS, tid, nt); break;
+        GPE_RADICES(GPE_M)
+#undef GPE_M
+    }
+}
+
+// ---------------------------------------------------------------------------
+// y lines: one x plane per blockIdx.y, tiles of 2^lb z columns along blockIdx.x,
+// first the kinetic ones (tk), then the dipolar ones
+// ---------------------------------------------------------------------------
+struct GYArgs {
+    void *psi, *S;
+    int ny, nz, tk, inverse;
+    int lb;
+    GPlan k, d;
+};
+template <class R> __global__ void __launch_bounds__(256, 2) g_y(const __grid_constant__ GYArgs a) {
+    using C        = cplx<R>;
+    const bool kin = (int)blockIdx.x < a.tk;
+    const int k0   = (kin ? blockIdx.x : blockIdx.x - a.tk) << a.lb;
+    const int cnt  = min(1 << a.lb, a.nz - k0);
+    const size_t plane = (size_t)blockIdx.y * a.ny * a.nz;
+    C *p = kin ? reinterpret_cast<C *>(a.psi) + plane + k0 : reinterpret_cast<C *>(a.S) + 2 * plane + k0;
+    const int nin  = kin || !a.inverse ? a.ny : 2 * a.ny;
+    const int nout = kin || a.inverse ? a.ny : 2 * a.ny;
+    g_lines<R>(kin ? a.k : a.d, p, a.nz, nin, nout, cnt, a.inverse, a.lb, threadIdx.x, blockDim.x);
+}
+
+// ---------------------------------------------------------------------------
+// x lines: forward, factor, inverse; tiles of 2^lb (y, z) columns, the kinetic
+// ones first
+// ---------------------------------------------------------------------------
+struct GXArgs {
+    void *psi, *S;
+    const void *ex, *ey, *ez;     // exp(i theta) - 1 per axis (kinetic)
+    double inv;                   // 1 / N
+    const void *vk;               // V_dd(|kx|, |ky|, kz), kz = 1..nz
+    const double *divisor;        // norm the spectrum is still to be divided by, or null
+    double dip_scale;
+    int nx, ny, nz, tk, lb;
+    GPlan k, d;
+};
+
+// The forward transform's last stage, the factor and the inverse's first stage
+// (radices reversed: it reads exactly the outputs the item holds).
+template <int RAD, class R>
+__device__ __forceinline__ void g_xmid_r(const GXArgs &a, const GPlan &pl, bool kin, int c0, int cnt, R scale,
+                                         unsigned src, unsigned dst, int tid, int nt) {
+    using C         = cplx<R>;
+    C *sm           = reinterpret_cast<C *>(g_smem);
+    const GStage st = pl.f[pl.n - 1];
+    const int TS = 1 << a.lb, items = st.nr << a.lb;
+    for (int it = tid; it < items; it += nt) {
+        const int b = it & (TS - 1), j = it >> a.lb;
+        const int c = c0 + min(b, cnt - 1), y = c / a.nz, z = c - y * a.nz;
+        C v[RAD];
+        g_load<RAD, R>(v, sm + src, st, j, j, b, TS, pl.L, pl.tw);
+        C in[sizeof(R) == 4 ? RAD : 1];
+        if constexpr (sizeof(R) == 4)
+#pragma unroll
+            for (int q = 0; q < RAD; ++q)
+                in[q] = v[q];
+        DFT<RAD, -1, R>::run(v);
+        if (kin) {
+            const C *ex = reinterpret_cast<const C *>(a.ex);
+            const C wy = __ldg(reinterpret_cast<const C *>(a.ey) + y), wz = __ldg(reinterpret_cast<const C *>(a.ez) + z);
+            const C wyz = cadd(cadd(wy, wz), cmul(wy, wz)); // (1+wy)(1+wz) - 1
+            const R ih  = (R)a.inv;
+#pragma unroll
+            for (int q = 0; q < RAD; ++q) {
+                const C wx = __ldg(&ex[j + q * st.nr]);
+                const C w  = cadd(cadd(wx, wyz), cmul(wx, wyz)); // exp(i theta) - 1
+                const C u  = sizeof(R) == 4 ? cmul(v[q], w) : apply_wm1(v[q], w);
+                v[q]       = C{u.y * ih, u.x * ih}; // swapped: inverse
+            }
+        } else {
+            const int iy = y <= a.ny ? y : 2 * a.ny - y;
+            const R *vk  = reinterpret_cast<const R *>(a.vk) + (size_t)iy * a.nz + z;
+            const size_t xs = (size_t)(a.ny + 1) * a.nz;
+#pragma unroll
+            for (int q = 0; q < RAD; ++q) {
+                const int t = j + q * st.nr, ix = t <= a.nx ? t : pl.L - t;
+                const R f   = __ldg(&vk[ix * xs]) * scale;
+                v[q]        = C{v[q].y * f, v[q].x * f};
+            }
+        }
+        DFT<RAD, -1, R>::run(v);
+        // complex64: the transform pair carries the kinetic factor's change of psi,
+        // exp(i theta) - 1, and psi itself, RAD / N times the pair's inputs, is added
+        // here.  Their rounding then scales with |theta|: done directly, the sums in
+        // this most concentrated space (few populated k) drift the norm the most.
+        if constexpr (sizeof(R) == 4)
+            if (kin) {
+                const double f = a.inv * RAD;
+                const R fh = (R)f, fl = (R)(f - (double)fh);
+#pragma unroll
+                for (int q = 0; q < RAD; ++q)
+                    v[q] = C{fma(in[q].y, fh, fma(in[q].y, fl, v[q].x)), fma(in[q].x, fh, fma(in[q].x, fl, v[q].y))};
+            }
+#pragma unroll
+        for (int q = 0; q < RAD; ++q)
+            sm[dst + (j * RAD + q) * TS + b] = v[q];
+    }
+}
+
+template <class R> __global__ void __launch_bounds__(256, 2) g_x(const __grid_constant__ GXArgs a) {
+    using C         = cplx<R>;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const bool kin  = (int)blockIdx.x < a.tk;
+    const GPlan &pl = kin ? a.k : a.d;
+    const int cols  = (kin ? 1 : 2) * a.ny * a.nz;
+    const int c0    = (kin ? blockIdx.x : blockIdx.x - a.tk) << a.lb;
+    const int cnt   = min(1 << a.lb, cols - c0);
+    C *p            = (kin ? reinterpret_cast<C *>(a.psi) : reinterpret_cast<C *>(a.S)) + c0;
+    const int TS    = 1 << a.lb;
+    const R scale   = (R)(a.divisor && !kin ? a.dip_scale / a.divisor[0] : a.dip_scale);
+    unsigned cur = 0, oth = (unsigned)(pl.L * TS);
+    auto flip = [&] {
+        __syncthreads();
+        const unsigned t = cur;
+        cur = oth, oth = t;
+    };
+    if (pl.n == 1) { // one stage: the columns as they are
+        C *sm = reinterpret_cast<C *>(g_smem);
+        for (int e = tid; e < pl.L << a.lb; e += nt) {
+            const int b = e & (TS - 1), t = e >> a.lb;
+            sm[oth + e] = t < a.nx && b < cnt ? p[(size_t)t * cols + b] : C{(R)0, (R)0};
+        }
+    } else {
+        switch (pl.f[0].r) {
+#define GPE_M(N)                                                                                   \
+    case N: g_first_r<N, R>(pl.f[0], p, cols, a.nx, cnt, false, oth, a.lb, TS, tid, nt); break;
+            GPE_RADICES(GPE_M)
+#undef GPE_M
+        }
+    }
+    flip();
+    for (int s = 1; s < pl.n - 1; ++s) {
+        g_mid<R>(pl.f[s], pl.tw, cur, oth, a.lb, TS, pl.L, tid, nt);
+        flip();
+    }
+    switch (pl.f[pl.n - 1].r) {
+#define GPE_M(N)                                                                                   \
+    case N: g_xmid_r<N, R>(a, pl, kin, c0, cnt, scale, cur, oth, tid, nt); break;
+        GPE_RADICES(GPE_M)
+#undef GPE_M
+    }
+    flip();
+    for (int s = 1; s < pl.n - 1; ++s) {
+        g_mid<R>(pl.v[s], pl.tw, cur, oth, a.lb, TS, pl.L, tid, nt);
+        flip();
+    }
+    if (pl.n == 1) {
+        const C *sm = reinterpret_cast<const C *>(g_smem) + cur;
+        for (int e = tid; e < a.nx << a.lb; e += nt) {
+            const int b = e & (TS - 1), t = e >> a.lb;
+            if (b < cnt)
+                p[(size_t)t * cols + b] = g_swap(sm[e], true);
+        }
+        return;
+    }
+    switch (pl.v[pl.n - 1].r) {
+#define GPE_M(N)                                                                                   \
+    case N: g_last_r<N, R>(pl.v[pl.n - 1], pl.tw, p, cols, a.nx, cnt, true, cur, a.lb, TS, tid, nt); break;
+        GPE_RADICES(GPE_M)
+#undef GPE_M
+    }
+}
+
+// ---------------------------------------------------------------------------
+// z rows
+// ---------------------------------------------------------------------------
+enum {
+    GZ_RT_PRO = 0, // first half step of a call, forward
+    GZ_RT_MID,     // inverse, both half steps, forward
+    GZ_RT_EPI,     // inverse, last half step; psi and phi stored
+    GZ_IT_PRO,     // rho of psi, forward
+    GZ_IT_MID,     // dipolar inverse, Euler step and norm, forward
+    GZ_DIP_INV,    // spectrum -> phi
+    GZ_KIN_FWD, GZ_KIN_INV,
+    GZ_PHASE,      // one half step, psi and phi in memory
+    GZ_IT_STEP,    // the Euler step alone, phi in memory
+    GZ_NORM,       // the norm alone
+    GZ_MODES
+};
+// The interface's single steps (GZ_DIP_INV and after) run the same code on the same
+// rows as the iterations, so both sequences agree to the last bits.
+
+// The pointwise arithmetic with its roundings written out: the compiler then contracts
+// it alike in every mode of g_z, and the iterations and the single steps agree to the
+// last bits.
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+template <class C> __device__ __forceinline__ auto g_abs2(C v) { return fma(v.x, v.x, mul_rn(v.y, v.y)); }
+
+// Potential half step (cpu_solver.cpp:99-131):
+//   v exp(i theta), theta = -dt/2 [V + cdd phi + g3 |v|^2 + gw |v|^3],
+// applied as v + v (exp(i theta) - 1), exp(i theta) - 1 = (-2 sin^2(theta/2), sin theta)
+template <class R>
+__device__ __forceinline__ cplx<R> g_turn(cplx<R> v, R V, R phi, R cdd, R hdt, R g3, R gw) {
+    const R dens  = g_abs2(v), am = sqrt(dens);
+    const R total = add_rn(fma(cdd, phi, V), fma(g3, dens, mul_rn(gw, mul_rn(mul_rn(am, am), am))));
+    R s, c;
+    sincos_r<R>(mul_rn(mul_rn((R)-0.5, hdt), total), &s, &c);
+    const R wx = mul_rn(mul_rn((R)-2, s), s), wy = mul_rn(mul_rn((R)2, s), c);
+    return cplx<R>{add_rn(v.x, fma(v.x, wx, -mul_rn(v.y, wy))), add_rn(v.y, fma(v.x, wy, mul_rn(v.y, wx)))};
+}
+
+struct GZArgs {
+    ZArgs z;
+    int write_phi, nz, lb; // 2^lb rows per CTA
+    unsigned mz;           // ceil(2^32 / nz)
+    unsigned buf;          // elements of one of the three tile buffers
+    GPlan k, d;
+};
+
+// All stages of the 2^lb lines in the tile at `cur`; returns with the result there.
+template <class R>
+__device__ __forceinline__ void g_tile(const GPlan &pl, unsigned &cur, unsigned &scr, int lb, int TS, int nin, int tid,
+                                       int nt) {
+    for (int s = 0; s < pl.n; ++s) {
+        g_mid<R>(pl.f[s], pl.tw, cur, scr, lb, TS, s == 0 ? nin : pl.L, tid, nt);
+        __syncthreads();
+        const unsigned t = cur;
+        cur = scr, scr = t;
+    }
+}
+
+template <class R, int MODE> __global__ void __launch_bounds__(256, 2) g_z(const __grid_constant__ GZArgs g) {
+    using C            = cplx<R>;
+    constexpr bool RT  = MODE <= GZ_RT_EPI || MODE == GZ_PHASE;
+    constexpr bool IT  = MODE == GZ_IT_MID || MODE == GZ_IT_STEP;
+    constexpr bool KIN_I = MODE == GZ_RT_MID || MODE == GZ_RT_EPI || MODE == GZ_KIN_INV;
+    constexpr bool KIN_F = MODE == GZ_RT_PRO || MODE == GZ_RT_MID || MODE == GZ_KIN_FWD;
+    constexpr bool DIP_I = MODE == GZ_RT_MID || MODE == GZ_RT_EPI || MODE == GZ_IT_MID || MODE == GZ_DIP_INV;
+    constexpr bool DIP_F = MODE == GZ_RT_PRO || MODE == GZ_RT_MID || MODE == GZ_IT_PRO || MODE == GZ_IT_MID;
+    const ZArgs &a = g.z;
+    const int tid = threadIdx.x, nt = blockDim.x, nz = g.nz, nx = a.nx, ny = a.ny;
+    const int RW = 1 << g.lb, lp = g.lb > 0 ? g.lb - 1 : 0, NP = 1 << lp; // rows, row pairs
+    const int TK = RW >= 4 ? RW + 1 : RW, TD = NP >= 2 ? NP + 1 : NP;     // odd tile strides
+    const int rows = nx * ny, r0 = blockIdx.x << g.lb, cnt = min(RW, rows - r0);
+    C *sm       = reinterpret_cast<C *>(g_smem);
+    unsigned K = 0, D = g.buf, T = 2 * g.buf; // kinetic rows, dipolar pair lines, scratch
+    const size_t base = (size_t)r0 * nz;
+    C *psi      = reinterpret_cast<C *>(a.psi_in) + base;
+    C *out      = reinterpret_cast<C *>(a.psi_out) + base;
+    C *S        = reinterpret_cast<C *>(a.S);
+    R *phi      = reinterpret_cast<R *>(a.phi) + base;
+    const R *V  = reinterpret_cast<const R *>(a.V) + base;
+    const int i0 = r0 / ny, j0 = r0 - i0 * ny;
+    // x plane and y of the tile's row
+    auto place = [&](int row, int &i, int &j) {
+        i = i0;
+        j = j0 + row;
+        while (j >= ny) {
+            j -= ny;
+            ++i;
+        }
+    };
+
+    R g3 = (R)0, gw = (R)0, g3n = (R)0, gwn = (R)0; // this iteration's, the next one's
+    if (RT) {
+        const int it      = *a.step.base + a.step.local;
+        const StepCoef c0 = a.step.coef[it];
+        g3 = (R)c0.g3w;
+        gw = (R)c0.gw15;
+        if (MODE == GZ_RT_MID) {
+            const StepCoef c1 = a.step.coef[it + 1];
+            g3n = (R)c1.g3w;
+            gwn = (R)c1.gw15;
+        }
+    } else if (IT) {
+        g3 = (R)a.step.coef[0].g3w;
+        gw = (R)a.step.coef[0].gw15;
+    }
+
+    // ---- in: psi rows (inverse: swapped) and the pair lines of the spectrum ----
+    if (KIN_I || MODE == GZ_KIN_FWD) {
+        for (int e = tid; e < cnt * nz; e += nt) {
+            const int row = g_div(e, nz, g.mz), k = e - row * nz;
+            sm[K + k * TK + row] = g_swap(psi[e], KIN_I);
+        }
+        for (int e = cnt * nz + tid; e < RW * nz; e += nt) {
+            const int row = g_div(e, nz, g.mz), k = e - row * nz;
+            sm[K + k * TK + row] = C{(R)0, (R)0};
+        }
+    }
+    if (DIP_I) {
+        // line z[m] = xa[m] + i xb[m] over the full 2nz-point spectrum: bin 0 is
+        // zero, bins > nz by symmetry; stored swapped (inverse transform)
+        for (int e = tid; e < NP * nz; e += nt) {
+            const int p = g_div(e, nz, g.mz), m = e - p * nz + 1;
+            C xa{(R)0, (R)0}, xb{(R)0, (R)0};
+            int i, j;
+            if (2 * p < cnt) {
+                place(2 * p, i, j);
+                xa = S[((size_t)i * 2 * ny + j) * nz + (m - 1)];
+            }
+            if (2 * p + 1 < cnt) {
+                place(2 * p + 1, i, j);
+                xb = S[((size_t)i * 2 * ny + j) * nz + (m - 1)];
+            }
+            if (m == nz) {
+                sm[D + m * TD + p] = C{xb.x, xa.x}; // self-conjugate bin: real parts only
+                sm[D + p]          = C{(R)0, (R)0};
+            } else {
+                sm[D + m * TD + p]            = C{xa.y + xb.x, xa.x - xb.y};
+                sm[D + (2 * nz - m) * TD + p] = C{xb.x - xa.y, xa.x + xb.y};
+            }
+        }
+    }
+    if (KIN_I || DIP_I || MODE == GZ_KIN_FWD)
+        __syncthreads();
+    if (KIN_I)
+        g_tile<R>(g.k, K, T, g.lb, TK, nz, tid, nt);
+    if (DIP_I)
+        g_tile<R>(g.d, D, T, lp, TD, 2 * nz, tid, nt);
+
+    // ---- the step on row pairs: element k of rows 2p and 2p + 1 ----------------
+    double acc = 0.0;
+    if (MODE == GZ_KIN_INV) {
+        for (int e = tid; e < cnt * nz; e += nt) {
+            const int row = g_div(e, nz, g.mz), k = e - row * nz;
+            out[e]        = g_swap(sm[K + k * TK + row], true);
+        }
+        return;
+    }
+    if (MODE != GZ_KIN_FWD) {
+        const R sc   = (R)(IT ? 1.0 / sqrt(a.norm_state[1]) : 1.0);
+        const R wat  = (R)a.w_atoms;
+        const R hdt = (R)a.half_dt, cdd = (R)a.cdd;
+        const R cx = (R)a.cx, cy = (R)a.cy, cz = (R)a.cz, dtau = (R)a.dtau;
+        const ptrdiff_t plane = (ptrdiff_t)ny * nz;
+        for (int e = tid; e < NP * nz; e += nt) {
+            const int p = g_div(e, nz, g.mz), k = e - p * nz;
+            C z{(R)0, (R)0};
+            if (DIP_I)
+                z = sm[D + k * TD + p]; // swapped: (row 2p + 1, row 2p)
+            R rho[2] = {(R)0, (R)0};
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int row = 2 * p + h;
+                if (row >= cnt)
+                    break;
+                const int q = row * nz + k;
+                R f         = h == 0 ? z.y : z.x;
+                if (MODE == GZ_RT_PRO || MODE == GZ_PHASE || MODE == GZ_IT_STEP)
+                    f = phi[q];
+                if (MODE == GZ_DIP_INV || MODE == GZ_RT_EPI || (MODE == GZ_IT_MID && g.write_phi))
+                    phi[q] = f;
+                if (MODE == GZ_DIP_INV)
+                    continue;
+                int i, j;
+                place(row, i, j);
+                const bool in = i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
+                C v;
+                if (RT) {
+                    v = MODE == GZ_RT_PRO || MODE == GZ_PHASE ? psi[q] : g_swap(sm[K + k * TK + row], true);
+                    if (in) {
+                        v = g_turn<R>(v, V[q], f, cdd, hdt, g3, gw);
+                        if (MODE == GZ_RT_MID) // the next iteration's first half step
+                            v = g_turn<R>(v, V[q], f, cdd, hdt, g3n, gwn);
+                    }
+                    if (MODE == GZ_RT_EPI || MODE == GZ_PHASE)
+                        out[q] = v;
+                    else
+                        sm[K + k * TK + row] = v;
+                } else if (MODE == GZ_IT_PRO) {
+                    v = psi[q];
+                } else if (MODE == GZ_NORM) {
+                    v = psi[q];
+                    acc = add_rn(acc, g_abs2(double2{(double)v.x, (double)v.y}));
+                } else { // the Euler step of psi_in / sqrt(divisor)
+                    if (!in) {
+                        v = reinterpret_cast<const C *>(a.bnd)[base + q];
+                    } else {
+                        const C c0 = cscale(psi[q], sc);
+                        const C xm = cscale(psi[q - plane], sc), xp = cscale(psi[q + plane], sc);
+                        const C ym = cscale(psi[q - nz], sc), yp = cscale(psi[q + nz], sc);
+                        const C zm = cscale(psi[q - 1], sc), zp = cscale(psi[q + 1], sc);
+                        const R dens = g_abs2(c0), am = sqrt(dens);
+                        const R h    = add_rn(fma(cdd, f, V[q]), fma(g3, dens, mul_rn(gw, mul_rn(mul_rn(am, am), am))));
+                        auto step    = [&](R c, R xa, R xb, R ya, R yb, R za, R zb) {
+                            const R dx = fma((R)-2, c, add_rn(xa, xb)), dy = fma((R)-2, c, add_rn(ya, yb)),
+                                    dz = fma((R)-2, c, add_rn(za, zb));
+                            return fma(-dtau, fma(cx, dx, fma(-cy, dy, fma(-cz, dz, mul_rn(c, h)))), c);
+                        };
+                        v = C{step(c0.x, xm.x, xp.x, ym.x, yp.x, zm.x, zp.x),
+                              step(c0.y, xm.y, xp.y, ym.y, yp.y, zm.y, zp.y)};
+                    }
+                    out[q] = v;
+                    if (MODE == GZ_IT_MID)
+                        acc = add_rn(acc, g_abs2(double2{(double)v.x, (double)v.y}));
+                }
+                rho[h] = mul_rn(wat, g_abs2(v));
+            }
+            if (DIP_F)
+                sm[D + k * TD + p] = C{rho[0], rho[1]};
+        }
+        if (!DIP_F && MODE != GZ_NORM)
+            return;
+        if (KIN_F) // rows beyond the grid's last
+            for (int e = cnt * nz + tid; e < RW * nz; e += nt) {
+                const int row = g_div(e, nz, g.mz), k = e - row * nz;
+                sm[K + k * TK + row] = C{(R)0, (R)0};
+            }
+        if (MODE != GZ_NORM)
+            __syncthreads();
+    }
+
+    // ---- out: kinetic spectrum, then bins 1..nz of the row pairs -----------------
+    if (KIN_F) {
+        g_tile<R>(g.k, K, T, g.lb, TK, nz, tid, nt);
+        for (int e = tid; e < cnt * nz; e += nt) {
+            const int row = g_div(e, nz, g.mz), k = e - row * nz;
+            out[e]        = sm[K + k * TK + row];
+        }
+    }
+    if (DIP_F) {
+        g_tile<R>(g.d, D, T, lp, TD, nz, tid, nt); // the padding half is not read
+        for (int e = tid; e < NP * nz; e += nt) {
+            const int p = g_div(e, nz, g.mz), m = e - p * nz + 1;
+            const C zm = sm[D + m * TD + p], zc = sm[D + (2 * nz - m) * TD + p];
+            int i, j;
+            if (2 * p < cnt) { // (Z_m + conj(Z_{L-m}))/2
+                place(2 * p, i, j);
+                S[((size_t)i * 2 * ny + j) * nz + (m - 1)] = C{(R)0.5 * (zm.x + zc.x), (R)0.5 * (zm.y - zc.y)};
+            }
+            if (2 * p + 1 < cnt) { // (Z_m - conj(Z_{L-m}))/(2i)
+                place(2 * p + 1, i, j);
+                S[((size_t)i * 2 * ny + j) * nz + (m - 1)] = C{(R)0.5 * (zm.y + zc.y), (R)0.5 * (zc.x - zm.x)};
+            }
+        }
+    }
+
+    // ---- norm of psi' (imaginary time): deterministic two-level reduction --------
+    if (MODE == GZ_IT_MID || MODE == GZ_NORM)
+        norm_by_last_block(acc, a);
+}
+
+} // namespace gpe

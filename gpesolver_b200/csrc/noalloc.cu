@@ -25,8 +25,7 @@
 //    kernels' shared-memory limit to the device's opt-in maximum); make that
 //    first call before any stream capture on that device.
 #include "../../include/gpe_b200.h"
-#include "kernels.cuh"
-#include "plan.hpp"
+#include "general_plan.hpp"
 
 #include <cuda_runtime.h>
 
@@ -52,27 +51,30 @@ NoallocSlot g_noalloc_slots[kMaxDevices];
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// exp(-2 pi i m / L) in FP64, rounded to float2 (tw) with the rounding
-// remainder in twlo (the FFT stages multiply by tw + twlo, compensated).
-__global__ void k_na_twiddles(float2 *tw, float2 *twlo, int L) {
-    for (int m = blockIdx.x * blockDim.x + threadIdx.x; m < L; m += gridDim.x * blockDim.x) {
-        double s, c;
-        sincospi(2.0 * (double)m / (double)L, &s, &c);
-        const float ch = (float)c, sh = (float)-s;
-        tw[m]          = make_float2(ch, sh);
-        twlo[m]        = make_float2((float)(c - (double)ch), (float)(-s - (double)sh));
-    }
-}
-
-// V_dd(k) = kz^2 / k^2 on the (2nx, 2ny, 2nz) box, reduced by |kx|, |ky| symmetry
+// The tables of a grid in one launch: twiddles exp(-2 pi i m / L) of the three
+// doubled axes (FP64, hi rounded to float and lo the rounding remainder) and V_dd(k) =
+// kz^2 / k^2 on the (2nx, 2ny, 2nz) box for kz = 1..nz, reduced by |kx|, |ky| symmetry
 // (fftw_poisson_solver.cpp:12-49), FP64 then rounded to float.
-__global__ void k_na_vdip(float *vk, int nx, int ny, int nz, double dx, double dy, double dz) {
-    const int H = nz + 1, px = 2 * nx, py = 2 * ny, pz = 2 * nz;
+__global__ void k_na_tables(float4 *twx, float4 *twy, float4 *twz, float *vk, int nx, int ny, int nz, double dx,
+                            double dy, double dz) {
+    const int first = blockIdx.x * blockDim.x + threadIdx.x, step = gridDim.x * blockDim.x;
+    auto tw = [&](float4 *t, int L) {
+        for (int m = first; m < L; m += step) {
+            double s, c;
+            sincospi(2.0 * (double)m / (double)L, &s, &c);
+            const float ch = (float)c, sh = (float)-s;
+            t[m]           = make_float4(ch, sh, (float)(c - (double)ch), (float)(-s - (double)sh));
+        }
+    };
+    tw(twx, 2 * nx);
+    tw(twy, 2 * ny);
+    tw(twz, 2 * nz);
+    const int px = 2 * nx, py = 2 * ny, pz = 2 * nz;
     const double dkx = 2. * M_PI / (px * dx), dky = 2. * M_PI / (py * dy), dkz = 2. * M_PI / (pz * dz);
-    const size_t total = (size_t)(nx + 1) * (ny + 1) * H;
-    for (size_t q = blockIdx.x * (size_t)blockDim.x + threadIdx.x; q < total;
-         q += (size_t)gridDim.x * blockDim.x) {
-        const int k = (int)(q % H), j = (int)((q / H) % (ny + 1)), i = (int)(q / ((size_t)H * (ny + 1)));
+    const size_t total = (size_t)(nx + 1) * (ny + 1) * nz;
+    for (size_t q = first; q < total; q += step) {
+        const unsigned r = (unsigned)(q / nz);
+        const int k = (int)(q - (size_t)r * nz) + 1, i = (int)(r / (ny + 1)), j = (int)(r - (unsigned)i * (ny + 1));
         const double kx = i * dkx, ky = j * dky, kz = k * dkz;
         const double k2 = __dadd_rn(__dadd_rn(__dmul_rn(kx, kx), __dmul_rn(ky, ky)), __dmul_rn(kz, kz));
         vk[q]           = (k2 > 1e-30) ? (float)__ddiv_rn(__dmul_rn(kz, kz), k2) : 0.0f;
@@ -109,17 +111,6 @@ int tile_for(int L, int pad) {
     return TB;
 }
 
-LinePlan line(int L, const float2 *tw) {
-    LinePlan p{};
-    std::vector<int> r = factor_line(L);
-    p.L                = L;
-    p.nstages          = (int)r.size();
-    for (size_t s = 0; s < r.size(); ++s)
-        p.radix[s] = r[s];
-    p.tw = tw;
-    return p;
-}
-
 int fail(int code, const std::string &msg) {
     last_error() = msg;
     return code;
@@ -143,11 +134,15 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
                                       std::to_string(lay.total) + " bytes of scratch, above the " +
                                       std::to_string((size_t)GPE_NOALLOC_SCRATCH_BYTES) +
                                       "-byte limit");
-    LinePlan lx, ly, lz;
+    GPlan lx, ly, lz;
+    GShape sh;
     try {
-        lx = line(2 * nx, nullptr);
-        ly = line(2 * ny, nullptr);
-        lz = line(2 * nz, nullptr);
+        for (int n : {nx, ny, nz})
+            factor_line(2 * n); // rejects unsupported lengths
+        lx = g_plan(2 * nx, nullptr);
+        ly = g_plan(2 * ny, nullptr);
+        lz = g_plan(2 * nz, nullptr);
+        sh = g_shape<float>(nx, ny, nz, false);
     } catch (const Error &e) {
         return fail(e.code, std::string("gpe_calc_fi3d_noalloc: ") + e.what());
     }
@@ -159,6 +154,7 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
         return fail(GPE_ERR_ARG, "gpe_calc_fi3d_noalloc: device ordinal out of range");
     cudaStream_t s = (cudaStream_t)cuda_stream;
     const int TBx = tile_for(lx.L, 0), TBy = tile_for(ly.L, 0), TBz = tile_for(lz.L, 1);
+    // the limits on line lengths
     const size_t smx = 2 * sizeof(float2) * (size_t)TBx * lx.L;
     const size_t smy = 2 * sizeof(float2) * (size_t)TBy * ly.L;
     const size_t smz = 2 * sizeof(float2) * (size_t)(TBz + 1) * lz.L; // z tiles: odd stride TB + 1
@@ -177,11 +173,14 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
             err       = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
             if (err != cudaSuccess)
                 return fail(GPE_ERR_CUDA, std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(err));
-            const void *kern[] = {(const void *)k_dip_z_fwd<float>, (const void *)k_dip_y<-1, float>,
-                                  (const void *)k_dip_y<+1, float>, (const void *)k_dip_x<float>,
-                                  (const void *)k_dip_z_inv<float>};
+            const void *kern[] = {(const void *)g_z<float, GZ_IT_PRO>, (const void *)g_y<float>,
+                                  (const void *)g_x<float>, (const void *)g_z<float, GZ_DIP_INV>};
             for (const void *f : kern) {
-                err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, optin);
+                cudaFuncAttributes fa{};
+                err = cudaFuncGetAttributes(&fa, f);
+                if (err == cudaSuccess)
+                    err = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               optin - (int)fa.sharedSizeBytes);
                 if (err != cudaSuccess)
                     return fail(GPE_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(err));
             }
@@ -190,7 +189,8 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
             slot.ready    = true;
         }
     }
-    if (smx > slot.smem_max || smy > slot.smem_max || smz > slot.smem_max)
+    const size_t most = std::max({smx, smy, smz, sh.smx, sh.smy, sh.smz});
+    if (most > slot.smem_max)
         return fail(GPE_ERR_SIZE, "gpe_calc_fi3d_noalloc: the line tiles of this grid need more shared memory "
                                   "than the device allows per block");
     // An error left by earlier, unrelated work would be reported as this call's:
@@ -200,36 +200,39 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
         return fail(GPE_ERR_CUDA, std::string("gpe_calc_fi3d_noalloc: a CUDA error from earlier work is pending: ") +
                                       cudaGetErrorString(err));
     unsigned char *base = slot.base;
-    float2 *A           = reinterpret_cast<float2 *>(base + lay.a_off);
+    float2 *S           = reinterpret_cast<float2 *>(base + lay.a_off);
     float *vk           = reinterpret_cast<float *>(base + lay.vk_off);
-    float2 *twx         = reinterpret_cast<float2 *>(base + lay.twx_off);
-    float2 *twy         = reinterpret_cast<float2 *>(base + lay.twy_off);
-    float2 *twz         = reinterpret_cast<float2 *>(base + lay.twz_off);
-    lx.tw               = twx;
-    ly.tw               = twy;
-    lz.tw               = twz;
-    lx.twlo             = twx + 2 * nx;
-    ly.twlo             = twy + 2 * ny;
-    lz.twlo             = twz + 2 * nz;
-    const int H         = nz + 1;
+    float4 *twx         = reinterpret_cast<float4 *>(base + lay.twx_off);
+    float4 *twy         = reinterpret_cast<float4 *>(base + lay.twy_off);
+    float4 *twz         = reinterpret_cast<float4 *>(base + lay.twz_off);
+    lx.tw = twx, ly.tw = twy, lz.tw = twz;
 
     // the tables of this grid, rebuilt by every call (in stream order before the
     // passes that read them)
-    k_na_twiddles<<<(2 * nx + 255) / 256, 256, 0, s>>>(twx, twx + 2 * nx, 2 * nx);
-    k_na_twiddles<<<(2 * ny + 255) / 256, 256, 0, s>>>(twy, twy + 2 * ny, 2 * ny);
-    k_na_twiddles<<<(2 * nz + 255) / 256, 256, 0, s>>>(twz, twz + 2 * nz, 2 * nz);
-    k_na_vdip<<<592, 256, 0, s>>>(vk, nx, ny, nz, dx, dy, dz);
-    // The pruned dipolar convolution: every element of A that a pass reads was
-    // written by the pass before it in this call, so nothing needs clearing.
-    const int lines = nx * ny;
-    const float2 *psi = static_cast<const float2 *>(psi_c64_dev);
-    k_dip_z_fwd<float><<<(lines + TBz - 1) / TBz, 256, smz, s>>>(psi, nullptr, 0, A, nx, ny, nz,
-                                                                 (float)n_atoms, lz, TBz);
-    k_dip_y<-1, float><<<dim3((H + TBy - 1) / TBy, nx), 256, smy, s>>>(A, ny, H, ny, 2 * ny, ly, TBy);
-    k_dip_x<float><<<(2 * ny * H + TBx - 1) / TBx, 256, smx, s>>>(A, vk, nx, ny, H, 1.0f, lx, TBx);
-    k_dip_y<+1, float><<<dim3((H + TBy - 1) / TBy, nx), 256, smy, s>>>(A, ny, H, 2 * ny, ny, ly, TBy);
-    k_dip_z_inv<float><<<(lines + TBz - 1) / TBz, 256, smz, s>>>(
-        A, fi3d_dev, nx, ny, nz, (float)(1.0 / (8.0 * (double)nx * ny * nz)), lz, TBz);
+    k_na_tables<<<592, 256, 0, s>>>(twx, twy, twz, vk, nx, ny, nz, dx, dy, dz);
+    // The pruned dipolar convolution (general.cuh): every element of S that a pass
+    // reads was written by the pass before it in this call, so nothing needs clearing.
+    GZArgs z{};
+    z.z.psi_in  = const_cast<void *>(psi_c64_dev);
+    z.z.S       = S;
+    z.z.phi     = fi3d_dev;
+    z.z.w_atoms = n_atoms;
+    z.z.nx = nx, z.z.ny = ny;
+    z.nz = nz, z.mz = g_magic(nz), z.lb = sh.lbz, z.buf = sh.buf;
+    z.d = lz;
+    GYArgs y{};
+    y.S = S, y.ny = ny, y.nz = nz, y.lb = sh.lby, y.d = ly;
+    GXArgs x{};
+    x.S = S, x.vk = vk, x.dip_scale = 1.0 / (8.0 * (double)nx * ny * nz);
+    x.nx = nx, x.ny = ny, x.nz = nz, x.lb = sh.lbx, x.d = lx;
+    const int wx = 1 << sh.lbx, zt = (nx * ny + (1 << sh.lbz) - 1) >> sh.lbz;
+    const dim3 yt((nz + (1 << sh.lby) - 1) >> sh.lby, nx);
+    g_z<float, GZ_IT_PRO><<<zt, sh.ntz, sh.smz, s>>>(z);
+    g_y<float><<<yt, sh.nty, sh.smy, s>>>(y);
+    g_x<float><<<(2 * ny * nz + wx - 1) / wx, sh.ntx, sh.smx, s>>>(x);
+    y.inverse = 1;
+    g_y<float><<<yt, sh.nty, sh.smy, s>>>(y);
+    g_z<float, GZ_DIP_INV><<<zt, sh.ntz, sh.smz, s>>>(z);
     err = cudaGetLastError();
     if (err != cudaSuccess)
         return fail(GPE_ERR_CUDA, std::string("gpe_calc_fi3d_noalloc launch: ") + cudaGetErrorString(err));

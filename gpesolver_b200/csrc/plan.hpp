@@ -18,7 +18,8 @@ struct Error : std::runtime_error {
     Error(int c, const std::string &m) : std::runtime_error(m), code(c) {}
 };
 
-// Radices of a length-L line: the power-of-two part in as few balanced stages of
+// Radices of a length-L line of the compiled transforms, and the check of every
+// length: the power-of-two part in as few balanced stages of
 // radix <= 16 as possible, then one stage per factor 3, 5 or 7.  Lengths with a
 // prime factor above 7 are rejected (GPE_ERR_SIZE).
 inline std::vector<int> factor_line(int L) {
@@ -60,6 +61,35 @@ inline std::vector<double> twiddles(int L) {
         t[2 * m + 1]   = -std::sin(a);
     }
     return t;
+}
+
+// Radices (2..16, factors 2, 3, 5, 7) of a length for the run-time transforms: as
+// few stages as possible, then the smallest sum (balanced radices), largest first.
+inline std::vector<int> general_radices(int L) {
+    if (L == 1)
+        return {1};
+    static const int cand[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+    std::vector<int> best, cur;
+    int best_sum = 0;
+    auto search = [&](auto &&self, int m, int most, int sum) -> void {
+        if (m == 1) {
+            if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && sum < best_sum)) {
+                best     = cur;
+                best_sum = sum;
+            }
+            return;
+        }
+        if (!best.empty() && cur.size() + 1 > best.size())
+            return;
+        for (int r : cand)
+            if (r <= most && m % r == 0) {
+                cur.push_back(r);
+                self(self, m / r, r, sum + r);
+                cur.pop_back();
+            }
+    };
+    search(search, L, 16, 0);
+    return best;
 }
 
 } // namespace gpe

@@ -7,6 +7,7 @@
 // exported fields).
 #include "../../include/gpe_b200.h"
 #include "fused_yz.cuh"
+#include "general_plan.hpp"
 #include "plane_pair.cuh"
 #include "init.cuh"
 #include "kernels.cuh"
@@ -30,29 +31,6 @@ namespace gpe {
 // ---------------------------------------------------------------------------
 // Non-template kernels
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-    k_norm_finalize(const double *__restrict__ partial, int nparts, double dV,
-                    double *__restrict__ norm_state, int *__restrict__ status) {
-    __shared__ double red[256];
-    double acc = 0.0;
-    for (int t = threadIdx.x; t < nparts; t += blockDim.x)
-        acc += partial[t];
-    red[threadIdx.x] = acc;
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
-            red[threadIdx.x] += red[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        const double x = red[0] * dV;
-        norm_state[0]  = x;
-        norm_state[1]  = x;
-        if (!(x > 0.0) || !isfinite(x))
-            status[0] = 1;
-    }
-}
-
 __global__ void __launch_bounds__(256)
     k_energy_finalize(const double *__restrict__ partial, int nparts, double *__restrict__ out) {
     __shared__ double red[256];
@@ -195,13 +173,11 @@ __global__ void k_amplitude_in(const float *__restrict__ amp, double *__restrict
 template <class R> class Solver final : public SolverBase {
     using C = cplx<R>;
 
-    // A planned line transform plus its launch tile.
+    // A line length: its twiddles apart (compiled transforms) and paired (general.cuh).
     struct Line {
-        LinePlan plan{};
         DevBuf<C> tw, twlo;
-        int TB  = 1;
-        int pad = 0; // z-pass tiles use the odd stride TB + 1
-        size_t smem() const { return 2 * sizeof(C) * (size_t)(TB + pad) * plan.L; }
+        DevBuf<typename GTwid<R>::T> gtw;
+        GPlan plan{};
     };
 
   public:
@@ -216,7 +192,6 @@ template <class R> class Solver final : public SolverBase {
         if ((long long)nx * ny * nz > (1LL << 30))
             throw Error(GPE_ERR_SIZE, "grid larger than 2^30 points");
         N = (size_t)nx * ny * nz;
-        H = nz + 1;
         GPE_CUDA(cudaSetDevice(p.device));
         GPE_CUDA(cudaStreamCreateWithFlags(&own_stream, cudaStreamNonBlocking));
         GPE_CUDA(cudaStreamCreateWithFlags(&cap_stream, cudaStreamNonBlocking));
@@ -225,19 +200,19 @@ template <class R> class Solver final : public SolverBase {
         GPE_CUDA(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
         cur = own_stream;
 
-        plan_line(kz, nz, 16, 1);
-        plan_line(ky, ny, 32, 0);
-        plan_line(kx, nx, 32, 0);
-        plan_line(dz, 2 * nz, 16, 1);
-        plan_line(dy, 2 * ny, 32, 0);
-        plan_line(dx, 2 * nx, 32, 0);
+        plan_line(kz, nz, 1);
+        plan_line(ky, ny, 0);
+        plan_line(kx, nx, 0);
+        plan_line(dz, 2 * nz, 1);
+        plan_line(dy, 2 * ny, 0);
+        plan_line(dx, 2 * nx, 0);
 
         psi.alloc(N);
         psii.alloc(N);
         bnd.alloc(N);
         V.alloc(N);
         phi.alloc(N);
-        A.alloc((size_t)nx * 2 * ny * H);
+        S2.alloc((size_t)nx * 2 * ny * nz);
         staging.alloc(2 * N);
         norm_state.alloc(4);
         status.alloc(4);
@@ -247,26 +222,26 @@ template <class R> class Solver final : public SolverBase {
         eout.alloc(8);
 
         nblk_elem = 148 * 8;
-        partial.alloc(nblk_elem);
         epartial.alloc(5 * (size_t)nblk_elem);
 
         build_tables();
         fused = std::is_same<R, float>::value && p.schedule == 0 && fused_dim_xy(nx) &&
                 fused_dim_xy(ny) && fused_dim_z(nz);
+        shape = g_shape<R>(nx, ny, nz, true);
+        // per-CTA partial norms: one per row tile of the z passes (at least 32 rows a
+        // CTA in k2_z), one per CTA of a plane kernel (2 nx with two CTAs per plane)
+        zpartial.alloc(std::max<size_t>((size_t)((nx * ny + (1 << shape.lbz) - 1) >> shape.lbz),
+                                        std::max<size_t>((size_t)(nx * ny + 31) / 32, (size_t)2 * nx)));
+        ticket.alloc(1);
+        build_vk2();
         if (fused) {
-            S2.alloc((size_t)nx * 2 * ny * nz);
             psir.alloc(N);
             GPE_CUDA(cudaMemsetAsync(psir.p, 0, sizeof(C) * N, cur)); // defined before any RT call
-            // per-CTA partial norms: one per 32 rows (four-kernel z pass), one per
-            // CTA of a plane kernel (2 nx with two CTAs per plane)
-            zpartial.alloc(std::max<size_t>((size_t)(nx * ny + 31) / 32, (size_t)2 * nx));
-            ticket.alloc(1);
-            build_vk2();
         }
         set_coeffs(p.ggp11, p.gamma);
         set_divisor_one();
         GPE_CUDA(cudaStreamSynchronize(cur));
-        set_smem_attrs();
+        set_general_attrs();
         if (fused) {
             set_fused_attrs();
             autotune_x();
@@ -312,7 +287,7 @@ template <class R> class Solver final : public SolverBase {
         GPE_CUDA(cudaMemcpyAsync(psii.p, psi.p, sizeof(C) * N, cudaMemcpyDeviceToDevice, cur));
         GPE_CUDA(cudaMemcpyAsync(bnd.p, psi.p, sizeof(C) * N, cudaMemcpyDeviceToDevice, cur));
         // calc_norm + normalize: the normalisation is held as the lazy divisor.
-        enqueue_norm(cur, psi.p, /*set_divisor=*/true);
+        gen_z<GZ_NORM>(cur, psi.p, psi.p, cur_coef.p, 0, 0);
         lazy = true;
         check_status();
     }
@@ -455,7 +430,9 @@ template <class R> class Solver final : public SolverBase {
     // ---- the reference's virtuals ------------------------------------------
     void calc_fi3d() override { enqueue_dipolar(cur, psi.p); }
 
-    void imag_linear() override { enqueue_it_update(cur, psi.p, psii.p); }
+    // cpu_solver.cpp:50-97, linear and nonlinear part fused: psi' of the interior from
+    // psi / sqrt(divisor), the boundary takes the values last loaded
+    void imag_linear() override { gen_z<GZ_IT_STEP>(cur, psi.p, psii.p, cur_coef.p, 0, 0); }
 
     void imag_nonlinear() override {
         std::swap(psi.p, psii.p);
@@ -468,7 +445,7 @@ template <class R> class Solver final : public SolverBase {
     // and load_psi report them.
     double calc_norm(bool to_host) override {
         materialize();
-        enqueue_norm(cur, psi.p, /*set_divisor=*/false);
+        gen_z<GZ_NORM>(cur, psi.p, psi.p, cur_coef.p, 0, 0);
         set_divisor_one();
         if (!to_host)
             return 0.0;
@@ -488,7 +465,7 @@ template <class R> class Solver final : public SolverBase {
 
     void potential_half_step() override {
         materialize();
-        enqueue_phase(cur, cur_coef.p, iter_zero.p, 0);
+        gen_z<GZ_PHASE>(cur, psi.p, psi.p, cur_coef.p, 0, 0, iter_zero.p);
     }
 
     void kinetic_step() override {
@@ -530,18 +507,8 @@ template <class R> class Solver final : public SolverBase {
         for (int c = 0; c < checks; ++c) {
             if (!lazy)
                 set_divisor_one();
-            if (fused) {
-                // the energy kernels between checks only read psi: one prologue
-                fused_imag(k, c == 0);
-            } else {
-                long done = 0;
-                while (k - done >= kItChunk) {
-                    run_graph(0, kItChunk);
-                    done += kItChunk;
-                }
-                if (k - done > 0)
-                    run_graph(0, (int)(k - done));
-            }
+            // the energy kernels between checks only read psi: one prologue
+            fused_imag(k, c == 0);
             lazy = true;
             launch(k_energy_partial<R>, nb, 256, 0, cur, (const C *)psi.p, (const R *)V.p, (const R *)phi.p,
                    (const double *)(norm_state.p + 1), 1, epartial.p, nx, ny, nz, 1.0 / (P.dx * P.dx),
@@ -576,20 +543,7 @@ template <class R> class Solver final : public SolverBase {
             return;
         if (!lazy)
             set_divisor_one();
-        if (fused) {
-            fused_imag(k);
-            lazy = true;
-            check_status();
-            return;
-        }
-        const int CH = kItChunk;
-        long done    = 0;
-        while (k - done >= CH) {
-            run_graph(0, CH);
-            done += CH;
-        }
-        if (k - done > 0)
-            run_graph(0, (int)(k - done));
+        fused_imag(k);
         lazy = true;
         check_status();
     }
@@ -615,19 +569,7 @@ template <class R> class Solver final : public SolverBase {
         GPE_CUDA(cudaMemcpyAsync(coef_dev.p, coef_host, sizeof(StepCoef) * k, cudaMemcpyHostToDevice, cur));
         GPE_CUDA(cudaEventRecord(coef_event, cur));
         GPE_CUDA(cudaMemsetAsync(iter_base.p, 0, sizeof(int), cur));
-        if (fused) {
-            fused_real(k);
-            check_status();
-            return;
-        }
-        const int CH = kRtChunk;
-        long done    = 0;
-        while (k - done >= CH) {
-            run_graph(1, CH);
-            done += CH;
-        }
-        if (k - done > 0)
-            run_graph(1, (int)(k - done));
+        fused_real(k);
         check_status();
     }
 
@@ -636,18 +578,14 @@ template <class R> class Solver final : public SolverBase {
             throw Error(GPE_ERR_ARG, "bad kernel id or repetition count");
         materialize();
         // save the state the kernels modify
-        DevBuf<C> save_psi, save_A, save_S2;
+        DevBuf<C> save_psi, save_S2;
         DevBuf<R> save_phi;
         save_psi.alloc(N);
-        save_A.alloc(A.n);
         save_phi.alloc(N);
         GPE_CUDA(cudaMemcpyAsync(save_psi.p, psi.p, sizeof(C) * N, cudaMemcpyDeviceToDevice, cur));
-        GPE_CUDA(cudaMemcpyAsync(save_A.p, A.p, sizeof(C) * A.n, cudaMemcpyDeviceToDevice, cur));
         GPE_CUDA(cudaMemcpyAsync(save_phi.p, phi.p, sizeof(R) * N, cudaMemcpyDeviceToDevice, cur));
-        if (fused) {
-            save_S2.alloc(S2.n);
-            GPE_CUDA(cudaMemcpyAsync(save_S2.p, S2.p, sizeof(C) * S2.n, cudaMemcpyDeviceToDevice, cur));
-        }
+        save_S2.alloc(S2.n);
+        GPE_CUDA(cudaMemcpyAsync(save_S2.p, S2.p, sizeof(C) * S2.n, cudaMemcpyDeviceToDevice, cur));
         if (which == GPE_K_F_Z || which == GPE_K_F_YZ) {
             // the merged phase reads the coefficients of two consecutive iterations
             ensure_coef_capacity(2);
@@ -661,63 +599,50 @@ template <class R> class Solver final : public SolverBase {
         GPE_CUDA(cudaEventCreate(&e0));
         GPE_CUDA(cudaEventCreate(&e1));
         const double F = (double)sizeof(C) * N, Rb = (double)sizeof(R) * N;
-        const double I = (double)sizeof(C) * nx * 2 * ny * H, half = (double)sizeof(C) * nx * ny * H;
+        const double I = (double)sizeof(C) * nx * 2 * ny * nz, half = (double)sizeof(C) * nx * ny * nz;
+        const double dscale = 1.0 / (8.0 * (double)N);
         double b = 0;
         auto one = [&]() {
-            const int lines = nx * ny;
             switch (which) {
             case GPE_K_DIP_Z_FWD:
-                launch(k_dip_z_fwd<R>, (lines + dz.TB - 1) / dz.TB, 256, dz.smem(), cur, (const C *)psi.p,
-                       (const double *)(norm_state.p + 1), 1, A.p, nx, ny, nz, (R)P.n_atoms, dz.plan, dz.TB);
+                gen_z<GZ_IT_PRO>(cur, psi.p, psi.p, cur_coef.p, 0, 0);
                 b = F + half;
                 break;
             case GPE_K_DIP_Y_FWD:
-                launch(k_dip_y<-1, R>, dim3((H + dy.TB - 1) / dy.TB, nx), 256, dy.smem(), cur, A.p, ny, H,
-                       ny, 2 * ny, dy.plan, dy.TB);
+                gen_y(cur, false, false, true);
                 b = half + I;
                 break;
             case GPE_K_DIP_X:
-                launch(k_dip_x<R>, (2 * ny * H + dx.TB - 1) / dx.TB, 256, dx.smem(), cur, A.p,
-                       (const R *)vk.p, nx, ny, H, (R)1, dx.plan, dx.TB);
+                gen_x(cur, false, true, nullptr, dscale);
                 b = 2 * I;
                 break;
             case GPE_K_DIP_Y_INV:
-                launch(k_dip_y<+1, R>, dim3((H + dy.TB - 1) / dy.TB, nx), 256, dy.smem(), cur, A.p, ny, H,
-                       2 * ny, ny, dy.plan, dy.TB);
+                gen_y(cur, true, false, true);
                 b = I + half;
                 break;
             case GPE_K_DIP_Z_INV:
-                launch(k_dip_z_inv<R>, (lines + dz.TB - 1) / dz.TB, 256, dz.smem(), cur, (const C *)A.p, phi.p,
-                       nx, ny, nz, (R)(1.0 / (8.0 * (double)N)), dz.plan, dz.TB);
+                gen_z<GZ_DIP_INV>(cur, psi.p, psi.p, cur_coef.p, 0, 1);
                 b = half + Rb;
                 break;
             case GPE_K_KIN_Z_FWD:
+                gen_z<GZ_KIN_FWD>(cur, psi.p, psi.p, cur_coef.p, 0, 0);
+                b = 2 * F;
+                break;
             case GPE_K_KIN_Z_INV:
-                if (which == GPE_K_KIN_Z_FWD)
-                    launch(k_kin_z<-1, R>, (lines + kz.TB - 1) / kz.TB, 256, kz.smem(), cur, psi.p, lines, nz,
-                           kz.plan, kz.TB);
-                else
-                    launch(k_kin_z<+1, R>, (lines + kz.TB - 1) / kz.TB, 256, kz.smem(), cur, psi.p, lines, nz,
-                           kz.plan, kz.TB);
+                gen_z<GZ_KIN_INV>(cur, psi.p, psi.p, cur_coef.p, 0, 0);
                 b = 2 * F;
                 break;
             case GPE_K_KIN_Y_FWD:
             case GPE_K_KIN_Y_INV:
-                if (which == GPE_K_KIN_Y_FWD)
-                    launch(k_kin_y<-1, R>, dim3((nz + ky.TB - 1) / ky.TB, nx), 256, ky.smem(), cur, psi.p, ny,
-                           nz, ky.plan, ky.TB);
-                else
-                    launch(k_kin_y<+1, R>, dim3((nz + ky.TB - 1) / ky.TB, nx), 256, ky.smem(), cur, psi.p, ny,
-                           nz, ky.plan, ky.TB);
+                gen_y(cur, which == GPE_K_KIN_Y_INV, true, false);
                 b = 2 * F;
                 break;
             case GPE_K_KIN_X:
-                launch(k_kin_x<R>, (ny * nz + kx.TB - 1) / kx.TB, 256, kx.smem(), cur, psi.p,
-                       (const C *)ex.p, (const C *)ey.p, (const C *)ez.p, inv_hi, inv_lo, nx, ny, nz, kx.plan, kx.TB);
+                gen_x(cur, true, false, nullptr, dscale);
                 b = 2 * F;
                 break;
             case GPE_K_PHASE:
-                enqueue_phase(cur, cur_coef.p, iter_zero.p, 0);
+                gen_z<GZ_PHASE>(cur, psi.p, psi.p, cur_coef.p, 0, 0, iter_zero.p);
                 b = 2 * F + 2 * Rb;
                 break;
             case GPE_K_F_X:
@@ -762,7 +687,7 @@ template <class R> class Solver final : public SolverBase {
                 break;
             }
             default:
-                enqueue_it_update(cur, psi.p, psii.p);
+                gen_z<GZ_IT_STEP>(cur, psi.p, psii.p, cur_coef.p, 0, 0);
                 b = 2 * F + 2 * Rb;
                 break;
             }
@@ -778,10 +703,8 @@ template <class R> class Solver final : public SolverBase {
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         GPE_CUDA(cudaMemcpyAsync(psi.p, save_psi.p, sizeof(C) * N, cudaMemcpyDeviceToDevice, cur));
-        GPE_CUDA(cudaMemcpyAsync(A.p, save_A.p, sizeof(C) * A.n, cudaMemcpyDeviceToDevice, cur));
         GPE_CUDA(cudaMemcpyAsync(phi.p, save_phi.p, sizeof(R) * N, cudaMemcpyDeviceToDevice, cur));
-        if (fused)
-            GPE_CUDA(cudaMemcpyAsync(S2.p, save_S2.p, sizeof(C) * S2.n, cudaMemcpyDeviceToDevice, cur));
+        GPE_CUDA(cudaMemcpyAsync(S2.p, save_S2.p, sizeof(C) * S2.n, cudaMemcpyDeviceToDevice, cur));
         GPE_CUDA(cudaStreamSynchronize(cur));
         *ms    = (double)t / reps;
         *bytes = b;
@@ -814,7 +737,7 @@ template <class R> class Solver final : public SolverBase {
         GPE_CUDA(cudaMemcpy(vk2.p, t.data(), sizeof(R) * t.size(), cudaMemcpyHostToDevice));
     }
 
-    static Twid twid(const Line &l) { return Twid{l.plan.tw, l.plan.twlo}; }
+    static Twid twid(const Line &l) { return Twid{l.tw.p, l.twlo.p}; }
 
 #define GPE_XY_CASES(M) M(32) M(64) M(96) M(128) M(256)
 #define GPE_Z_CASES(M) M(8) M(16) M(24) M(32) M(64)
@@ -1231,6 +1154,10 @@ template <class R> class Solver final : public SolverBase {
     // kind 10: RT prologue; 11: C mid RT iterations; 12: `count` mid + the last;
     // kind 20: IT prologue; 21: `count` IT iterations.
     void capture_fused(int kind, int count) {
+        if (!fused) {
+            capture_general(kind, count);
+            return;
+        }
         if (yz_plane()) {
             capture_fused_yz(kind, count);
             return;
@@ -1280,6 +1207,76 @@ template <class R> class Solver final : public SolverBase {
                 f_y<+1>(s, false);
                 f_z<ZM_IT_MID>(s, a, b, cur_coef.p, 0);
                 f_y<-1>(s, false);
+                std::swap(a, b);
+            }
+        }
+    }
+
+    // ---- every grid, both precisions (general.cuh): x, y inverse, z, y forward ----
+    void gen_x(cudaStream_t s, bool kin, bool dip, const double *divisor, double dscale) {
+        GXArgs a{};
+        a.psi = psi.p, a.S = S2.p;
+        a.ex = ex.p, a.ey = ey.p, a.ez = ez.p;
+        a.inv = 1.0 / (double)N;
+        a.vk = vk2.p, a.divisor = divisor, a.dip_scale = dscale;
+        a.nx = nx, a.ny = ny, a.nz = nz, a.lb = shape.lbx;
+        a.k = kx.plan, a.d = dx.plan;
+        const int w = 1 << a.lb, cols = ny * nz;
+        a.tk = kin ? (cols + w - 1) / w : 0;
+        launch(g_x<R>, a.tk + (dip ? (2 * cols + w - 1) / w : 0), shape.ntx, shape.smx, s, a);
+    }
+    void gen_y(cudaStream_t s, bool inverse, bool kin, bool dip) {
+        GYArgs a{};
+        a.psi = psi.p, a.S = S2.p;
+        a.ny = ny, a.nz = nz, a.inverse = inverse, a.lb = shape.lby;
+        a.k = ky.plan, a.d = dy.plan;
+        const int tiles = (nz + (1 << a.lb) - 1) >> a.lb;
+        a.tk            = kin ? tiles : 0;
+        launch(g_y<R>, dim3(a.tk + (dip ? tiles : 0), nx), shape.nty, shape.smy, s, a);
+    }
+    template <int MODE>
+    void gen_z(cudaStream_t s, C *pin, C *pout, const StepCoef *coef, int local, int write_phi,
+               const int *base = nullptr) {
+        GZArgs a{};
+        a.z = zargs(pin, pout, coef, local);
+        if (base)
+            a.z.step.base = base;
+        a.write_phi = write_phi;
+        a.nz = nz, a.mz = g_magic(nz), a.lb = shape.lbz, a.buf = shape.buf;
+        a.k = kz.plan, a.d = dz.plan;
+        // the single steps without a transform take no tile
+        constexpr bool tile = MODE < GZ_PHASE;
+        launch(g_z<R, MODE>, (nx * ny + (1 << a.lb) - 1) >> a.lb, shape.ntz, tile ? shape.smz : 0, s, a);
+    }
+    void capture_general(int kind, int count) {
+        cudaStream_t s      = cap_stream;
+        const double dscale = 1.0 / (8.0 * (double)N);
+        if (kind == 10) {
+            gen_z<GZ_RT_PRO>(s, psi.p, psi.p, coef_dev.p, 0, 0);
+            gen_y(s, false, true, true);
+        } else if (kind == 11 || kind == 12) {
+            for (int t = 0; t < count + (kind == 12); ++t) {
+                gen_x(s, true, true, nullptr, dscale);
+                gen_y(s, true, true, true);
+                if (t == count) {
+                    gen_z<GZ_RT_EPI>(s, psi.p, psi.p, coef_dev.p, t, 1);
+                } else {
+                    gen_z<GZ_RT_MID>(s, psi.p, psi.p, coef_dev.p, t, 0);
+                    gen_y(s, false, true, true);
+                }
+            }
+            if (kind == 11)
+                launch(k_advance, 1, 1, 0, s, iter_base.p, count);
+        } else if (kind == 20) {
+            gen_z<GZ_IT_PRO>(s, psi.p, psi.p, cur_coef.p, 0, 0);
+            gen_y(s, false, false, true);
+        } else {
+            C *a = psi.p, *b = psii.p;
+            for (int t = 0; t < count; ++t) {
+                gen_x(s, false, true, norm_state.p + 1, dscale);
+                gen_y(s, true, false, true);
+                gen_z<GZ_IT_MID>(s, a, b, cur_coef.p, 0, t == count - 1);
+                gen_y(s, false, false, true);
                 std::swap(a, b);
             }
         }
@@ -1385,12 +1382,12 @@ template <class R> class Solver final : public SolverBase {
     static constexpr int kRtChunk = 32;
 
     gpe_params P;
-    int nx, ny, nz, H;
+    int nx, ny, nz;
     size_t N;
     Line kz, ky, kx, dz, dy, dx;
-    DevBuf<C> psi, psii, bnd, A, ex, ey, ez;
-    DevBuf<R> V, phi, vk;
-    DevBuf<double> staging, norm_state, partial, epartial, eout;
+    DevBuf<C> psi, psii, bnd, ex, ey, ez;
+    DevBuf<R> V, phi;
+    DevBuf<double> staging, norm_state, epartial, eout;
     DevBuf<double> export_buf; // asynchronous exports
     DevBuf<double> ehist;      // energy history of imag_steps_energies
     cudaStream_t copy_stream = nullptr;
@@ -1404,7 +1401,8 @@ template <class R> class Solver final : public SolverBase {
     // imaginary-time k4_yz with twice the real-time block (at most 1024
     // threads) or the real-time block: picked by autotune_x
     bool it_wide = true;
-    DevBuf<C> S2;
+    DevBuf<C> S2; // dipolar spectrum, S[i][ky][kz - 1]
+    GShape shape{}; // launch shapes of general.cuh
     DevBuf<C> psir; // real time: psi in real space after the last phase step
     int xk_lines = 16, xd_lines = 16; // x-pass lines per CTA (autotune_x)
     int y_lines = 16;                 // y-pass z columns per CTA (four-kernel schedule; autotune_x)
@@ -1439,76 +1437,57 @@ template <class R> class Solver final : public SolverBase {
         ++n_launch;
     }
 
-    void plan_line(Line &ln, int L, int tbmax, int pad) {
-        std::vector<int> r = factor_line(L);
-        ln.plan.L          = L;
-        ln.plan.nstages    = (int)r.size();
-        ln.pad             = pad;
-        for (size_t s = 0; s < r.size(); ++s)
-            ln.plan.radix[s] = r[s];
+    void plan_line(Line &ln, int L, int pad) {
+        factor_line(L); // rejects unsupported lengths
+        if (2 * sizeof(C) * (size_t)(1 + pad) * L > 200 * 1024)
+            throw Error(GPE_ERR_SIZE, "FFT line of length " + std::to_string(L) + " too long");
         std::vector<double> t = twiddles(L);
         std::vector<C> tc(L), tl(L);
+        std::vector<typename GTwid<R>::T> tg(L);
         for (int m = 0; m < L; ++m) {
             tc[m] = C{(R)t[2 * m], (R)t[2 * m + 1]};
             tl[m] = C{(R)(t[2 * m] - (double)tc[m].x), (R)(t[2 * m + 1] - (double)tc[m].y)};
+            if constexpr (std::is_same<R, float>::value)
+                tg[m] = make_float4(tc[m].x, tc[m].y, tl[m].x, tl[m].y);
+            else
+                tg[m] = tc[m];
         }
         ln.tw.alloc(L);
         ln.twlo.alloc(L);
+        ln.gtw.alloc(L);
         GPE_CUDA(cudaMemcpy(ln.tw.p, tc.data(), sizeof(C) * L, cudaMemcpyHostToDevice));
         GPE_CUDA(cudaMemcpy(ln.twlo.p, tl.data(), sizeof(C) * L, cudaMemcpyHostToDevice));
-        ln.plan.tw   = ln.tw.p;
-        ln.plan.twlo = ln.twlo.p;
-        // Tile: two Stockham buffers of TB lines within a 64 KiB budget per CTA.
-        const size_t budget = 64 * 1024;
-        int TB              = tbmax;
-        while (TB > 1 && 2 * sizeof(C) * (size_t)(TB + pad) * L > budget)
-            TB >>= 1;
-        if (2 * sizeof(C) * (size_t)(TB + pad) * L > 200 * 1024)
-            throw Error(GPE_ERR_SIZE, "FFT line of length " + std::to_string(L) + " too long");
-        ln.TB = TB;
+        GPE_CUDA(cudaMemcpy(ln.gtw.p, tg.data(), sizeof(tg[0]) * L, cudaMemcpyHostToDevice));
+        ln.plan = g_plan(L, ln.gtw.p);
     }
 
-    void set_smem_attrs() {
-        auto set = [](const void *f, size_t bytes) {
-            if (bytes > 48 * 1024)
-                GPE_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    // The limit is a property of the kernel in this process, shared by handles of
+    // other grids: it goes to the device's maximum.
+    void set_general_attrs() {
+        int most = 0;
+        GPE_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, P.device));
+        auto set = [&](const void *f, size_t bytes) {
+            cudaFuncAttributes fa{};
+            GPE_CUDA(cudaFuncGetAttributes(&fa, f));
+            const int room = most - (int)fa.sharedSizeBytes;
+            if (bytes > (size_t)room)
+                throw Error(GPE_ERR_SIZE, "the line tiles of this grid need more shared memory than a block has");
+            GPE_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
         };
-        set((const void *)k_dip_z_fwd<R>, dz.smem());
-        set((const void *)k_dip_y<-1, R>, dy.smem());
-        set((const void *)k_dip_y<+1, R>, dy.smem());
-        set((const void *)k_dip_x<R>, dx.smem());
-        set((const void *)k_dip_z_inv<R>, dz.smem());
-        set((const void *)k_kin_z<-1, R>, kz.smem());
-        set((const void *)k_kin_z<+1, R>, kz.smem());
-        set((const void *)k_kin_y<-1, R>, ky.smem());
-        set((const void *)k_kin_y<+1, R>, ky.smem());
-        set((const void *)k_kin_x<R>, kx.smem());
+        set((const void *)g_x<R>, shape.smx);
+        set((const void *)g_y<R>, shape.smy);
+        set((const void *)g_z<R, GZ_RT_PRO>, shape.smz);
+        set((const void *)g_z<R, GZ_RT_MID>, shape.smz);
+        set((const void *)g_z<R, GZ_RT_EPI>, shape.smz);
+        set((const void *)g_z<R, GZ_IT_PRO>, shape.smz);
+        set((const void *)g_z<R, GZ_IT_MID>, shape.smz);
+        set((const void *)g_z<R, GZ_DIP_INV>, shape.smz);
+        set((const void *)g_z<R, GZ_KIN_FWD>, shape.smz);
+        set((const void *)g_z<R, GZ_KIN_INV>, shape.smz);
     }
 
-    // FP64 tables: V_dd(k) (fftw_poisson_solver.cpp:12-49) reduced by |kx|,|ky|
-    // symmetry, and the separable kinetic phase (fftw_split_solver.cpp:11-42).
+    // FP64 tables: the separable kinetic phase (fftw_split_solver.cpp:11-42).
     void build_tables() {
-        {
-            const int px = 2 * nx, py = 2 * ny, pz = 2 * nz;
-            const double dkx = 2. * M_PI / (px * P.dx);
-            const double dky = 2. * M_PI / (py * P.dy);
-            const double dkz = 2. * M_PI / (pz * P.dz);
-            std::vector<R> t((size_t)(nx + 1) * (ny + 1) * H);
-            for (int i = 0; i <= nx; ++i) {
-                const double kxv = (i <= (px / 2)) ? i * dkx : (i - px) * dkx;
-                for (int j = 0; j <= ny; ++j) {
-                    const double kyv = (j <= (py / 2)) ? j * dky : (j - py) * dky;
-                    for (int k = 0; k < H; ++k) {
-                        const double kzv = (k <= (pz / 2)) ? k * dkz : (k - pz) * dkz;
-                        const double k2  = kxv * kxv + kyv * kyv + kzv * kzv;
-                        const double v   = (k2 > 1e-30) ? (kzv * kzv / k2) : 0.0;
-                        t[((size_t)i * (ny + 1) + j) * H + k] = (R)v;
-                    }
-                }
-            }
-            vk.alloc(t.size());
-            GPE_CUDA(cudaMemcpy(vk.p, t.data(), sizeof(R) * t.size(), cudaMemcpyHostToDevice));
-        }
         {
             // Per-axis exp(i theta) - 1 with theta = -dt/(2m) k^2 (k as in
             // fftw_split_solver.cpp:26-31), in FP64; the kernel combines the three
@@ -1581,11 +1560,11 @@ template <class R> class Solver final : public SolverBase {
         coef_cap = cap;
         if (!coef_event)
             GPE_CUDA(cudaEventCreateWithFlags(&coef_event, cudaEventDisableTiming));
-        // cached real-time graphs (split schedule: kind 1; fused: kinds 10-12)
-        // hold the address of the old coefficient buffer
+        // cached real-time graphs (kinds 10-12) hold the address of the old
+        // coefficient buffer
         for (auto it = graphs.begin(); it != graphs.end();) {
             const int kind = std::get<0>(it->first);
-            if (kind == 1 || (kind >= 10 && kind <= 12)) {
+            if (kind >= 10 && kind <= 12) {
                 cudaGraphExecDestroy(it->second);
                 graph_nodes.erase(it->first);
                 it = graphs.erase(it);
@@ -1596,115 +1575,20 @@ template <class R> class Solver final : public SolverBase {
     }
 
     // ---- enqueue helpers (usable while capturing) ---------------------------
-    void enqueue_norm(cudaStream_t s, const C *p, bool set_divisor) {
-        launch(k_norm_partial<R>, nblk_elem, 256, 0, s, p, N, partial.p);
-        launch(k_norm_finalize, 1, 256, 0, s, (const double *)partial.p, nblk_elem,
-               P.dx * P.dy * P.dz, norm_state.p, status.p);
-        if (!set_divisor)
-            return;
-    }
-
-    void enqueue_dipolar(cudaStream_t s, const C *p) {
-        const int lines = nx * ny;
-        launch(k_dip_z_fwd<R>, (lines + dz.TB - 1) / dz.TB, 256, dz.smem(), s, p,
-               (const double *)(norm_state.p + 1), 1, A.p, nx, ny, nz, (R)P.n_atoms, dz.plan, dz.TB);
-        launch(k_dip_y<-1, R>, dim3((H + dy.TB - 1) / dy.TB, nx), 256, dy.smem(), s, A.p, ny, H, ny,
-               2 * ny, dy.plan, dy.TB);
-        const int cols = 2 * ny * H;
-        launch(k_dip_x<R>, (cols + dx.TB - 1) / dx.TB, 256, dx.smem(), s, A.p, (const R *)vk.p, nx,
-               ny, H, (R)1, dx.plan, dx.TB);
-        launch(k_dip_y<+1, R>, dim3((H + dy.TB - 1) / dy.TB, nx), 256, dy.smem(), s, A.p, ny, H,
-               2 * ny, ny, dy.plan, dy.TB);
-        const R inv_n = (R)(1.0 / (8.0 * (double)N));
-        launch(k_dip_z_inv<R>, (lines + dz.TB - 1) / dz.TB, 256, dz.smem(), s, (const C *)A.p, phi.p,
-               nx, ny, nz, inv_n, dz.plan, dz.TB);
+    void enqueue_dipolar(cudaStream_t s, C *p) {
+        gen_z<GZ_IT_PRO>(s, p, p, cur_coef.p, 0, 0);
+        gen_y(s, false, false, true);
+        gen_x(s, false, true, norm_state.p + 1, 1.0 / (8.0 * (double)N));
+        gen_y(s, true, false, true);
+        gen_z<GZ_DIP_INV>(s, p, p, cur_coef.p, 0, 1);
     }
 
     void enqueue_kinetic(cudaStream_t s) {
-        const int lines = nx * ny;
-        launch(k_kin_z<-1, R>, (lines + kz.TB - 1) / kz.TB, 256, kz.smem(), s, psi.p, lines, nz,
-               kz.plan, kz.TB);
-        launch(k_kin_y<-1, R>, dim3((nz + ky.TB - 1) / ky.TB, nx), 256, ky.smem(), s, psi.p, ny, nz,
-               ky.plan, ky.TB);
-        const int cols = ny * nz;
-        launch(k_kin_x<R>, (cols + kx.TB - 1) / kx.TB, 256, kx.smem(), s, psi.p, (const C *)ex.p,
-               (const C *)ey.p, (const C *)ez.p, inv_hi, inv_lo, nx, ny, nz, kx.plan, kx.TB);
-        launch(k_kin_y<+1, R>, dim3((nz + ky.TB - 1) / ky.TB, nx), 256, ky.smem(), s, psi.p, ny, nz,
-               ky.plan, ky.TB);
-        launch(k_kin_z<+1, R>, (lines + kz.TB - 1) / kz.TB, 256, kz.smem(), s, psi.p, lines, nz,
-               kz.plan, kz.TB);
-    }
-
-    void enqueue_phase(cudaStream_t s, const StepCoef *coef, const int *base, int local) {
-        launch(k_phase<R>, grid_elem(N), 256, 0, s, psi.p, (const R *)V.p, (const R *)phi.p, coef,
-               base, local, nx, ny, nz, (R)(P.real_time_dt / 2.), (R)P.cdd);
-    }
-
-    void enqueue_it_update(cudaStream_t s, const C *in, C *out) {
-        const double m = P.m;
-        launch(k_it_update<R>, nblk_elem, 256, 0, s, in, out, (const C *)bnd.p, (const R *)V.p,
-               (const R *)phi.p, (const double *)(norm_state.p + 1), (const StepCoef *)cur_coef.p,
-               partial.p, nx, ny, nz, (R)(-0.5 / (m * P.dx * P.dx)), (R)(0.5 / (m * P.dy * P.dy)),
-               (R)(0.5 / (m * P.dz * P.dz)), (R)P.imag_time_dt, (R)P.cdd);
-    }
-
-    // One fused imaginary-time iteration from psi `in` into `out`:
-    // calc_fi3d -> Euler update -> calc_norm (normalize held as the divisor).
-    void enqueue_it_step(cudaStream_t s, const C *in, C *out) {
-        enqueue_dipolar(s, in);
-        enqueue_it_update(s, in, out);
-        launch(k_norm_finalize, 1, 256, 0, s, (const double *)partial.p, nblk_elem,
-               P.dx * P.dy * P.dz, norm_state.p, status.p);
-    }
-
-    // One fused real-time iteration (real_time_iter) on psi in place.
-    void enqueue_rt_step(cudaStream_t s, int local) {
-        enqueue_phase(s, coef_dev.p, iter_base.p, local);
-        enqueue_dipolar(s, psi.p);
-        enqueue_kinetic(s);
-        enqueue_phase(s, coef_dev.p, iter_base.p, local);
-    }
-
-    // kind 0: `count` IT iterations; kind 1: `count` RT iterations.
-    void run_graph(int kind, int count) {
-        auto key = std::make_tuple(kind, count, (const void *)psi.p);
-        auto it  = graphs.find(key);
-        if (it == graphs.end()) {
-            const long long before = n_launch;
-            GPE_CUDA(cudaStreamBeginCapture(cap_stream, cudaStreamCaptureModeThreadLocal));
-            try {
-                if (kind == 0) {
-                    C *a = psi.p, *b = psii.p;
-                    for (int t = 0; t < count; ++t) {
-                        enqueue_it_step(cap_stream, a, b);
-                        std::swap(a, b);
-                    }
-                } else {
-                    for (int t = 0; t < count; ++t)
-                        enqueue_rt_step(cap_stream, t);
-                    launch(k_advance, 1, 1, 0, cap_stream, iter_base.p, count);
-                }
-            } catch (...) {
-                cudaGraph_t g;
-                cudaStreamEndCapture(cap_stream, &g);
-                if (g)
-                    cudaGraphDestroy(g);
-                throw;
-            }
-            cudaGraph_t g;
-            GPE_CUDA(cudaStreamEndCapture(cap_stream, &g));
-            cudaGraphExec_t ge;
-            GPE_CUDA(cudaGraphInstantiate(&ge, g, 0));
-            cudaGraphDestroy(g);
-            graphs[key]      = ge;
-            graph_nodes[key] = (int)(n_launch - before);
-            n_launch         = before;
-            it               = graphs.find(key);
-        }
-        GPE_CUDA(cudaGraphLaunch(it->second, cur));
-        n_launch += graph_nodes[key];
-        if (kind == 0 && (count & 1))
-            std::swap(psi.p, psii.p);
+        gen_z<GZ_KIN_FWD>(s, psi.p, psi.p, cur_coef.p, 0, 0);
+        gen_y(s, false, true, false);
+        gen_x(s, true, false, nullptr, 0.0);
+        gen_y(s, true, true, false);
+        gen_z<GZ_KIN_INV>(s, psi.p, psi.p, cur_coef.p, 0, 0);
     }
 };
 
@@ -2239,9 +2123,9 @@ int gpe_time_kernel(gpe_handle *h, int which, int reps, double *ms, double *byte
 }
 
 const char *gpe_kernel_name(int which) {
-    static const char *names[] = {"k_dip_z_fwd", "k_dip_y", "k_dip_x", "k_dip_y", "k_dip_z_inv",
-                                  "k_kin_z", "k_kin_y", "k_kin_x", "k_kin_y", "k_kin_z",
-                                  "k_phase", "k_it_update", "k3_x", "k3_y", "k2_z", "k3_y",
+    static const char *names[] = {"g_z", "g_y", "g_x", "g_y", "g_z",
+                                  "g_z", "g_y", "g_x", "g_y", "g_z",
+                                  "g_z", "g_z", "k3_x", "k3_y", "k2_z", "k3_y",
                                   "k3_x_kin", "k3_x_dip", "k4_yz"};
     if (which < 0 || which >= GPE_K_COUNT)
         return "";
