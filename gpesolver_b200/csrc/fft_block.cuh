@@ -252,14 +252,14 @@ template <> struct OddTab<7> {
     }
 };
 
+// acc + v c for a real constant, complex64 as packed FP32x2 multiply-adds
+__device__ __forceinline__ float2 cfma(float2 v, float c, float2 acc) { return __ffma2_rn(v, float2{c, c}, acc); }
+__device__ __forceinline__ double2 cfma(double2 v, double c, double2 acc) {
+    return double2{fma(v.x, c, acc.x), fma(v.y, c, acc.y)};
+}
+
 template <int P, int SIGN, class R, bool CMP = true> struct DFTOdd {
     using C = cplx<R>;
-    static __device__ __forceinline__ R mulc(R x, double c) {
-        if constexpr (CMP)
-            return cmulk<R>(x, c);
-        else
-            return x * (R)c;
-    }
     static __device__ __forceinline__ void run(C *a) {
         constexpr int H = P / 2;
         C t[H], d[H];
@@ -276,15 +276,25 @@ template <int P, int SIGN, class R, bool CMP = true> struct DFTOdd {
         a[0] = sum;
 #pragma unroll
         for (int q = 1; q <= H; ++q) {
-            C re = x0, im{(R)0, (R)0}; // X_q = re + SIGN i im, X_{P-q} = re - SIGN i im
+            // X_q = re + SIGN i im, X_{P-q} = re - SIGN i im.  Compensated: the constants'
+            // rounding remainders are summed first and enter the first rounding of the
+            // products' sum (added to x0 they would be rounded off, always to the same
+            // side, and the norm would drift)
+            C re{(R)0, (R)0}, im{(R)0, (R)0};
+            if constexpr (CMP && sizeof(R) == 4) {
+#pragma unroll
+                for (int k = 0; k < H; ++k) {
+                    const double c = OddTab<P>::c(((k + 1) * q) % P), s = OddTab<P>::s(((k + 1) * q) % P);
+                    re = cfma(t[k], (R)(c - (double)(R)c), re);
+                    im = cfma(d[k], (R)(s - (double)(R)s), im);
+                }
+            }
 #pragma unroll
             for (int k = 0; k < H; ++k) {
-                const int m = ((k + 1) * q) % P;
-                re.x += mulc(t[k].x, OddTab<P>::c(m));
-                re.y += mulc(t[k].y, OddTab<P>::c(m));
-                im.x += mulc(d[k].x, OddTab<P>::s(m));
-                im.y += mulc(d[k].y, OddTab<P>::s(m));
+                re = cfma(t[k], (R)OddTab<P>::c(((k + 1) * q) % P), re);
+                im = cfma(d[k], (R)OddTab<P>::s(((k + 1) * q) % P), im);
             }
+            re = cadd(x0, re);
             const C j = mul_si<SIGN>(im);
             a[q]      = cadd(re, j);
             a[P - q]  = csub(re, j);

@@ -90,10 +90,11 @@ __device__ __forceinline__ void g_mid_r(const GStage &st, const void *tw, unsign
         C a[RAD];
         g_load<RAD, R>(a, sm + src, st, jm, j, b, TS, nin, tw);
         DFT<RAD, -1, R>::run(a);
-        C *o = sm + dst + (d * st.ns * RAD + jm) * TS + b;
+        C *o         = sm + dst + (d * st.ns * RAD + jm) * TS + b;
+        const int os = st.ns * TS;
 #pragma unroll
         for (int q = 0; q < RAD; ++q)
-            o[q * st.ns * TS] = a[q];
+            o[q * os] = a[q];
     }
 }
 template <class R>
@@ -191,6 +192,13 @@ __device__ __forceinline__ void g_lines(const GPlan &pl, cplx<R> *p, size_t rs, 
     }
 }
 
+// g_x and g_y hold a radix's inputs in registers (g_x twice over, for the pair of
+// transforms): MB = 3 CTAs of 256 threads per SM (80 registers) in complex64 up to radix 15,
+// 2 (128 registers) for radix 16, where 3 would spill more, and in complex128.  Measured with 3
+// against 2: real time 100 x 90 x 30 45.3 against 50.6 us an iteration, 144 x 144 x 40
+// 106 against 123; the field at 128 x 128 x 32 (radix 16) 65.6 against 60.7 us.
+template <class R> constexpr int g_blocks(int most_radix) { return sizeof(R) == 4 && most_radix <= 15 ? 3 : 2; }
+
 // ---------------------------------------------------------------------------
 // y lines: one x plane per blockIdx.y, tiles of 2^lb z columns along blockIdx.x,
 // first the kinetic ones (tk), then the dipolar ones
@@ -201,7 +209,7 @@ struct GYArgs {
     int lb;
     GPlan k, d;
 };
-template <class R> __global__ void __launch_bounds__(256, 2) g_y(const __grid_constant__ GYArgs a) {
+template <class R, int MB> __global__ void __launch_bounds__(256, MB) g_y(const __grid_constant__ GYArgs a) {
     using C        = cplx<R>;
     const bool kin = (int)blockIdx.x < a.tk;
     const int k0   = (kin ? blockIdx.x : blockIdx.x - a.tk) << a.lb;
@@ -290,7 +298,7 @@ __device__ __forceinline__ void g_xmid_r(const GXArgs &a, const GPlan &pl, bool 
     }
 }
 
-template <class R> __global__ void __launch_bounds__(256, 2) g_x(const __grid_constant__ GXArgs a) {
+template <class R, int MB> __global__ void __launch_bounds__(256, MB) g_x(const __grid_constant__ GXArgs a) {
     using C         = cplx<R>;
     const int tid = threadIdx.x, nt = blockDim.x;
     const bool kin  = (int)blockIdx.x < a.tk;
@@ -399,23 +407,43 @@ struct GZArgs {
     ZArgs z;
     int write_phi, nz, lb; // 2^lb rows per CTA
     unsigned mz;           // ceil(2^32 / nz)
-    unsigned buf;          // elements of one of the three tile buffers
+    unsigned buf;          // elements of one of the four tiles
     GPlan k, d;
 };
 
-// All stages of the 2^lb lines in the tile at `cur`; returns with the result there.
-template <class R>
-__device__ __forceinline__ void g_tile(const GPlan &pl, unsigned &cur, unsigned &scr, int lb, int TS, int nin, int tid,
-                                       int nt) {
-    for (int s = 0; s < pl.n; ++s) {
-        g_mid<R>(pl.f[s], pl.tw, cur, scr, lb, TS, s == 0 ? nin : pl.L, tid, nt);
+// The kinetic rows in tile K and the dipolar pair lines in tile D (offsets in g_smem)
+// transformed, stage by stage side by side: each by half of the warps (all of them where only
+// one runs), so that a warp executes one of them and they share the
+// synchronisations.  The results are left in the tiles that K and D name on return.
+template <class R, bool KIN, bool DIP>
+__device__ __forceinline__ void g_tiles(const GPlan &pk, unsigned &K, unsigned &K2, int lk, int TK, const GPlan &pd,
+                                        unsigned &D, unsigned &D2, int ld, int TD, int nin) {
+    const int nt    = KIN && DIP ? blockDim.x >> 1 : blockDim.x;
+    const bool kin  = KIN && (!DIP || (int)threadIdx.x < nt);
+    const int tid   = KIN && DIP && !kin ? threadIdx.x - nt : threadIdx.x;
+    const GPlan &pl = kin ? pk : pd;
+    unsigned cur = kin ? K : D, oth = kin ? K2 : D2;
+    const int lb = kin ? lk : ld, TS = kin ? TK : TD;
+    const int ns = KIN && DIP ? max(pk.n, pd.n) : pl.n;
+    for (int s = 0; s < ns; ++s) {
+        if (s < pl.n) {
+            g_mid<R>(pl.f[s], pl.tw, cur, oth, lb, TS, s == 0 && !kin ? nin : pl.L, tid, nt);
+            const unsigned t = cur;
+            cur = oth, oth = t;
+        }
         __syncthreads();
-        const unsigned t = cur;
-        cur = scr, scr = t;
+    }
+    if (KIN && (pk.n & 1)) {
+        const unsigned t = K;
+        K = K2, K2 = t;
+    }
+    if (DIP && (pd.n & 1)) {
+        const unsigned t = D;
+        D = D2, D2 = t;
     }
 }
 
-template <class R, int MODE> __global__ void __launch_bounds__(256, 2) g_z(const __grid_constant__ GZArgs g) {
+template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) g_z(const __grid_constant__ GZArgs g) {
     using C            = cplx<R>;
     constexpr bool RT  = MODE <= GZ_RT_EPI || MODE == GZ_PHASE;
     constexpr bool IT  = MODE == GZ_IT_MID || MODE == GZ_IT_STEP;
@@ -428,16 +456,17 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, 2) g_z(const
     const int RW = 1 << g.lb, lp = g.lb > 0 ? g.lb - 1 : 0, NP = 1 << lp; // rows, row pairs
     const int TK = RW >= 4 ? RW + 1 : RW, TD = NP >= 2 ? NP + 1 : NP;     // odd tile strides
     const int rows = nx * ny, r0 = blockIdx.x << g.lb, cnt = min(RW, rows - r0);
-    C *sm       = reinterpret_cast<C *>(g_smem);
-    unsigned K = 0, D = g.buf, T = 2 * g.buf; // kinetic rows, dipolar pair lines, scratch
+    // kinetic rows and dipolar pair lines, two tiles each
+    C *sm      = reinterpret_cast<C *>(g_smem);
+    unsigned D = 0, D2 = g.buf, K = 2 * g.buf, K2 = 3 * g.buf;
     const size_t base = (size_t)r0 * nz;
     C *psi      = reinterpret_cast<C *>(a.psi_in) + base;
     C *out      = reinterpret_cast<C *>(a.psi_out) + base;
-    C *S        = reinterpret_cast<C *>(a.S);
+    C *S        = reinterpret_cast<C *>(a.S) - 1; // bins from 1
     R *phi      = reinterpret_cast<R *>(a.phi) + base;
     const R *V  = reinterpret_cast<const R *>(a.V) + base;
+    // x plane and y of the tile's row; its spectrum row i 2ny + j
     const int i0 = r0 / ny, j0 = r0 - i0 * ny;
-    // x plane and y of the tile's row
     auto place = [&](int row, int &i, int &j) {
         i = i0;
         j = j0 + row;
@@ -446,49 +475,35 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, 2) g_z(const
             ++i;
         }
     };
+    auto srow = [&](int row) {
+        int i, j;
+        place(row, i, j);
+        return (size_t)(2 * i * ny + j) * nz;
+    };
 
-    R g3 = (R)0, gw = (R)0, g3n = (R)0, gwn = (R)0; // this iteration's, the next one's
-    if (RT) {
-        const int it      = *a.step.base + a.step.local;
-        const StepCoef c0 = a.step.coef[it];
-        g3 = (R)c0.g3w;
-        gw = (R)c0.gw15;
-        if (MODE == GZ_RT_MID) {
-            const StepCoef c1 = a.step.coef[it + 1];
-            g3n = (R)c1.g3w;
-            gwn = (R)c1.gw15;
-        }
-    } else if (IT) {
-        g3 = (R)a.step.coef[0].g3w;
-        gw = (R)a.step.coef[0].gw15;
-    }
-
-    // ---- in: psi rows (inverse: swapped) and the pair lines of the spectrum ----
+    // ---- in: psi rows (inverse: swapped) and the pair lines of the spectrum ------
     if (KIN_I || MODE == GZ_KIN_FWD) {
-        for (int e = tid; e < cnt * nz; e += nt) {
+        for (int e = tid; e < RW * nz; e += nt) {
             const int row = g_div(e, nz, g.mz), k = e - row * nz;
-            sm[K + k * TK + row] = g_swap(psi[e], KIN_I);
+            sm[K + k * TK + row] = row < cnt ? g_swap(psi[e], KIN_I) : C{(R)0, (R)0};
         }
-        for (int e = cnt * nz + tid; e < RW * nz; e += nt) {
-            const int row = g_div(e, nz, g.mz), k = e - row * nz;
-            sm[K + k * TK + row] = C{(R)0, (R)0};
-        }
+    }
+    // step coefficients, this iteration's and the next one's: two dependent reads, by one
+    // thread and behind the others' loads
+    __shared__ R cf[4];
+    if ((RT || IT) && tid == nt - 1) {
+        const int it      = RT ? *a.step.base + a.step.local : 0;
+        const StepCoef c0 = a.step.coef[it], c1 = a.step.coef[MODE == GZ_RT_MID ? it + 1 : it];
+        cf[0] = (R)c0.g3w, cf[1] = (R)c0.gw15;
+        cf[2] = (R)c1.g3w, cf[3] = (R)c1.gw15;
     }
     if (DIP_I) {
         // line z[m] = xa[m] + i xb[m] over the full 2nz-point spectrum: bin 0 is
         // zero, bins > nz by symmetry; stored swapped (inverse transform)
         for (int e = tid; e < NP * nz; e += nt) {
             const int p = g_div(e, nz, g.mz), m = e - p * nz + 1;
-            C xa{(R)0, (R)0}, xb{(R)0, (R)0};
-            int i, j;
-            if (2 * p < cnt) {
-                place(2 * p, i, j);
-                xa = S[((size_t)i * 2 * ny + j) * nz + (m - 1)];
-            }
-            if (2 * p + 1 < cnt) {
-                place(2 * p + 1, i, j);
-                xb = S[((size_t)i * 2 * ny + j) * nz + (m - 1)];
-            }
+            const C xa = 2 * p < cnt ? S[srow(2 * p) + m] : C{(R)0, (R)0};
+            const C xb = 2 * p + 1 < cnt ? S[srow(2 * p + 1) + m] : C{(R)0, (R)0};
             if (m == nz) {
                 sm[D + m * TD + p] = C{xb.x, xa.x}; // self-conjugate bin: real parts only
                 sm[D + p]          = C{(R)0, (R)0};
@@ -498,12 +513,9 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, 2) g_z(const
             }
         }
     }
-    if (KIN_I || DIP_I || MODE == GZ_KIN_FWD)
-        __syncthreads();
-    if (KIN_I)
-        g_tile<R>(g.k, K, T, g.lb, TK, nz, tid, nt);
-    if (DIP_I)
-        g_tile<R>(g.d, D, T, lp, TD, 2 * nz, tid, nt);
+    __syncthreads();
+    if (KIN_I || DIP_I)
+        g_tiles<R, KIN_I, DIP_I>(g.k, K, K2, g.lb, TK, g.d, D, D2, lp, TD, 2 * nz);
 
     // ---- the step on row pairs: element k of rows 2p and 2p + 1 ----------------
     double acc = 0.0;
@@ -515,6 +527,7 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, 2) g_z(const
         return;
     }
     if (MODE != GZ_KIN_FWD) {
+        const R g3 = cf[0], gw = cf[1], g3n = cf[2], gwn = cf[3];
         const R sc   = (R)(IT ? 1.0 / sqrt(a.norm_state[1]) : 1.0);
         const R wat  = (R)a.w_atoms;
         const R hdt = (R)a.half_dt, cdd = (R)a.cdd;
@@ -598,27 +611,22 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, 2) g_z(const
     }
 
     // ---- out: kinetic spectrum, then bins 1..nz of the row pairs -----------------
+    if (KIN_F || DIP_F) // the pair lines' padding half is not read
+        g_tiles<R, KIN_F, DIP_F>(g.k, K, K2, g.lb, TK, g.d, D, D2, lp, TD, nz);
     if (KIN_F) {
-        g_tile<R>(g.k, K, T, g.lb, TK, nz, tid, nt);
         for (int e = tid; e < cnt * nz; e += nt) {
             const int row = g_div(e, nz, g.mz), k = e - row * nz;
             out[e]        = sm[K + k * TK + row];
         }
     }
     if (DIP_F) {
-        g_tile<R>(g.d, D, T, lp, TD, nz, tid, nt); // the padding half is not read
         for (int e = tid; e < NP * nz; e += nt) {
             const int p = g_div(e, nz, g.mz), m = e - p * nz + 1;
             const C zm = sm[D + m * TD + p], zc = sm[D + (2 * nz - m) * TD + p];
-            int i, j;
-            if (2 * p < cnt) { // (Z_m + conj(Z_{L-m}))/2
-                place(2 * p, i, j);
-                S[((size_t)i * 2 * ny + j) * nz + (m - 1)] = C{(R)0.5 * (zm.x + zc.x), (R)0.5 * (zm.y - zc.y)};
-            }
-            if (2 * p + 1 < cnt) { // (Z_m - conj(Z_{L-m}))/(2i)
-                place(2 * p + 1, i, j);
-                S[((size_t)i * 2 * ny + j) * nz + (m - 1)] = C{(R)0.5 * (zm.y + zc.y), (R)0.5 * (zc.x - zm.x)};
-            }
+            if (2 * p < cnt) // (Z_m + conj(Z_{L-m}))/2
+                S[srow(2 * p) + m] = C{(R)0.5 * (zm.x + zc.x), (R)0.5 * (zm.y - zc.y)};
+            if (2 * p + 1 < cnt) // (Z_m - conj(Z_{L-m}))/(2i)
+                S[srow(2 * p + 1) + m] = C{(R)0.5 * (zm.y + zc.y), (R)0.5 * (zc.x - zm.x)};
         }
     }
 

@@ -36,7 +36,8 @@ struct GShape {
     int lbx, lby, lbz;    // log2 of the lines per CTA
     int ntx, nty, ntz;    // threads
     size_t smx, smy, smz; // shared memory
-    unsigned buf;         // elements of one of the z pass's three buffers
+    int mbx, mby;         // CTAs per SM the x and y kernels are compiled for
+    unsigned buf;         // elements of one of the z pass's four tiles
 };
 
 // Tiles as wide as a 128-byte row of columns (z: 32 rows), halved while a tile takes
@@ -54,10 +55,16 @@ template <class R> GShape g_shape(int nx, int ny, int nz, bool kinetic) {
         return l;
     };
     auto threads = [](const GPlan &p, int lb) {
-        int most = 1;
+        int n = 1;
         for (int s = 0; s < p.n; ++s)
-            most = std::max(most, p.f[s].nr << lb);
-        return std::min(256, std::max(64, (most + 31) / 32 * 32));
+            n = std::max(n, p.f[s].nr << lb);
+        return std::min(256, std::max(64, (n + 31) / 32 * 32));
+    };
+    auto most = [](const GPlan &p) {
+        int r = 0;
+        for (int s = 0; s < p.n; ++s)
+            r = std::max(r, p.f[s].r);
+        return r;
     };
     GShape g{};
     const GPlan px = g_plan(2 * nx, nullptr), py = g_plan(2 * ny, nullptr);
@@ -69,6 +76,7 @@ template <class R> GShape g_shape(int nx, int ny, int nz, bool kinetic) {
             --g.lbx;
         g.smx = sm(g.lbx);
         g.ntx = threads(px, g.lbx);
+        g.mbx = g_blocks<R>(most(px));
     }
     {
         auto sm = [&](int lb) { return (py.n > 2 ? 2 : 1) * c * ((size_t)(2 * ny) << lb); };
@@ -79,6 +87,7 @@ template <class R> GShape g_shape(int nx, int ny, int nz, bool kinetic) {
             --g.lby;
         g.smy = sm(g.lby);
         g.nty = threads(py, g.lby);
+        g.mby = g_blocks<R>(most(py));
     }
     {
         const int rows = nx * ny;
@@ -87,13 +96,27 @@ template <class R> GShape g_shape(int nx, int ny, int nz, bool kinetic) {
             return (size_t)nz * std::max(rw >= 4 ? rw + 1 : rw, 2 * (np >= 2 ? np + 1 : np));
         };
         g.lbz = 5;
-        while (g.lbz > 0 && (3 * c * buf(g.lbz) > want || ((rows >> g.lbz) < enough && g.lbz > 3)))
+        while (g.lbz > 0 && (4 * c * buf(g.lbz) > want || ((rows >> g.lbz) < enough && g.lbz > 3)))
             --g.lbz;
         g.buf = (unsigned)buf(g.lbz);
-        g.smz = 3 * c * (size_t)g.buf;
+        g.smz = 4 * c * (size_t)g.buf;
         g.ntz = ((size_t)nz << g.lbz) < 1024 ? 128 : 256;
     }
     return g;
+}
+
+// f(kernel): the x or y kernel for `mb` CTAs per SM
+template <class R, class F> void g_with_x(int mb, F &&f) {
+    if constexpr (sizeof(R) == 4)
+        if (mb == 3)
+            return f(g_x<R, 3>);
+    f(g_x<R, 2>);
+}
+template <class R, class F> void g_with_y(int mb, F &&f) {
+    if constexpr (sizeof(R) == 4)
+        if (mb == 3)
+            return f(g_y<R, 3>);
+    f(g_y<R, 2>);
 }
 
 } // namespace gpe

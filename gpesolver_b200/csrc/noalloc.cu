@@ -173,8 +173,9 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
             err       = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
             if (err != cudaSuccess)
                 return fail(GPE_ERR_CUDA, std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(err));
-            const void *kern[] = {(const void *)g_z<float, GZ_IT_PRO>, (const void *)g_y<float>,
-                                  (const void *)g_x<float>, (const void *)g_z<float, GZ_DIP_INV>};
+            const void *kern[] = {(const void *)g_z<float, GZ_IT_PRO>, (const void *)g_z<float, GZ_DIP_INV>,
+                                  (const void *)g_y<float, 2>, (const void *)g_y<float, 3>,
+                                  (const void *)g_x<float, 2>, (const void *)g_x<float, 3>};
             for (const void *f : kern) {
                 cudaFuncAttributes fa{};
                 err = cudaFuncGetAttributes(&fa, f);
@@ -228,10 +229,10 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
     const int wx = 1 << sh.lbx, zt = (nx * ny + (1 << sh.lbz) - 1) >> sh.lbz;
     const dim3 yt((nz + (1 << sh.lby) - 1) >> sh.lby, nx);
     g_z<float, GZ_IT_PRO><<<zt, sh.ntz, sh.smz, s>>>(z);
-    g_y<float><<<yt, sh.nty, sh.smy, s>>>(y);
-    g_x<float><<<(2 * ny * nz + wx - 1) / wx, sh.ntx, sh.smx, s>>>(x);
+    g_with_y<float>(sh.mby, [&](auto k) { k<<<yt, sh.nty, sh.smy, s>>>(y); });
+    g_with_x<float>(sh.mbx, [&](auto k) { k<<<(2 * ny * nz + wx - 1) / wx, sh.ntx, sh.smx, s>>>(x); });
     y.inverse = 1;
-    g_y<float><<<yt, sh.nty, sh.smy, s>>>(y);
+    g_with_y<float>(sh.mby, [&](auto k) { k<<<yt, sh.nty, sh.smy, s>>>(y); });
     g_z<float, GZ_DIP_INV><<<zt, sh.ntz, sh.smz, s>>>(z);
     err = cudaGetLastError();
     if (err != cudaSuccess)

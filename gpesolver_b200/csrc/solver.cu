@@ -1223,7 +1223,9 @@ template <class R> class Solver final : public SolverBase {
         a.k = kx.plan, a.d = dx.plan;
         const int w = 1 << a.lb, cols = ny * nz;
         a.tk = kin ? (cols + w - 1) / w : 0;
-        launch(g_x<R>, a.tk + (dip ? (2 * cols + w - 1) / w : 0), shape.ntx, shape.smx, s, a);
+        g_with_x<R>(shape.mbx, [&](auto k) {
+            launch(k, a.tk + (dip ? (2 * cols + w - 1) / w : 0), shape.ntx, shape.smx, s, a);
+        });
     }
     void gen_y(cudaStream_t s, bool inverse, bool kin, bool dip) {
         GYArgs a{};
@@ -1232,7 +1234,9 @@ template <class R> class Solver final : public SolverBase {
         a.k = ky.plan, a.d = dy.plan;
         const int tiles = (nz + (1 << a.lb) - 1) >> a.lb;
         a.tk            = kin ? tiles : 0;
-        launch(g_y<R>, dim3(a.tk + (dip ? tiles : 0), nx), shape.nty, shape.smy, s, a);
+        g_with_y<R>(shape.mby, [&](auto k) {
+            launch(k, dim3(a.tk + (dip ? tiles : 0), nx), shape.nty, shape.smy, s, a);
+        });
     }
     template <int MODE>
     void gen_z(cudaStream_t s, C *pin, C *pout, const StepCoef *coef, int local, int write_phi,
@@ -1474,8 +1478,8 @@ template <class R> class Solver final : public SolverBase {
                 throw Error(GPE_ERR_SIZE, "the line tiles of this grid need more shared memory than a block has");
             GPE_CUDA(cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, room));
         };
-        set((const void *)g_x<R>, shape.smx);
-        set((const void *)g_y<R>, shape.smy);
+        g_with_x<R>(shape.mbx, [&](auto k) { set((const void *)k, shape.smx); });
+        g_with_y<R>(shape.mby, [&](auto k) { set((const void *)k, shape.smy); });
         set((const void *)g_z<R, GZ_RT_PRO>, shape.smz);
         set((const void *)g_z<R, GZ_RT_MID>, shape.smz);
         set((const void *)g_z<R, GZ_RT_EPI>, shape.smz);
