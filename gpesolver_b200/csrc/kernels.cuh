@@ -126,14 +126,15 @@ __global__ void __launch_bounds__(256)
 }
 
 // ---------------------------------------------------------------------------
-// Energies (cpu_solver.cpp:137-194): per-block FP64 partials of the five sums
-// over the interior; partial layout [5][nblocks].
+// Energies (cpu_solver.cpp:137-194): the five FP64 sums over the interior, as block
+// partials [5][blocks] that the last block to finish adds up in block order into out[5]
+// (a second launch of one block that walked 5 x 1184 partials took 16 us, at any grid).
 // ---------------------------------------------------------------------------
 template <class R>
 __global__ void __launch_bounds__(256)
-    k_energy_partial(const cplx<R> *__restrict__ pin, const R *__restrict__ V,
+    k_energy(const cplx<R> *__restrict__ pin, const R *__restrict__ V,
                      const R *__restrict__ phi, const double *__restrict__ norm_state, int lazy,
-                     double *__restrict__ partial, int nx, int ny, int nz, double idx2, double idy2,
+                     double *__restrict__ partial, unsigned *ticket, double *out, int nx, int ny, int nz, double idx2, double idy2,
                      double idz2, double ggp11, double cdd, double n_atoms, double gamma) {
     const double s     = lazy ? 1.0 / sqrt(norm_state[0]) : 1.0;
     const size_t N     = (size_t)nx * ny * nz;
@@ -166,31 +167,48 @@ __global__ void __launch_bounds__(256)
                 cdd / 3. * (nrm * nrm) / 2. * (n_atoms * n_atoms);
         e[4] += 2. / 5. * gamma * (nrm * nrm * sqrt(nrm));
     }
-    __shared__ double red[5][32];
-#pragma unroll
-    for (int t = 0; t < 5; ++t) {
-        double v = e[t];
-        for (int off = 16; off > 0; off >>= 1)
-            v += __shfl_down_sync(0xffffffffu, v, off);
-        if ((threadIdx.x & 31) == 0)
-            red[t][threadIdx.x >> 5] = v;
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
+    __shared__ double red[5][8];
+    __shared__ bool last;
+    const int tid = threadIdx.x;
+    auto block_sums = [&] { // e[t] of all threads -> thread t < 5
 #pragma unroll
         for (int t = 0; t < 5; ++t) {
-            double v = threadIdx.x < (blockDim.x >> 5) ? red[t][threadIdx.x] : 0.0;
             for (int off = 16; off > 0; off >>= 1)
-                v += __shfl_down_sync(0xffffffffu, v, off);
-            if (threadIdx.x == 0)
-                partial[(size_t)t * gridDim.x + blockIdx.x] = v;
+                e[t] += __shfl_down_sync(0xffffffffu, e[t], off);
+            if ((tid & 31) == 0)
+                red[t][tid >> 5] = e[t];
         }
+        __syncthreads();
+        double v = 0;
+        if (tid < 5)
+            for (int w = 0; w < 8; ++w)
+                v += red[tid][w];
+        return v;
+    };
+    const double mine = block_sums();
+    if (tid < 5) {
+        partial[(size_t)tid * gridDim.x + blockIdx.x] = mine;
+        __threadfence();
     }
+    __syncthreads();
+    if (tid == 0)
+        last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!last)
+        return;
+    __threadfence();
+#pragma unroll
+    for (int t = 0; t < 5; ++t) {
+        e[t] = 0;
+        for (int b = tid; b < (int)gridDim.x; b += 256)
+            e[t] += ((volatile double *)partial)[(size_t)t * gridDim.x + b];
+    }
+    const double total = block_sums();
+    if (tid < 5)
+        out[tid] = total;
+    if (tid == 0)
+        *ticket = 0u;
 }
-
-// out[t] = sum over blocks of partial[t][*] (t < 5), fixed order.
-__global__ void __launch_bounds__(256)
-    k_energy_finalize(const double *__restrict__ partial, int nparts, double *__restrict__ out);
 
 // ---------------------------------------------------------------------------
 // Host-format conversion: FP64 staging <-> working precision.

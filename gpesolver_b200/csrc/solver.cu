@@ -31,26 +31,6 @@ namespace gpe {
 // ---------------------------------------------------------------------------
 // Non-template kernels
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
-    k_energy_finalize(const double *__restrict__ partial, int nparts, double *__restrict__ out) {
-    __shared__ double red[256];
-    for (int t = 0; t < 5; ++t) {
-        double acc = 0.0;
-        for (int b = threadIdx.x; b < nparts; b += blockDim.x)
-            acc += partial[(size_t)t * nparts + b];
-        red[threadIdx.x] = acc;
-        __syncthreads();
-        for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-            if (threadIdx.x < s)
-                red[threadIdx.x] += red[threadIdx.x + s];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0)
-            out[t] = red[0];
-        __syncthreads();
-    }
-}
-
 __global__ void k_advance(int *counter, int by) { counter[0] += by; }
 
 __global__ void k_set_f64(double *p, double v) { p[0] = v; }
@@ -223,6 +203,7 @@ template <class R> class Solver final : public SolverBase {
 
         nblk_elem = 148 * 8;
         epartial.alloc(5 * (size_t)nblk_elem);
+        eticket.alloc(1);
 
         build_tables();
         fused = std::is_same<R, float>::value && p.schedule == 0 && fused_dim_xy(nx) &&
@@ -474,12 +455,7 @@ template <class R> class Solver final : public SolverBase {
     }
 
     void energy(double *out) override {
-        const int nb = nblk_elem;
-        launch(k_energy_partial<R>, nb, 256, 0, cur, (const C *)psi.p, (const R *)V.p,
-               (const R *)phi.p, (const double *)(norm_state.p + 1), 1, epartial.p, nx, ny, nz,
-               1.0 / (P.dx * P.dx), 1.0 / (P.dy * P.dy), 1.0 / (P.dz * P.dz), ggp11_cur, P.cdd,
-               P.n_atoms, gamma_cur);
-        launch(k_energy_finalize, 1, 256, 0, cur, (const double *)epartial.p, nb, eout.p);
+        enqueue_energy(eout.p);
         double e[5];
         GPE_CUDA(cudaMemcpyAsync(e, eout.p, sizeof(e), cudaMemcpyDeviceToHost, cur));
         GPE_CUDA(cudaStreamSynchronize(cur));
@@ -503,17 +479,13 @@ template <class R> class Solver final : public SolverBase {
             throw Error(GPE_ERR_ARG, "iterations and checks must be positive");
         if (ehist.n < (size_t)5 * checks)
             ehist.alloc((size_t)5 * checks);
-        const int nb = nblk_elem;
         for (int c = 0; c < checks; ++c) {
             if (!lazy)
                 set_divisor_one();
             // the energy kernels between checks only read psi: one prologue
             fused_imag(k, c == 0);
             lazy = true;
-            launch(k_energy_partial<R>, nb, 256, 0, cur, (const C *)psi.p, (const R *)V.p, (const R *)phi.p,
-                   (const double *)(norm_state.p + 1), 1, epartial.p, nx, ny, nz, 1.0 / (P.dx * P.dx),
-                   1.0 / (P.dy * P.dy), 1.0 / (P.dz * P.dz), ggp11_cur, P.cdd, P.n_atoms, gamma_cur);
-            launch(k_energy_finalize, 1, 256, 0, cur, (const double *)epartial.p, nb, ehist.p + 5 * c);
+            enqueue_energy(ehist.p + 5 * c);
         }
         std::vector<double> e((size_t)5 * checks);
         GPE_CUDA(cudaMemcpyAsync(e.data(), ehist.p, sizeof(double) * e.size(), cudaMemcpyDeviceToHost, cur));
@@ -1412,7 +1384,7 @@ template <class R> class Solver final : public SolverBase {
     int y_lines = 16;                 // y-pass z columns per CTA (four-kernel schedule; autotune_x)
     DevBuf<R> vk2;
     DevBuf<double> zpartial;
-    DevBuf<unsigned> ticket;
+    DevBuf<unsigned> ticket, eticket;
     DevBuf<StepCoef> cur_coef, coef_dev;
     StepCoef host_coef{};
     StepCoef *coef_host   = nullptr;
@@ -1579,6 +1551,15 @@ template <class R> class Solver final : public SolverBase {
     }
 
     // ---- enqueue helpers (usable while capturing) ---------------------------
+    // the five sums of calc_energy into out5 (device)
+    void enqueue_energy(double *out5) {
+        // at least one point a thread, at most four blocks per SM
+        const int nb = (int)std::min<size_t>((N + 255) / 256, 148 * 4);
+        launch(k_energy<R>, nb, 256, 0, cur, (const C *)psi.p, (const R *)V.p, (const R *)phi.p,
+               (const double *)(norm_state.p + 1), 1, epartial.p, eticket.p, out5, nx, ny, nz, 1.0 / (P.dx * P.dx),
+               1.0 / (P.dy * P.dy), 1.0 / (P.dz * P.dz), ggp11_cur, P.cdd, P.n_atoms, gamma_cur);
+    }
+
     void enqueue_dipolar(cudaStream_t s, C *p) {
         gen_z<GZ_IT_PRO>(s, p, p, cur_coef.p, 0, 0);
         gen_y(s, false, false, true);
