@@ -254,6 +254,94 @@ __global__ void __launch_bounds__(NT, NX >= 256 ? 2 : 3) // 512-point lines: two
         twu, nullptr, tid);
 }
 
+// Dipolar x pencils of 2nx = 512 points as two transforms of nx = 256 each: the even
+// bins are FFT_nx(S), the odd ones FFT_nx(S w^x), w = exp(-2 pi i / 2nx), and the kept
+// half of the inverse is iFFT_nx(even) + w^-x iFFT_nx(odd).  256 points are two stages of
+// radix 16 where 512 were three of radix 8 (a third fewer trips through shared memory
+// and synchronisations, no arithmetic on the padding), and one butterfly a thread
+// needs 32 registers for its points instead of 64.  A tile holds CNT even and CNT odd lines; both
+// of a column lie in one warp, read the same addresses and are added by a shuffle.
+// Bound by instruction issue (62%).  256 x 256 x 64: 79 -> 72 us, the iteration 253 ->
+// 248 us against k3_x_dip with 8 lines, 267 against its 16 (spilled).
+template <class R, int NX, int CNT> constexpr size_t x_dip_eo_smem() {
+    return sizeof(cplx<R>) * (2 * CNT * NX + 3 * NX) + sizeof(R) * (NX + 1) * CNT;
+}
+
+template <class R, int NX, int CNT>
+__global__ void __launch_bounds__(CNT * NX / 8, CNT == 8 ? 3 : 1)
+    k3_x_dip_eo(cplx<R> *__restrict__ S, const R *__restrict__ vk, const double *__restrict__ divisor,
+                double dip_scale, int ny, int nz, Twid td, Twid tk) {
+    using C          = cplx<R>;
+    constexpr int NT = CNT * NX / 8, LN = 2 * CNT, L = 2 * NX;
+    using Fw = LinePass<-1, R, NX, LN, LN, NT, false, false, false, false, true>;
+    using Iv = LinePass<+1, R, NX, LN, LN, NT, false, true, false, false, true>;
+    static_assert(Fw::NSTG == 2 && Fw::RL == Iv::R0 && Fw::ROUNDSL == 1 && Fw::ROUNDS0 == 1 && Fw::ITEMS0 == NT &&
+                      Fw::ITEMSL == NT && 32 % LN == 0,
+                  "one butterfly a thread, both lines of a column in one warp");
+    const int tid  = threadIdx.x;
+    C *buf         = reinterpret_cast<C *>(g_smem);
+    C *w2          = buf + LN * NX;                  // exp(-2 pi i m / 2nx), m < 2nx
+    C *tws         = w2 + L;                         // exp(-2 pi i m / nx)
+    R *vs          = reinterpret_cast<R *>(tws + NX); // V_dd of |kx| = 0..NX, column b: vs[|kx| CNT + b]
+    const int cols = 2 * ny * nz;
+    const int c0   = blockIdx.x * CNT;
+    const int cnt  = min(CNT, cols - c0);
+    const size_t xs = (size_t)(ny + 1) * nz;
+    // w2 is read by the first stage's loader: its own group, waited for there
+    for (int m = tid; m < L; m += NT)
+        cp_async8(&w2[m], reinterpret_cast<const C *>(td.tw) + m);
+    cp_async_commit();
+    for (int m = tid; m < NX; m += NT)
+        cp_async8(&tws[m], reinterpret_cast<const C *>(tk.tw) + m);
+    for (int e = tid; e < (NX + 1) * CNT; e += NT) {
+        const int ix = e / CNT, b = e - ix * CNT;
+        const int c  = min(c0 + b, cols - 1);
+        const int ky = c / nz, kz = c - ky * nz;
+        const int iy = ky <= ny ? ky : 2 * ny - ky;
+        cp_async4(&vs[e], &vk[(size_t)ix * xs + (size_t)iy * nz + kz]);
+    }
+    cp_async_commit();
+    const R scale = (R)(divisor ? dip_scale / divisor[0] : dip_scale);
+    const int j = tid / LN, b2 = tid - j * LN, b = b2 % CNT, odd = b2 / CNT;
+    C a[1][Fw::R0];
+#pragma unroll
+    for (int k = 0; k < Fw::R0; ++k)
+        a[0][k] = b < cnt ? S[(size_t)(j + k * Fw::NR0) * cols + c0 + b] : C{(R)0, (R)0};
+    cp_async_wait<1>();
+    __syncthreads();
+    if (odd) {
+#pragma unroll
+        for (int k = 0; k < Fw::R0; ++k)
+            a[0][k] = cmul(a[0][k], w2[j + k * Fw::NR0]);
+    }
+    DFT<Fw::R0, -1, R, false>::run(a[0]);
+    Fw::store0(buf, a[0], j, b2);
+    cp_async_wait<0>();
+    __syncthreads();
+    Fw::loadL(buf, a[0], j, b2, tws, nullptr);
+#pragma unroll
+    for (int q = 0; q < Fw::RL; ++q) {
+        const int t  = 2 * (j + q * Fw::NSL) + odd; // bin of the 2nx points
+        const int ix = 2 * q < Fw::RL ? t : L - t;
+        a[0][q]      = cscale(a[0][q], vs[ix * CNT + b] * scale);
+    }
+    __syncthreads();
+    DFT<Iv::R0, +1, R, false>::run(a[0]);
+    Iv::store0(buf, a[0], j, b2);
+    __syncthreads();
+    Iv::loadL(buf, a[0], j, b2, tws, nullptr);
+#pragma unroll
+    for (int q = 0; q < Iv::RL; ++q) {
+        const int t = j + q * Iv::NSL;
+        C v         = a[0][q];
+        if (odd)
+            v = cmulc(v, w2[t]);
+        const C o{__shfl_xor_sync(0xffffffffu, v.x, CNT), __shfl_xor_sync(0xffffffffu, v.y, CNT)};
+        if (b < cnt && odd == (q & 1)) // the two lanes of a column share its stores
+            S[(size_t)t * cols + c0 + b] = cadd(v, o);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Y lines (one x plane per blockIdx.y; z-column tiles along blockIdx.x)
 // ---------------------------------------------------------------------------
@@ -302,329 +390,5 @@ template <class R, int N, int CNT> struct YShape {
     static constexpr int NTK = pass_threads<N, CNT>(), NTD = pass_threads<2 * N, CNT>();
     static constexpr size_t SK = xy_smem<R, N, CNT>(), SD = xy_smem<R, 2 * N, CNT>();
 };
-
-// ---------------------------------------------------------------------------
-// Z rows
-// ---------------------------------------------------------------------------
-template <class R, int NZ, int MODE>
-__global__ void __launch_bounds__(256, 4) k2_z(ZArgs a, Twid tk, Twid td) {
-    using C          = cplx<R>;
-    constexpr int NT = 256;
-    constexpr int RW = 32;          // rows per CTA
-    constexpr int NP = RW / 2;      // row pairs for the real transforms
-    constexpr int LD = 2 * NZ;      // dipolar line length
-    constexpr int TK = RW + 1;      // tile strides (odd: transposing loads avoid bank conflicts)
-    constexpr int TD = NP + 1;
-    constexpr bool RT      = MODE <= ZM_RT_EPI;
-    constexpr bool HAS_INV = (MODE == ZM_RT_MID || MODE == ZM_RT_EPI || MODE == ZM_IT_MID);
-    constexpr bool HAS_FWD = (MODE != ZM_RT_EPI);
-    const int tid          = threadIdx.x;
-    const int nx = a.nx, ny = a.ny;
-    const int rows = nx * ny;
-    const int r0   = blockIdx.x * RW;
-
-    C *kb0  = reinterpret_cast<C *>(g_smem); // kinetic tile [k][row]
-    C *db0  = kb0 + TK * NZ;                 // dipolar pair tile [m][pair]
-    R *phis = reinterpret_cast<R *>(db0 + TD * LD); // phi, then rho, [k][row]
-    R *vs   = phis + TK * NZ;                // V tile [k][row] (real time)
-    C *prs  = db0;                           // kept psi [row][k] (real time, after the C2R)
-    __shared__ double red[8];
-
-    const C *S_in = reinterpret_cast<const C *>(a.S);
-    C *S_out      = reinterpret_cast<C *>(a.S);
-    C *pr         = reinterpret_cast<C *>(a.psi_r);
-    constexpr bool KEPT = MODE == ZM_RT_MID || MODE == ZM_RT_EPI;
-
-    // real time: the kinetic tile and V are copied in (cp.async) behind the C2R
-    if (RT) {
-        const C *pin = reinterpret_cast<const C *>(a.psi_in);
-        const R *Vg  = reinterpret_cast<const R *>(a.V);
-        for (int e = tid; e < RW * NZ; e += NT) {
-            const int row = e / NZ, k = e % NZ;
-            const int rr  = r0 + row;
-            if (rr < rows) {
-                cp_async8(&kb0[row + k * TK], &pin[(size_t)rr * NZ + k]);
-                cp_async4(&vs[row + k * TK], &Vg[(size_t)rr * NZ + k]);
-            } else {
-                kb0[row + k * TK] = C{(R)0, (R)0};
-                vs[row + k * TK]  = (R)0;
-            }
-        }
-        cp_async_commit();
-    }
-
-    // ---- phi: dipolar C2R of the row pairs -------------------------------
-    if (HAS_INV) {
-        // consecutive threads take consecutive m: the spectrum rows are read
-        // contiguously (coalesced)
-        for (int e = tid; e < NP * LD; e += NT) {
-            const int m = e % LD, p = e / LD;
-            const int ra = r0 + 2 * p, rb = ra + 1;
-            C z = C{(R)0, (R)0};
-            if (m > 0 && ra < rows) {
-                const int ia = ra / ny, ja = ra - ia * ny;
-                const int mm = m <= NZ ? m : LD - m;
-                const C xa   = S_in[((size_t)ia * 2 * ny + ja) * NZ + (mm - 1)];
-                C xb         = C{(R)0, (R)0};
-                if (rb < rows) {
-                    const int ib = rb / ny, jb = rb - ib * ny;
-                    xb           = S_in[((size_t)ib * 2 * ny + jb) * NZ + (mm - 1)];
-                }
-                if (m == NZ)
-                    z = C{xa.x, xb.x}; // self-conjugate bin: real parts only
-                else if (m < NZ)
-                    z = C{xa.x - xb.y, xa.y + xb.x};   // xa + i xb
-                else
-                    z = C{xa.x + xb.y, xb.x - xa.y};   // conj(xa) + i conj(xb)
-            }
-            db0[p + m * TD] = z;
-        }
-        __syncthreads();
-        ct_fft_ip<+1, R, LD, NP, TD, NT, false, false, true>(db0, (const C *)td.tw, (const C *)td.lo, tid);
-        const C *r = db0;
-        R *phi_g = reinterpret_cast<R *>(a.phi);
-        for (int e = tid; e < RW * NZ; e += NT) {
-            const int row = e / NZ, k = e % NZ; // coalesced store along k
-            const int p = row >> 1;
-            const C zz  = r[p + k * TD];
-            const R v   = (row & 1) ? zz.y : zz.x;
-            phis[row + k * TK] = v;
-            if (r0 + row < rows)
-                phi_g[(size_t)(r0 + row) * NZ + k] = v;
-        }
-        __syncthreads();
-        if (KEPT) {
-            // the pair tile is free until the R2C: the kept psi goes there
-            for (int e = tid; e < RW * NZ; e += NT) {
-                const int row = e / NZ, k = e % NZ;
-                const int rr  = r0 + row;
-                if (rr < rows)
-                    cp_async8(&prs[e], &pr[(size_t)rr * NZ + k]);
-                else
-                    prs[e] = C{(R)0, (R)0};
-            }
-            cp_async_commit();
-        }
-    } else if (RT) {
-        // prologue: phi from the previous calc_fi3d
-        const R *phi_g = reinterpret_cast<const R *>(a.phi);
-        for (int e = tid; e < RW * NZ; e += NT) {
-            const int row = e / NZ, k = e % NZ;
-            phis[row + k * TK] = (r0 + row < rows) ? phi_g[(size_t)(r0 + row) * NZ + k] : (R)0;
-        }
-    }
-
-    // ---- psi for the physics step -----------------------------------------
-    C *kt = kb0; // tile holding psi in real space, [k][row]
-    if (RT) {
-        if (KEPT)
-            cp_async_wait<1>(); // kinetic tile and V (the kept psi may still be in flight)
-        else
-            cp_async_wait<0>();
-        __syncthreads();
-        if (MODE != ZM_RT_PRO)
-            ct_fft_ip<+1, R, NZ, RW, TK, NT>(kb0, (const C *)tk.tw, (const C *)tk.lo, tid);
-    }
-
-    double acc = 0.0;
-    if (RT) {
-        // merged potential half steps: theta = -dt/2 [cV (V + cdd phi) + g3 |psi|^2 + gw |psi|^3]
-        R cV, g3, gw;
-        {
-            const int base = *a.step.base + a.step.local;
-            const StepCoef c0 = a.step.coef[base];
-            if (MODE == ZM_RT_MID) {
-                const StepCoef c1 = a.step.coef[base + 1];
-                cV = (R)2;
-                g3 = (R)(c0.g3w + c1.g3w);
-                gw = (R)(c0.gw15 + c1.gw15);
-            } else {
-                cV = (R)1;
-                g3 = (R)c0.g3w;
-                gw = (R)c0.gw15;
-            }
-        }
-        const R hdt   = (R)a.half_dt, cdd = (R)a.cdd, wat = (R)a.w_atoms;
-        if (KEPT) {
-            cp_async_wait<0>();
-            __syncthreads();
-        }
-        for (int e = tid; e < RW * NZ; e += NT) {
-            const int row = e / NZ, k = e % NZ;
-            const int rr  = r0 + row;
-            if (rr >= rows)
-                continue;
-            const int i = rr / ny, j = rr - i * ny;
-            C p         = kt[row + k * TK];
-            if (MODE != ZM_RT_PRO)
-                p = cadd(p, prs[e]); // psi + kinetic increment
-            if (i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < NZ - 1) {
-                const R dens  = p.x * p.x + p.y * p.y;
-                const R am    = sqrt(dens);
-                const R total = cV * (vs[row + k * TK] + cdd * phis[row + k * TK]) + g3 * dens +
-                                gw * (am * am * am);
-                R s, c;
-                sincos_r<R>((R)-0.5 * hdt * total, &s, &c);
-                p = apply_wm1(p, C{(R)-2 * s * s, (R)2 * s * c});
-            }
-            kt[row + k * TK] = p;
-            if (MODE != ZM_RT_EPI)
-                pr[(size_t)rr * NZ + k] = p;
-            // rho for the next dipolar spectrum (stored in the phi tile)
-            phis[row + k * TK] = wat * (p.x * p.x + p.y * p.y);
-        }
-        __syncthreads();
-        if (MODE == ZM_RT_EPI) {
-            C *pout = reinterpret_cast<C *>(a.psi_out);
-            for (int e = tid; e < RW * NZ; e += NT) {
-                const int row = e / NZ, k = e % NZ;
-                if (r0 + row < rows)
-                    pout[(size_t)(r0 + row) * NZ + k] = kt[row + k * TK];
-            }
-            return;
-        }
-        // kinetic forward z
-        ct_fft_ip<-1, R, NZ, RW, TK, NT>(kb0, (const C *)tk.tw, (const C *)tk.lo, tid);
-        const C *kf = kb0;
-        C *pout     = reinterpret_cast<C *>(a.psi_out);
-        for (int e = tid; e < RW * NZ; e += NT) {
-            const int row = e / NZ, k = e % NZ;
-            if (r0 + row < rows)
-                pout[(size_t)(r0 + row) * NZ + k] = kf[row + k * TK];
-        }
-    } else {
-        // imaginary time: psi_in / sqrt(divisor)
-        const C *pin  = reinterpret_cast<const C *>(a.psi_in);
-        C *pout       = reinterpret_cast<C *>(a.psi_out);
-        const C *bnd  = reinterpret_cast<const C *>(a.bnd);
-        const R sc    = (R)(1.0 / sqrt(a.norm_state[1]));
-        const R wat   = (R)a.w_atoms;
-        const size_t plane = (size_t)ny * NZ;
-        if (MODE == ZM_IT_PRO) {
-            for (int e = tid; e < RW * NZ; e += NT) {
-                const int row = e / NZ, k = e % NZ;
-                const int rr  = r0 + row;
-                R rho         = (R)0;
-                if (rr < rows) {
-                    const C p = pin[(size_t)rr * NZ + k];
-                    rho       = wat * (p.x * p.x + p.y * p.y);
-                }
-                phis[row + k * TK] = rho;
-            }
-        } else {
-            const StepCoef cf = a.step.coef[0];
-            const R g3w = (R)cf.g3w, gw15 = (R)cf.gw15;
-            const R *Vg = reinterpret_cast<const R *>(a.V);
-            const R cx = (R)a.cx, cy = (R)a.cy, cz = (R)a.cz, dtau = (R)a.dtau, cdd = (R)a.cdd;
-            for (int e = tid; e < RW * NZ; e += NT) {
-                const int row = e / NZ, k = e % NZ;
-                const int rr  = r0 + row;
-                R rho         = (R)0;
-                if (rr < rows) {
-                    const int i = rr / ny, j = rr - i * ny;
-                    const size_t q = (size_t)rr * NZ + k;
-                    C o;
-                    if (i < 1 || i >= nx - 1 || j < 1 || j >= ny - 1 || k < 1 || k >= NZ - 1) {
-                        o = bnd[q];
-                    } else {
-                        const C c0 = cscale(pin[q], sc);
-                        const C xm = cscale(pin[q - plane], sc), xp = cscale(pin[q + plane], sc);
-                        const C ym = cscale(pin[q - NZ], sc), yp = cscale(pin[q + NZ], sc);
-                        const C zm = cscale(pin[q - 1], sc), zp = cscale(pin[q + 1], sc);
-                        const R vv   = Vg[q] + cdd * phis[row + k * TK];
-                        const R dens = c0.x * c0.x + c0.y * c0.y;
-                        const R am   = sqrt(dens);
-                        const R nl   = g3w * dens + gw15 * (am * am * am);
-                        const R lr   = cx * ((xm.x + xp.x) - 2 * c0.x) - cy * ((ym.x + yp.x) - 2 * c0.x) -
-                                     cz * ((zm.x + zp.x) - 2 * c0.x) + c0.x * vv + nl * c0.x;
-                        const R li = cx * ((xm.y + xp.y) - 2 * c0.y) - cy * ((ym.y + yp.y) - 2 * c0.y) -
-                                     cz * ((zm.y + zp.y) - 2 * c0.y) + c0.y * vv + nl * c0.y;
-                        o = C{c0.x - dtau * lr, c0.y - dtau * li};
-                    }
-                    pout[q] = o;
-                    acc += (double)o.x * o.x + (double)o.y * o.y;
-                    rho = wat * (o.x * o.x + o.y * o.y);
-                }
-                phis[row + k * TK] = rho;
-            }
-        }
-        __syncthreads();
-    }
-
-    // ---- dipolar R2C of rho (row pairs) -> spectrum -------------------------
-    if (HAS_FWD) {
-        // rows NZ..LD-1 are the zero padding (not read by the pruned first stage)
-        for (int e = tid; e < NP * NZ; e += NT) {
-            const int m = e % NZ, p = e / NZ;
-            db0[p + m * TD] = C{phis[2 * p + m * TK], phis[2 * p + 1 + m * TK]};
-        }
-        __syncthreads();
-        ct_fft_ip<-1, R, LD, NP, TD, NT, false, true, false>(db0, (const C *)td.tw, (const C *)td.lo, tid);
-        const C *r = db0;
-        for (int e = tid; e < RW * NZ; e += NT) {
-            const int row = e / NZ, m = e % NZ + 1; // bins 1..NZ
-            const int rr  = r0 + row;
-            if (rr >= rows)
-                continue;
-            const int p  = row >> 1;
-            const C zm   = r[p + m * TD];
-            const C zc   = r[p + (LD - m) * TD];
-            C x;
-            if ((row & 1) == 0)
-                x = C{(R)0.5 * (zm.x + zc.x), (R)0.5 * (zm.y - zc.y)};   // (Z_m + conj(Z_{L-m}))/2
-            else
-                x = C{(R)0.5 * (zm.y + zc.y), (R)0.5 * (zc.x - zm.x)};   // (Z_m - conj(Z_{L-m}))/(2i)
-            const int i = rr / ny, j = rr - i * ny;
-            S_out[((size_t)i * 2 * ny + j) * NZ + (m - 1)] = x;
-        }
-    }
-
-    // ---- norm of psi' (imaginary time): deterministic two-level reduction ---
-    if (MODE == ZM_IT_MID) {
-        for (int off = 16; off > 0; off >>= 1)
-            acc += __shfl_down_sync(0xffffffffu, acc, off);
-        if ((tid & 31) == 0)
-            red[tid >> 5] = acc;
-        __syncthreads();
-        __shared__ bool last;
-        if (tid == 0) {
-            double v = 0;
-            for (int w = 0; w < NT / 32; ++w)
-                v += red[w];
-            a.partial[blockIdx.x] = v;
-            __threadfence();
-            const unsigned t = atomicAdd(a.ticket, 1u);
-            last             = (t == gridDim.x - 1);
-        }
-        __syncthreads();
-        if (last) {
-            __threadfence();
-            double v = 0;
-            for (int b = tid; b < (int)gridDim.x; b += NT)
-                v += ((volatile double *)a.partial)[b];
-            for (int off = 16; off > 0; off >>= 1)
-                v += __shfl_down_sync(0xffffffffu, v, off);
-            if ((tid & 31) == 0)
-                red[tid >> 5] = v;
-            __syncthreads();
-            if (tid == 0) {
-                double x = 0;
-                for (int w = 0; w < NT / 32; ++w)
-                    x += red[w];
-                x *= a.dV;
-                a.norm_state[0] = x;
-                a.norm_state[1] = x;
-                if (!(x > 0.0) || !isfinite(x))
-                    a.status[0] = 1;
-                *a.ticket = 0u;
-            }
-        }
-    }
-}
-
-// Shared memory of k2_z<R, NZ, *>.
-template <class R, int NZ> constexpr size_t z_smem() {
-    return sizeof(cplx<R>) * (33 * NZ + 17 * 2 * NZ) + sizeof(R) * 2 * 33 * NZ;
-}
 
 } // namespace gpe

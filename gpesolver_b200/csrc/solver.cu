@@ -7,6 +7,7 @@
 // exported fields).
 #include "../../include/gpe_b200.h"
 #include "fused_yz.cuh"
+#include "fused_z.cuh"
 #include "general_plan.hpp"
 #include "plane_pair.cuh"
 #include "init.cuh"
@@ -773,6 +774,8 @@ template <class R> class Solver final : public SolverBase {
     // x-pass launches for nx = NN with CNT lines per CTA (the autotuned choice)
     template <int NN, int CNT, class Set> static void set_x_attrs(Set &set) {
         set((const void *)k3_x_kin<R, NN, CNT, pass_threads<NN, CNT>()>, xy_smem<R, NN, CNT>());
+        if constexpr (NN == 256)
+            set((const void *)k3_x_dip_eo<R, NN, CNT>, x_dip_eo_smem<R, NN, CNT>());
         set((const void *)k3_x_dip<R, NN, CNT, pass_threads<2 * NN, CNT>()>, x_dip_smem<R, NN, CNT>());
     }
     template <int NN, int CNT> void launch_xk(cudaStream_t s) {
@@ -781,9 +784,20 @@ template <class R> class Solver final : public SolverBase {
                (const C *)ex.p, (const C *)ey.p, (const C *)ez.p, inv_hi, inv_lo, ny, nz, twid(kx));
     }
     template <int NN, int CNT> void launch_xd(cudaStream_t s, const double *divisor, double dscale) {
+        const int tiles = (2 * ny * nz + CNT - 1) / CNT;
+        if constexpr (NN == 256) {
+            // split lines where a CTA's instructions count, three waves of CTAs and more;
+            // fewer leave each SM to one CTA's latency, which k3_x_dip has less of
+            // (256 x 32 x 16: 14.9 against 16.1 us a real-time iteration)
+            if (tiles >= 3 * 148) {
+                launch(k3_x_dip_eo<R, NN, CNT>, tiles, CNT * NN / 8, x_dip_eo_smem<R, NN, CNT>(), s, S2.p,
+                       (const R *)vk2.p, divisor, dscale, ny, nz, twid(dx), twid(kx));
+                return;
+            }
+        }
         constexpr int NT = pass_threads<2 * NN, CNT>();
-        launch(k3_x_dip<R, NN, CNT, NT>, (2 * ny * nz + CNT - 1) / CNT, NT, x_dip_smem<R, NN, CNT>(), s, S2.p,
-               (const R *)vk2.p, divisor, dscale, ny, nz, twid(dx));
+        launch(k3_x_dip<R, NN, CNT, NT>, tiles, NT, x_dip_smem<R, NN, CNT>(), s, S2.p, (const R *)vk2.p, divisor,
+               dscale, ny, nz, twid(dx));
     }
     template <int NN> void f_x_n(cudaStream_t s, bool kin, const double *divisor, int part, double dscale) {
         if (kin) {
