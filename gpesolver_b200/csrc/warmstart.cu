@@ -375,7 +375,7 @@ struct WgTile {
 };
 
 template <int OT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
     k_up_wgrad(const float *__restrict__ in, const float *__restrict__ gy, float *__restrict__ partial,
                float *__restrict__ bpartial, ConvGeom g, WgTile w, size_t in_stride, size_t g_stride) {
     extern __shared__ __align__(16) float wg_smem[];
@@ -406,30 +406,40 @@ __global__ void __launch_bounds__(256)
         const int x0 = bx * w.tx, y0 = by * w.ty, z0 = bz * w.tz;
         const float *inb = in + smp * in_stride, *gyb = gy + smp * g_stride;
         __syncthreads(); // the previous tile's reads
-        // u: one row of z per warp and step
-        const int hy = w.ty + 2, hx = w.tx + 2;
-        for (int row = warp; row < 8 * hx * hy; row += 8) {
-            const int c = row / (hx * hy), q = row - c * hx * hy, xl = q / hy, yl = q - xl * hy;
-            const int x = x0 + xl - 1, y = y0 + yl - 1;
-            const bool ok = c0 + c < g.cin && x >= 0 && x < Xi && y >= 0 && y < Yi;
-            const float *src = inb + ((size_t)(c0 + c) * Xi + x) * Yi * Zi + (size_t)y * Zi;
-            for (int zl = lane; zl < w.tz + 2; zl += 32) {
-                const int z = z0 + zl - 1;
-                us[c * w.cs + xl * w.xs + yl * w.ys + zl] = ok && z >= 0 && z < Zi ? __ldg(&src[z]) : 0.f;
-            }
+        // u: a channel per warp, one row of z per step
+        {
+            const bool cok   = c0 + warp < g.cin;
+            const float *src = inb + ((size_t)(c0 + warp) * Xi + x0 - 1) * Yi * Zi + (ptrdiff_t)(y0 - 1) * Zi + z0 - 1;
+            const bool zok   = z0 + lane - 1 >= 0 && z0 + lane - 1 < Zi; // tz + 2 <= 18 lanes
+            float *dst       = us + warp * w.cs + lane;
+            for (int xl = 0; xl < w.tx + 2; ++xl)
+#pragma unroll 2
+                for (int yl = 0; yl < w.ty + 2; ++yl) {
+                    const bool ok = cok && zok && (unsigned)(x0 + xl - 1) < (unsigned)Xi &&
+                                    (unsigned)(y0 + yl - 1) < (unsigned)Yi;
+                    if (lane < w.tz + 2)
+                        dst[xl * w.xs + yl * w.ys] = ok ? __ldg(&src[(xl * Yi + yl) * Zi + lane]) : 0.f;
+                }
         }
-        // gy: lanes take the output channels first (conflict-free stores)
-        for (int row = warp; row < 4 * w.tx * w.ty; row += 8) {
-            const int p = row & 3, q = row >> 2, xl = q / w.ty, yl = q - xl * w.ty;
-            const int x = 2 * (x0 + xl) + (p >> 1), y = 2 * (y0 + yl) + (p & 1);
-            const bool ok = x < g.X && y < g.Y;
-            const float *src = gyb + ((size_t)(o0 + lane % OT) * g.X + x) * g.Y * g.Z + (size_t)y * g.Z + 2 * z0;
-            float *dst = gs + (size_t)(p * nvox + q * w.tz) * 2 * OT;
-            for (int fz = lane / OT; fz < 2 * w.tz; fz += 32 / OT) {
-                const float v = ok && 2 * z0 + fz < g.Z ? __ldg(&src[fz]) : 0.f;
-                dst[fz * OT + lane % OT] = v;
-                bsum += v;
-            }
+        // gy: an (x, y) parity per pair of warps; lanes take the output channels first
+        // (conflict-free stores)
+        {
+            const int o      = lane % OT, f0 = lane / OT;
+            const float *src = gyb + ((size_t)(o0 + o) * g.X + 2 * x0 + px) * g.Y * g.Z + (size_t)(2 * y0 + py) * g.Z +
+                               2 * z0;
+            float *dst = gs + (size_t)pxy * nvox * 2 * OT + o;
+            for (int xl = 0; xl < w.tx; ++xl)
+                for (int yl = half; yl < w.ty; yl += 2) {
+                    const bool ok  = 2 * (x0 + xl) < g.X && 2 * (y0 + yl) < g.Y;
+                    const float *r = src + (size_t)(2 * xl * g.Y + 2 * yl) * g.Z;
+                    float *d       = dst + (xl * w.ty + yl) * w.tz * 2 * OT;
+#pragma unroll 4
+                    for (int fz = f0; fz < 2 * w.tz; fz += 32 / OT) {
+                        const float v = ok && 2 * z0 + fz < g.Z ? __ldg(&r[fz]) : 0.f;
+                        d[fz * OT]    = v;
+                        bsum += v;
+                    }
+                }
         }
         __syncthreads();
         for (int row = half; row < w.tx * w.ty; row += 2) {
@@ -491,6 +501,25 @@ __global__ void __launch_bounds__(256)
     }
 }
 
+// First level of the parts' sum where there are many: parts p = blockIdx.y, blockIdx.y +
+// gridDim.y, ... of every element into out[blockIdx.y] (one block per channel alone walked 444
+// parts in 44 us).
+__global__ void __launch_bounds__(256)
+    k_sum_parts(const float *__restrict__ partial, float *__restrict__ out, int n, int nparts) {
+    const int e = blockIdx.x * 256 + threadIdx.x;
+    if (e >= n)
+        return;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    int p      = blockIdx.y;
+    for (; p + 3 * (int)gridDim.y < nparts; p += 4 * gridDim.y)
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            s[k] += partial[(size_t)(p + k * gridDim.y) * n + e];
+    for (; p < nparts; p += gridDim.y)
+        s[0] += partial[(size_t)p * n + e];
+    out[(size_t)blockIdx.y * n + e] = (s[0] + s[1]) + (s[2] + s[3]);
+}
+
 // Sums the CTAs' parts of one input channel (blockIdx.x) and output-channel
 // group (blockIdx.y), then unfolds the 64 products into the 27 tap gradients:
 // tap -1 of an axis collects k = 2, 3, tap 0 k = 1, 2, tap 1 k = 0, 1.
@@ -499,7 +528,7 @@ template <int OT> constexpr int up_reduce_slices() { return 1024 / (64 * OT) > 4
 template <int OT>
 __global__ void __launch_bounds__(64 * OT * up_reduce_slices<OT>())
     k_up_wgrad_reduce(const float *__restrict__ partial, const float *__restrict__ bpartial, float *__restrict__ dW,
-                      float *__restrict__ db, int cout, int cin, int ncg, int nparts) {
+                      float *__restrict__ db, int cout, int cin, int ncg, int nparts, int nbparts) {
     constexpr int SL = up_reduce_slices<OT>();
     __shared__ float red[SL][64 * OT];
     const int c = blockIdx.x, og = blockIdx.y, tid = threadIdx.x;
@@ -532,7 +561,7 @@ __global__ void __launch_bounds__(64 * OT * up_reduce_slices<OT>())
     if (c == 0 && tid < 32)
         for (int o = 0; o < OT; ++o) {
             float b = 0.f;
-            for (int q = tid; q < nparts; q += 32)
+            for (int q = tid; q < nbparts; q += 32)
                 b += bpartial[(size_t)q * cout + og * OT + o];
             for (int off = 16; off > 0; off >>= 1)
                 b += __shfl_down_sync(0xffffffffu, b, off);
@@ -547,7 +576,7 @@ __global__ void __launch_bounds__(64 * OT * up_reduce_slices<OT>())
 // sums in registers: 9 loads (L1) and 27 multiply-adds per voxel.  The block's
 // sums meet in shared memory.  8 channels, 128 x 128 x 32, 8 samples: 4.2 ms -> 250 us.
 //  blockIdx.x = column block x segment, z = sample.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 3)
     k_last_wgrad(const float *__restrict__ in, const float *__restrict__ gy, float *__restrict__ partial,
                  ConvGeom g, int sx, int nseg, size_t in_stride, size_t g_stride) {
     __shared__ float red[28][257];
@@ -570,21 +599,29 @@ __global__ void __launch_bounds__(256)
         w[1][k] = ok[k] && x0 < g.X ? __ldg(&u[(size_t)x0 * cols + col + off]) : 0.f;
     }
     // sx is a multiple of 3: the window's planes rotate by renaming
+    const float *r[3], *gp = gyb + (size_t)x0 * cols + col;
+#pragma unroll
+    for (int d = 0; d < 3; ++d)
+        r[d] = u + (size_t)(x0 + 1) * cols + col + (d - 1) * g.Z;
 #pragma unroll 1
     for (int xb = x0; xb < x1; xb += 3) {
 #pragma unroll
         for (int s = 0; s < 3; ++s) {
-            const int x = xb + s;
-            const float gv = col < cols && x < x1 ? __ldg(&gyb[(size_t)x * cols + col]) : 0.f;
+            const int x    = xb + s;
+            const bool in  = x + 1 < g.X;
+            const float gv = col < cols && x < x1 ? __ldg(gp) : 0.f;
             gsum += gv;
 #pragma unroll
             for (int k = 0; k < 9; ++k) {
-                const int off = (k / 3 - 1) * g.Z + k % 3 - 1;
-                w[(s + 2) % 3][k] = ok[k] && x + 1 < g.X ? __ldg(&u[(size_t)(x + 1) * cols + col + off]) : 0.f;
+                w[(s + 2) % 3][k] = ok[k] && in ? __ldg(r[k / 3] + k % 3 - 1) : 0.f;
 #pragma unroll
                 for (int d = 0; d < 3; ++d)
                     acc[d][k] = fmaf(gv, w[(s + d) % 3][k], acc[d][k]);
             }
+            gp += cols;
+#pragma unroll
+            for (int d = 0; d < 3; ++d)
+                r[d] += cols;
         }
     }
 #pragma unroll
@@ -732,13 +769,12 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         const int yy = y + k / 3 - 1, zz = z + k % 3 - 1;
-        if (yy < 0 || yy >= g.Y || zz < 0 || zz >= g.Z)
-            continue;
+        const bool ok = yy >= 0 && yy < g.Y && zz >= 0 && zz < g.Z;
         float gv[RX + 2];
 #pragma unroll
         for (int r = 0; r < RX + 2; ++r) {
             const int x = x0 + r - 1;
-            gv[r] = x >= 0 && x < g.X ? __ldg(gyb + (size_t)x * cols + (k / 3 - 1) * g.Z + k % 3 - 1) : 0.f;
+            gv[r] = ok && x >= 0 && x < g.X ? __ldg(gyb + (size_t)x * cols + (k / 3 - 1) * g.Z + k % 3 - 1) : 0.f;
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d)
@@ -917,10 +953,12 @@ void forward(gpe_warm *W, int B, float *amp, bool training) {
         };
         using I1 = std::integral_constant<int, 1>;
         using I2 = std::integral_constant<int, 2>;
-        // two voxels and eight channels a thread where that still leaves 512
-        // threads per SM, else one voxel and two channels (or one)
+        // two voxels and eight channels a thread where that still leaves 512 threads
+        // per SM, one voxel and four channels where that does, else two (or one)
         if (Xi % 2 == 0 && L.cout >= 8 && (size_t)nvox / 2 * 4 * (L.cout / 8) * B >= 148 * 512)
             go(std::integral_constant<int, 8>{}, I2{});
+        else if (L.cout >= 4 && (size_t)nvox * 4 * (L.cout / 4) * B >= 148 * 512)
+            go(std::integral_constant<int, 4>{}, I1{});
         else if (L.cout >= 2)
             go(I2{}, I1{});
         else
@@ -962,21 +1000,22 @@ size_t wg_smem(const gpe::WgTile &w, int ot) {
     return sizeof(float) * (((size_t)8 * w.cs + 3) / 4 * 4 + std::max<size_t>(gs, (size_t)512 * ot));
 }
 int wg_ot(const gpe_warm::Layer &L) { return std::min(L.cout, 8); }
-// CTAs along the tiles: up to four per SM over all channel groups
-int wg_parts(const gpe::WgTile &w, int pairs) { return std::min(w.ntile, std::max(1, 148 * 4 / pairs)); }
+// CTAs along the tiles: up to three per SM (all resident) over all channel groups
+int wg_parts(const gpe::WgTile &w, int pairs) { return std::min(w.ntile, std::max(1, 148 * 3 / pairs)); }
 // planes per segment of the last layer's gradient (a multiple of 3) and segments
 int last_segments(const gpe_warm::Layer &L) { return (L.g.X + 32) / 33; }
 int last_segment(const gpe_warm::Layer &L) {
     const int n = last_segments(L);
     return ((L.g.X + n - 1) / n + 2) / 3 * 3;
 }
+constexpr int kSumSlices = 16; // of the parts, in their sum's first level
 // floats of partial sums that layer l's weight gradient needs
 size_t wg_partial(const gpe_warm::Layer &L, int B) {
     if (!L.g.up)
         return (size_t)B * last_segments(L) * (((size_t)L.g.Y * L.g.Z + 255) / 256) * L.cin * 28;
     const gpe::WgTile w = wg_tile(L, B);
     const int ot = wg_ot(L), pairs = w.ncg * (L.cout / ot);
-    return (size_t)wg_parts(w, pairs) * ((size_t)pairs * 512 * ot + L.cout);
+    return (size_t)wg_parts(w, pairs) * ((size_t)pairs * 512 * ot + L.cout) + (size_t)kSumSlices * pairs * 512 * ot;
 }
 
 // weight and bias gradients of layer l from its input and dL/d(pre-activation)
@@ -998,8 +1037,12 @@ void conv_wgrad(gpe_warm *W, int l, int B, const float *in, size_t in_stride, co
         float *bp = W->partial.p + (size_t)parts * pairs * 512 * OT;
         gpe::k_up_wgrad<OT><<<dim3(parts, pairs), 256, wg_smem(w, OT), s>>>(in, gy, W->partial.p, bp, L.g, w,
                                                                             in_stride, g_stride);
+        const int n   = pairs * 512 * OT, lvl = parts > 4 * kSumSlices ? kSumSlices : parts;
+        float *sums   = lvl < parts ? bp + (size_t)parts * L.cout : W->partial.p;
+        if (lvl < parts)
+            gpe::k_sum_parts<<<dim3((n + 255) / 256, lvl), 256, 0, s>>>(W->partial.p, sums, n, parts);
         gpe::k_up_wgrad_reduce<OT><<<dim3(L.cin, nog), 64 * OT * gpe::up_reduce_slices<OT>(), 0, s>>>(
-            W->partial.p, bp, W->grad.p + L.w, W->grad.p + L.b, L.cout, L.cin, w.ncg, parts);
+            sums, bp, W->grad.p + L.w, W->grad.p + L.b, L.cout, L.cin, w.ncg, lvl, parts);
     });
 }
 
@@ -1024,10 +1067,12 @@ void conv_xgrad(gpe_warm *W, int l, int B, const float *gy, size_t g_stride, con
     };
     using I1 = std::integral_constant<int, 1>;
     using I2 = std::integral_constant<int, 2>;
-    // two voxels and eight channels a thread where that still leaves 512 threads
-    // per SM, else one voxel and two channels (or one)
-    if (Xi % 2 == 0 && L.cin >= 8 && (size_t)nvox / 2 * (L.cin / 8) * B >= 148 * 512)
+    // two voxels and eight channels a thread where that still leaves 256 threads
+    // per SM, one voxel and four channels where that does, else two (or one)
+    if (Xi % 2 == 0 && L.cin >= 8 && (size_t)nvox / 2 * (L.cin / 8) * B >= 148 * 256)
         go(std::integral_constant<int, 8>{}, I2{});
+    else if (L.cin >= 4 && (size_t)nvox * (L.cin / 4) * B >= 148 * 256)
+        go(std::integral_constant<int, 4>{}, I1{});
     else if (L.cin >= 2)
         go(I2{}, I1{});
     else
