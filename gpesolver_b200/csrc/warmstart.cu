@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(128)
 // along x, whose windows share their loads (L1); lanes take neighbouring (y, z)
 // columns.  Bound by the L1 reads (54 per 108 multiply-adds): 448 -> 182 us at 8
 // channels, 128 x 128 x 32, 8 samples (one voxel a thread, staged tiles, before).
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 8)
     k_last_fwd(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ W,
                const __nv_bfloat16 *__restrict__ bias, float *__restrict__ out, ConvGeom g, size_t in_stride) {
     constexpr int RX = 4;
@@ -769,12 +769,13 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
         const int yy = y + k / 3 - 1, zz = z + k % 3 - 1;
-        const bool ok = yy >= 0 && yy < g.Y && zz >= 0 && zz < g.Z;
+        if (yy < 0 || yy >= g.Y || zz < 0 || zz >= g.Z)
+            continue;
         float gv[RX + 2];
 #pragma unroll
         for (int r = 0; r < RX + 2; ++r) {
             const int x = x0 + r - 1;
-            gv[r] = ok && x >= 0 && x < g.X ? __ldg(gyb + (size_t)x * cols + (k / 3 - 1) * g.Z + k % 3 - 1) : 0.f;
+            gv[r] = x >= 0 && x < g.X ? __ldg(gyb + (size_t)x * cols + (k / 3 - 1) * g.Z + k % 3 - 1) : 0.f;
         }
 #pragma unroll
         for (int d = 0; d < 3; ++d)
@@ -786,15 +787,24 @@ __global__ void __launch_bounds__(128)
                     acc[r][c] = fmaf(wc, gv[r + d], acc[r][c]);
             }
     }
+    // SiLU' of four channels' voxels at a time: their reads of `pre` together
+    constexpr int CB = CT < 4 ? CT : 4;
 #pragma unroll
-    for (int c = 0; c < CT; ++c)
+    for (int cb = 0; cb < CT; cb += CB) {
+        float pv[CB][RX];
+        const size_t q0 = blockIdx.z * dx_stride + ((size_t)(c0 + cb) * g.X + x0) * cols + col;
 #pragma unroll
-        for (int r = 0; r < RX; ++r) {
-            if (x0 + r >= g.X)
-                break;
-            const size_t q = blockIdx.z * dx_stride + ((size_t)(c0 + c) * g.X + x0 + r) * cols + col;
-            dx[q]          = acc[r][c] * silu_grad(pre_in[q]);
-        }
+        for (int c = 0; c < CB; ++c)
+#pragma unroll
+            for (int r = 0; r < RX; ++r)
+                pv[c][r] = x0 + r < g.X ? __ldg(&pre_in[q0 + ((size_t)c * g.X + r) * cols]) : 0.f;
+#pragma unroll
+        for (int c = 0; c < CB; ++c)
+#pragma unroll
+            for (int r = 0; r < RX; ++r)
+                if (x0 + r < g.X)
+                    dx[q0 + ((size_t)c * g.X + r) * cols] = acc[r][cb + c] * silu_grad(pv[c][r]);
+    }
 }
 
 // loss partials of (u - target)^2 per block and gu = dL/du = 2 (u - t) / (B n)
