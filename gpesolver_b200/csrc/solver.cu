@@ -34,7 +34,7 @@ namespace gpe {
 // ---------------------------------------------------------------------------
 __global__ void k_advance(int *counter, int by) { counter[0] += by; }
 
-__global__ void k_set_f64(double *p, double v) { p[0] = v; }
+__global__ void k_set_coef(StepCoef *p, StepCoef c) { p[0] = c; }
 
 // ---------------------------------------------------------------------------
 // Error helpers
@@ -63,6 +63,33 @@ template <class T> struct DevBuf {
     ~DevBuf() {
         if (p)
             cudaFree(p);
+    }
+};
+
+// Pinned host memory that kernels write (h and p are the same memory, host and device
+// address): results the host reads after a stream synchronisation, without a copy of
+// their own.
+template <class T> struct MappedBuf {
+    T *h     = nullptr;
+    T *p     = nullptr;
+    size_t n = 0;
+    void alloc(size_t count) {
+        if (h)
+            cudaFreeHost(h);
+        h = p = nullptr;
+        GPE_CUDA(cudaHostAlloc(&h, sizeof(T) * count, cudaHostAllocMapped | cudaHostAllocPortable));
+        GPE_CUDA(cudaHostGetDevicePointer(&p, h, 0));
+        n = count;
+        clear();
+    }
+    void clear() {
+        for (size_t i = 0; i < n; ++i)
+            ((volatile T *)h)[i] = T(0);
+    }
+    T operator[](size_t i) const { return ((const volatile T *)h)[i]; }
+    ~MappedBuf() {
+        if (h)
+            cudaFreeHost(h);
     }
 };
 
@@ -431,11 +458,10 @@ template <class R> class Solver final : public SolverBase {
         set_divisor_one();
         if (!to_host)
             return 0.0;
-        double x = 0;
-        GPE_CUDA(cudaMemcpyAsync(&x, norm_state.p, sizeof(double), cudaMemcpyDeviceToHost, cur));
-        GPE_CUDA(cudaMemsetAsync(status.p, 0, sizeof(int), cur));
+        GPE_CUDA(cudaMemcpyAsync(eout.h, norm_state.p, sizeof(double), cudaMemcpyDeviceToHost, cur));
         GPE_CUDA(cudaStreamSynchronize(cur));
-        return x;
+        ((volatile int *)status.h)[0] = 0;
+        return eout[0];
     }
 
     void normalize() override {
@@ -457,9 +483,8 @@ template <class R> class Solver final : public SolverBase {
 
     void energy(double *out) override {
         enqueue_energy(eout.p);
-        double e[5];
-        GPE_CUDA(cudaMemcpyAsync(e, eout.p, sizeof(e), cudaMemcpyDeviceToHost, cur));
         GPE_CUDA(cudaStreamSynchronize(cur));
+        const double e[5] = {eout[0], eout[1], eout[2], eout[3], eout[4]};
         // Post-scaling of CpuGrossPitaevskiSolver::calc_energy (cpu_solver.cpp:185-191).
         const double dV = P.dx * P.dy * P.dz, w = P.n_atoms;
         out[0]          = e[0] * (dV / (2 * P.m) * w);
@@ -483,17 +508,18 @@ template <class R> class Solver final : public SolverBase {
         for (int c = 0; c < checks; ++c) {
             if (!lazy)
                 set_divisor_one();
-            // the energy kernels between checks only read psi: one prologue
-            fused_imag(k, c == 0);
+            // the energy kernels between checks only read psi: one prologue.  After the
+            // two-CTA kernel it runs again: its spectrum agrees with the prologue's (a
+            // one-CTA kernel's) to rounding only, and this history is that of
+            // imag_steps(k) + calc_energy() to the bit.
+            fused_imag(k, c == 0 || pair_it);
             lazy = true;
             enqueue_energy(ehist.p + 5 * c);
         }
-        std::vector<double> e((size_t)5 * checks);
-        GPE_CUDA(cudaMemcpyAsync(e.data(), ehist.p, sizeof(double) * e.size(), cudaMemcpyDeviceToHost, cur));
         check_status();
         const double dV = P.dx * P.dy * P.dz, w = P.n_atoms;
         for (int c = 0; c < checks; ++c) {
-            const double *x = &e[(size_t)5 * c];
+            const volatile double *x = ehist.h + (size_t)5 * c;
             e_total[c] = x[0] * (dV / (2 * P.m) * w) + x[1] * (dV * w) + x[2] * (dV * std::pow(w, 2)) + x[3] * dV +
                          x[4] * (dV * std::pow(w, 2.5));
             if (!std::isfinite(e_total[c]))
@@ -502,12 +528,15 @@ template <class R> class Solver final : public SolverBase {
     }
 
     void set_coeffs(double ggp11, double gamma) override {
+        put_coeffs(ggp11, gamma);
+        GPE_CUDA(cudaStreamSynchronize(cur));
+    }
+    // set_coeffs in stream order, without waiting
+    void put_coeffs(double ggp11, double gamma) {
         ggp11_cur = ggp11;
         gamma_cur = gamma;
-        StepCoef c{(ggp11 - P.cdd / 3) * P.n_atoms, gamma * P.w_15};
-        host_coef = c;
-        GPE_CUDA(cudaMemcpyAsync(cur_coef.p, &host_coef, sizeof(StepCoef), cudaMemcpyHostToDevice, cur));
-        GPE_CUDA(cudaStreamSynchronize(cur));
+        host_coef = StepCoef{(ggp11 - P.cdd / 3) * P.n_atoms, gamma * P.w_15};
+        launch(k_set_coef, 1, 1, 0, cur, cur_coef.p, host_coef);
     }
 
     // ---- fused iterations ---------------------------------------------------
@@ -537,7 +566,7 @@ template <class R> class Solver final : public SolverBase {
             }
             coef_host[t] = StepCoef{(g - P.cdd / 3) * P.n_atoms, gm * P.w_15};
             if (t == k - 1 && !P.const_edd)
-                set_coeffs(g, gm);
+                put_coeffs(g, gm);
         }
         GPE_CUDA(cudaMemcpyAsync(coef_dev.p, coef_host, sizeof(StepCoef) * k, cudaMemcpyHostToDevice, cur));
         GPE_CUDA(cudaEventRecord(coef_event, cur));
@@ -1019,10 +1048,10 @@ template <class R> class Solver final : public SolverBase {
             GPE_CUDA(cudaMemsetAsync(psir.p, 0, sizeof(C) * N, cur));
             GPE_CUDA(cudaMemsetAsync(S2.p, 0, sizeof(C) * S2.n, cur));
             GPE_CUDA(cudaMemsetAsync(phi.p, 0, sizeof(R) * N, cur));
-            GPE_CUDA(cudaMemsetAsync(status.p, 0, sizeof(int) * 4, cur));
             GPE_CUDA(cudaMemcpyAsync(norm_state.p, one_buf.p, sizeof(double), cudaMemcpyDeviceToDevice, cur));
             set_divisor_one();
             GPE_CUDA(cudaStreamSynchronize(cur));
+            status.clear();
             if (!fix_w) // only measured choices are shared
                 chosen_p[keyp] = (pair_rt ? 1 : 0) | (pair_it ? 2 : 0) | (it_wide ? 0 : 4);
         }
@@ -1377,12 +1406,14 @@ template <class R> class Solver final : public SolverBase {
     Line kz, ky, kx, dz, dy, dx;
     DevBuf<C> psi, psii, bnd, ex, ey, ez;
     DevBuf<R> V, phi;
-    DevBuf<double> staging, norm_state, epartial, eout;
+    DevBuf<double> staging, norm_state, epartial;
+    MappedBuf<double> eout;    // energies, norm
     DevBuf<double> export_buf; // asynchronous exports
-    DevBuf<double> ehist;      // energy history of imag_steps_energies
+    MappedBuf<double> ehist;   // energy history of imag_steps_energies
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev_widened = nullptr, ev_copied = nullptr;
-    DevBuf<int> status, iter_zero, iter_base;
+    DevBuf<int> iter_zero, iter_base;
+    MappedBuf<int> status;
     // fused pipeline (compile-time line lengths; complex64 only)
     bool fused = false;
     // middle real- / imaginary-time iterations on the two-CTA plane kernels
@@ -1524,11 +1555,10 @@ template <class R> class Solver final : public SolverBase {
     // status[0]: a non-finite or non-positive norm; status[1]: a bulk copy into
     // shared memory that a plane kernel stopped waiting for
     void check_status() {
-        int st[2] = {0, 0};
-        GPE_CUDA(cudaMemcpyAsync(st, status.p, sizeof(st), cudaMemcpyDeviceToHost, cur));
         GPE_CUDA(cudaStreamSynchronize(cur));
+        const int st[2] = {status[0], status[1]};
         if (st[0] != 0 || st[1] != 0) {
-            GPE_CUDA(cudaMemset(status.p, 0, sizeof(st)));
+            status.clear();
             if (st[1] != 0)
                 throw Error(GPE_ERR_CUDA, "a plane kernel's bulk copy into shared memory did not complete");
             throw Error(GPE_ERR_NUMERIC, "non-finite or non-positive norm of psi");
@@ -1565,7 +1595,7 @@ template <class R> class Solver final : public SolverBase {
     }
 
     // ---- enqueue helpers (usable while capturing) ---------------------------
-    // the five sums of calc_energy into out5 (device)
+    // the five sums of calc_energy into out5 (device address)
     void enqueue_energy(double *out5) {
         // at least one point a thread, at most four blocks per SM
         const int nb = (int)std::min<size_t>((N + 255) / 256, 148 * 4);
