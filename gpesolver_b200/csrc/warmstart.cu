@@ -177,6 +177,23 @@ struct ConvGeom {
 
 constexpr int kMaxCout = 32;
 
+// acc[n] += w[n] u: two channels per instruction (packed FP32x2, each with the scalar
+// rounding)
+template <int N> __device__ __forceinline__ void axpy(float (&acc)[N], const float *w, float u) {
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int n = 0; n < N; n += 2) {
+            const float2 a = __ffma2_rn(float2{w[n], w[n + 1]}, float2{u, u}, float2{acc[n], acc[n + 1]});
+            acc[n]         = a.x;
+            acc[n + 1]     = a.y;
+        }
+    } else {
+#pragma unroll
+        for (int n = 0; n < N; ++n)
+            acc[n] = fmaf(w[n], u, acc[n]);
+    }
+}
+
 // Folded weights of the upsampling convolutions, refreshed whenever the BF16
 // weights change.  Of the 27 fine taps an output voxel reads, the nearest
 // upsampling makes 1, 2, 4 or 8 meet in one coarse voxel: per axis an output of
@@ -273,13 +290,13 @@ __global__ void __launch_bounds__(128)
         for (int k = 0; k < 16; ++k) {
             const int tx = k >> 3, ty = (k >> 2) & 1, pz = (k >> 1) & 1, tz = k & 1;
             const float *w = uf_ws + (size_t)(c * 16 + k) * OT;
+            float wo[OT];
 #pragma unroll
-            for (int o = 0; o < OT; ++o) {
-                const float wo = w[o];
+            for (int o = 0; o < OT; ++o)
+                wo[o] = w[o];
 #pragma unroll
-                for (int v = 0; v < VX; ++v)
-                    acc[v][pz][o] = fmaf(wo, u[v + tx][ty][pz + tz], acc[v][pz][o]);
-            }
+            for (int v = 0; v < VX; ++v)
+                axpy(acc[v][pz], wo, u[v + tx][ty][pz + tz]);
         }
     }
 #pragma unroll
@@ -458,13 +475,10 @@ __global__ void __launch_bounds__(256, 3)
                 } else {
                     ga[0] = gr[z * 2], ga[1] = gr[z * 2 + 1];
                 }
-#pragma unroll
-                for (int o = 0; o < OT; ++o) {
-                    acc[0][o] = fmaf(ga[o], u0, acc[0][o]);
-                    acc[1][o] = fmaf(ga[o], u1, acc[1][o]);
-                    acc[2][o] = fmaf(ga[OT + o], u1, acc[2][o]);
-                    acc[3][o] = fmaf(ga[OT + o], u2, acc[3][o]);
-                }
+                axpy(acc[0], ga, u0);
+                axpy(acc[1], ga, u1);
+                axpy(acc[2], ga + OT, u1);
+                axpy(acc[3], ga + OT, u2);
                 u0 = u1;
                 u1 = u2;
             }
@@ -722,13 +736,13 @@ __global__ void __launch_bounds__(128)
 #pragma unroll
                 for (int d = 0; d < 4; ++d) {
                     const float *w = xg_ws + (size_t)(o * 64 + (kx * 4 + b) * 4 + d) * CT;
+                    float wc[CT];
 #pragma unroll
-                    for (int c = 0; c < CT; ++c) {
-                        const float wc = w[c];
+                    for (int c = 0; c < CT; ++c)
+                        wc[c] = w[c];
 #pragma unroll
-                        for (int v = 0; v < VX; ++v)
-                            acc[v][c] = fmaf(wc, gv[2 * v + kx][d], acc[v][c]);
-                    }
+                    for (int v = 0; v < VX; ++v)
+                        axpy(acc[v], wc, gv[2 * v + kx][d]);
                 }
         }
     }
@@ -778,14 +792,15 @@ __global__ void __launch_bounds__(128)
             gv[r] = x >= 0 && x < g.X ? __ldg(gyb + (size_t)x * cols + (k / 3 - 1) * g.Z + k % 3 - 1) : 0.f;
         }
 #pragma unroll
-        for (int d = 0; d < 3; ++d)
+        for (int d = 0; d < 3; ++d) {
+            float wc[CT];
 #pragma unroll
-            for (int c = 0; c < CT; ++c) {
-                const float wc = ws[(d * 9 + k) * CT + c];
+            for (int c = 0; c < CT; ++c)
+                wc[c] = ws[(d * 9 + k) * CT + c];
 #pragma unroll
-                for (int r = 0; r < RX; ++r)
-                    acc[r][c] = fmaf(wc, gv[r + d], acc[r][c]);
-            }
+            for (int r = 0; r < RX; ++r)
+                axpy(acc[r], wc, gv[r + d]);
+        }
     }
     // SiLU' of four channels' voxels at a time: their reads of `pre` together
     constexpr int CB = CT < 4 ? CT : 4;
