@@ -25,6 +25,12 @@
 // reads global memory and the last one stores there, so a two-stage transform crosses shared
 // memory once.  All transforms run forward: an inverse one swaps re and im at both ends.
 // Twiddles are those of plan.hpp, in complex64 hi + lo (compensated).
+//
+// Bound by the chain of dependent instructions on small grids (one or two warps per
+// scheduler; 30 x 20 x 12: 20 us an iteration, 5 a launch), by instruction issue on large ones
+// (100 x 90 x 30: 44-54% of the slots).  Real time, us an iteration, one kernel per
+// axis pass -> now: 100 x 90 x 30 149 -> 45; complex128 128 x 128 x 32 220 -> 80; imaginary
+// time, complex128 64 x 64 x 16: 37 -> 28.
 #pragma once
 
 #include "kernels.cuh"

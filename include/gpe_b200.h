@@ -72,8 +72,8 @@ typedef struct gpe_params {
 enum {
     GPE_SCHED_AUTO  = 0, /* the four-kernel fused pipeline where the grid has compiled
                             line lengths (nx, ny in {32,64,96,128,256}, nz in
-                            {8,16,24,32,64}, complex64), else the split schedule */
-    GPE_SCHED_SPLIT = 1  /* one kernel per FFT axis pass (any supported grid) */
+                            {8,16,24,32,64}, complex64), else as GPE_SCHED_SPLIT */
+    GPE_SCHED_SPLIT = 1  /* the passes with run-time line lengths (any supported grid) */
 };
 
 typedef struct gpe_handle gpe_handle;
