@@ -17,19 +17,9 @@ struct Radices {
     int r[8];
 };
 
-// The power-of-two part in as few balanced stages of radix <= 16 as possible, then a
-// stage per factor 3, 5 or 7; lengths with one factor 3 (grids of 96 and 24) take it
-// into the second stage, radix 6 or 12, first stages 4, 8 or 16 (the pruned ones).
+// Same factorisation as the host planner (plan.hpp factor_line).
 __host__ __device__ constexpr Radices radices_of(int L) {
     Radices R{0, {0, 0, 0, 0, 0, 0, 0, 0}};
-    if (L == 24)
-        return Radices{2, {4, 6, 0, 0, 0, 0, 0, 0}};
-    if (L == 48)
-        return Radices{2, {8, 6, 0, 0, 0, 0, 0, 0}};
-    if (L == 96)
-        return Radices{2, {8, 12, 0, 0, 0, 0, 0, 0}};
-    if (L == 192)
-        return Radices{2, {16, 12, 0, 0, 0, 0, 0, 0}};
     int m = L, e = 0;
     while (m % 2 == 0) {
         m /= 2;

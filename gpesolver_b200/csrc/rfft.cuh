@@ -263,14 +263,12 @@ struct LinePass {
     }
 };
 
-// Block size for a pass of COUNT lines of length L: one butterfly of the largest
-// radix per thread (lines with a factor 3: of the smallest, so that no stage takes a second,
-// partly filled round), 64..256 threads.
+// Block size for a pass of COUNT lines of length L: one butterfly of the
+// largest radix per thread, 64..256 threads.
 template <int L, int COUNT> constexpr int pass_threads() {
-    constexpr Radices q = radices_of(L);
-    int r               = q.r[0];
-    for (int s = 1; s < q.n; ++s)
-        r = (L % 3 == 0) == (q.r[s] < r) ? q.r[s] : r;
+    int r = 1;
+    for (int s = 0; s < radices_of(L).n; ++s)
+        r = radices_of(L).r[s] > r ? radices_of(L).r[s] : r;
     int nt = COUNT * L / r;
     nt     = nt < 64 ? 64 : (nt > 256 ? 256 : nt);
     return (nt + 31) / 32 * 32;
