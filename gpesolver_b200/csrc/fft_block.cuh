@@ -301,9 +301,31 @@ template <int P, int SIGN, class R, bool CMP = true> struct DFTOdd {
         }
     }
 };
+// Three points as direct sums: the compile-time lines of 24, 48, 96 and 192 keep the
+// roundings that their users' results have (imaginary-time runs near collapse amplify the
+// last bit by 1e3 and more); composite radices take the paired sums (DFTPart).
 template <int SIGN, class R, bool CMP> struct DFT<3, SIGN, R, CMP> {
-    static __device__ __forceinline__ void run(cplx<R> *a) { DFTOdd<3, SIGN, R, CMP>::run(a); }
+    using C = cplx<R>;
+    static __device__ __forceinline__ void run(C *a) {
+        C out[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            C acc = a[0];
+#pragma unroll
+            for (int k = 1; k < 3; ++k) {
+                const int m = (k * q) % 3;
+                acc         = cadd(acc, mul_wc<SIGN, C, R, CMP>(a[k], m == 0 ? 1.0 : OddTab<3>::c(m),
+                                                                m == 0 ? 0.0 : OddTab<3>::s(m)));
+            }
+            out[q] = acc;
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+            a[q] = out[q];
+    }
 };
+template <int N, int SIGN, class R, bool CMP> struct DFTPart : DFT<N, SIGN, R, CMP> {};
+template <int SIGN, class R, bool CMP> struct DFTPart<3, SIGN, R, CMP> : DFTOdd<3, SIGN, R, CMP> {};
 template <int SIGN, class R, bool CMP> struct DFT<5, SIGN, R, CMP> {
     static __device__ __forceinline__ void run(cplx<R> *a) { DFTOdd<5, SIGN, R, CMP>::run(a); }
 };
@@ -323,7 +345,7 @@ template <int N1, int N2, int SIGN, class R, bool CMP> struct DFTCoprime {
 #pragma unroll
             for (int n1 = 0; n1 < N1; ++n1)
                 y[n2][n1] = a[(N2 * n1 + N1 * n2) % N];
-            DFT<N1, SIGN, R, CMP>::run(y[n2]);
+            DFTPart<N1, SIGN, R, CMP>::run(y[n2]);
         }
 #pragma unroll
         for (int k1 = 0; k1 < N1; ++k1) {
@@ -331,7 +353,7 @@ template <int N1, int N2, int SIGN, class R, bool CMP> struct DFTCoprime {
 #pragma unroll
             for (int n2 = 0; n2 < N2; ++n2)
                 z[n2] = y[n2][k1];
-            DFT<N2, SIGN, R, CMP>::run(z);
+            DFTPart<N2, SIGN, R, CMP>::run(z);
 #pragma unroll
             for (int n2 = 0; n2 < N2; ++n2)
                 y[n2][k1] = z[n2];
@@ -365,7 +387,7 @@ template <int SIGN, class R, bool CMP> struct DFT<9, SIGN, R, CMP> {
 #pragma unroll
             for (int n1 = 0; n1 < 3; ++n1)
                 y[n2][n1] = a[3 * n1 + n2];
-            DFT<3, SIGN, R, CMP>::run(y[n2]);
+            DFTPart<3, SIGN, R, CMP>::run(y[n2]);
         }
         y[1][1] = mul_wc<SIGN, C, R, CMP>(y[1][1], c1, s1);
         y[1][2] = mul_wc<SIGN, C, R, CMP>(y[1][2], c2, s2);
@@ -374,7 +396,7 @@ template <int SIGN, class R, bool CMP> struct DFT<9, SIGN, R, CMP> {
 #pragma unroll
         for (int k1 = 0; k1 < 3; ++k1) {
             C z[3] = {y[0][k1], y[1][k1], y[2][k1]};
-            DFT<3, SIGN, R, CMP>::run(z);
+            DFTPart<3, SIGN, R, CMP>::run(z);
 #pragma unroll
             for (int k2 = 0; k2 < 3; ++k2)
                 a[k1 + 3 * k2] = z[k2];

@@ -95,7 +95,7 @@ __device__ __forceinline__ void g_mid_r(const GStage &st, const void *tw, unsign
         const int d = g_div(j, st.ns, st.m), jm = j - d * st.ns;
         C a[RAD];
         g_load<RAD, R>(a, sm + src, st, jm, j, b, TS, nin, tw);
-        DFT<RAD, -1, R>::run(a);
+        DFTPart<RAD, -1, R, true>::run(a);
         C *o         = sm + dst + (d * st.ns * RAD + jm) * TS + b;
         const int os = st.ns * TS;
 #pragma unroll
@@ -133,7 +133,7 @@ __device__ __forceinline__ void g_first_r(const GStage &st, const cplx<R> *__res
 #pragma unroll
         for (int k = 0; k < RAD; ++k)
             a[k] = g_swap(a[k], swap);
-        DFT<RAD, -1, R>::run(a);
+        DFTPart<RAD, -1, R, true>::run(a);
 #pragma unroll
         for (int q = 0; q < RAD; ++q)
             sm[(j * RAD + q) * TS + b] = a[q];
@@ -150,7 +150,7 @@ __device__ __forceinline__ void g_last_r(const GStage &st, const void *tw, cplx<
         const int b = it & ((1 << lb) - 1), j = it >> lb;
         C a[RAD];
         g_load<RAD, R>(a, sm, st, j, j, b, TS, st.nr * RAD, tw);
-        DFT<RAD, -1, R>::run(a);
+        DFTPart<RAD, -1, R, true>::run(a);
 #pragma unroll
         for (int q = 0; q < RAD; ++q) {
             const int t = j + q * st.nr;
@@ -261,7 +261,7 @@ __device__ __forceinline__ void g_xmid_r(const GXArgs &a, const GPlan &pl, bool 
 #pragma unroll
             for (int q = 0; q < RAD; ++q)
                 in[q] = v[q];
-        DFT<RAD, -1, R>::run(v);
+        DFTPart<RAD, -1, R, true>::run(v);
         if (kin) {
             const C *ex = reinterpret_cast<const C *>(a.ex);
             const C wy = __ldg(reinterpret_cast<const C *>(a.ey) + y), wz = __ldg(reinterpret_cast<const C *>(a.ez) + z);
@@ -285,7 +285,7 @@ __device__ __forceinline__ void g_xmid_r(const GXArgs &a, const GPlan &pl, bool 
                 v[q]        = C{v[q].y * f, v[q].x * f};
             }
         }
-        DFT<RAD, -1, R>::run(v);
+        DFTPart<RAD, -1, R, true>::run(v);
         // complex64: the transform pair carries the kinetic factor's change of psi,
         // exp(i theta) - 1, and psi itself, RAD / N times the pair's inputs, is added
         // here.  Their rounding then scales with |theta|: done directly, the sums in
