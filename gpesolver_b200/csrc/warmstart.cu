@@ -242,21 +242,25 @@ __global__ void k_fold(const __nv_bfloat16 *__restrict__ wb, float *__restrict__
 // of VX coarse voxels along x, so that a step's weights (shared memory, warp-uniform
 // 16-byte reads) serve 2 VX x OT sums and its u (L1) all of them; lanes run along z and
 // store 8 bytes each.  Bound by FP32 issue at <8, 2>; small volumes take fewer
-// channels a thread, so that the layer fills the SMs.  pre may be null (prediction).
-// Measured: 32 -> 32 channels to 16 x 16 x 4, 1 sample, 190 -> 18 us; 8 -> 8 to
+// channels a thread, so that the layer fills the SMs, and the smallest split the input
+// channels over KS groups of 128 threads, summed in order through shared memory: there a
+// thread's chain of loads is the time.  pre may be null (prediction).
+// Measured: 32 -> 32 channels to 16 x 16 x 4, 1 sample, 190 -> 18 (KS = 1) -> 8.8 us; 8 -> 8 to
 // 128 x 128 x 32, 8 samples, 747 -> 195 us.
-template <int OT, int VX>
-__global__ void __launch_bounds__(128)
+template <int OT, int VX, int KS>
+__global__ void __launch_bounds__(128 * KS)
     k_up_fwd(const float *__restrict__ in, const float *__restrict__ fwd, const __nv_bfloat16 *__restrict__ bias,
              float *__restrict__ pre, float *__restrict__ out, ConvGeom g, size_t in_stride, size_t out_stride) {
-    extern __shared__ __align__(16) float uf_ws[]; // [c][16][OT]
+    extern __shared__ __align__(16) float uf_ws[]; // [c][16][OT], then the other groups' sums [KS - 1][2 VX OT][128]
     const int pxy = blockIdx.y & 3, px = pxy >> 1, py = pxy & 1, o0 = (blockIdx.y >> 2) * OT;
-    for (int e = threadIdx.x; e < g.cin * 16 * OT; e += 128)
+    for (int e = threadIdx.x; e < g.cin * 16 * OT; e += 128 * KS)
         uf_ws[e] = fwd[((size_t)pxy * g.cin * 16 + e / OT) * g.cout + o0 + e % OT];
     __syncthreads();
     const int Xi = g.X >> 1, Yi = g.Y >> 1, Zi = g.Z >> 1;
-    const int idx = blockIdx.x * 128 + threadIdx.x;
-    if (idx >= Xi / VX * Yi * Zi)
+    const int grp = KS > 1 ? threadIdx.x / 128 : 0, lane = threadIdx.x - grp * 128;
+    const int idx = blockIdx.x * 128 + lane;
+    const bool live = idx < Xi / VX * Yi * Zi;
+    if (KS == 1 && !live)
         return;
     const int zi = idx % Zi, yi = idx / Zi % Yi, xi = idx / Zi / Yi * VX;
     const size_t ni  = (size_t)Xi * Yi * Zi;
@@ -266,10 +270,10 @@ __global__ void __launch_bounds__(128)
     for (int v = 0; v < VX; ++v)
 #pragma unroll
         for (int o = 0; o < OT; ++o)
-            acc[v][0][o] = acc[v][1][o] = __bfloat162float(bias[o0 + o]);
+            acc[v][0][o] = acc[v][1][o] = grp ? 0.f : __bfloat162float(bias[o0 + o]);
     const bool zl = zi > 0, zr = zi + 1 < Zi;
 #pragma unroll 2
-    for (int c = 0; c < g.cin; ++c) {
+    for (int c = live ? grp : g.cin; c < g.cin; c += KS) {
         float u[VX + 1][2][3];
 #pragma unroll
         for (int a = 0; a <= VX; ++a)
@@ -298,6 +302,22 @@ __global__ void __launch_bounds__(128)
             for (int v = 0; v < VX; ++v)
                 axpy(acc[v][pz], wo, u[v + tx][ty][pz + tz]);
         }
+    }
+    if constexpr (KS > 1) {
+        float *red = uf_ws + g.cin * 16 * OT + lane;
+        if (grp) {
+#pragma unroll
+            for (int j = 0; j < 2 * VX * OT; ++j)
+                red[((grp - 1) * 2 * VX * OT + j) * 128] = acc[j / (2 * OT)][j / OT & 1][j % OT];
+        }
+        __syncthreads();
+        if (grp || !live)
+            return;
+#pragma unroll
+        for (int k = 0; k < KS - 1; ++k)
+#pragma unroll
+            for (int j = 0; j < 2 * VX * OT; ++j)
+                acc[j / (2 * OT)][j / OT & 1][j % OT] += red[(k * 2 * VX * OT + j) * 128];
     }
 #pragma unroll
     for (int v = 0; v < VX; ++v)
@@ -684,20 +704,23 @@ __global__ void __launch_bounds__(256)
 // coarse voxels along x and CT input channels (blockIdx.y: channel group), the
 // weights of a step shared by its voxels; lanes run along z (8-byte loads).
 // Bound by FP32 issue and the shared-memory weight reads (VX = 2 halves them);
-// small volumes take CT = 2, VX = 1 so that the layer fills the SMs.  8 -> 8
+// small volumes take CT = 2, VX = 1 so that the layer fills the SMs, the smallest with
+// the output channels over KS groups of 128 threads.  8 -> 8
 // channels at 128 x 128 x 32, 8 samples: 1086 + 2 x 70 (SiLU' pass) -> 200 us.
-template <int CT, int VX>
-__global__ void __launch_bounds__(128)
+template <int CT, int VX, int KS>
+__global__ void __launch_bounds__(128 * KS)
     k_up_xgrad(const float *__restrict__ gy, const float *__restrict__ bwd, const float *__restrict__ pre_in,
                float *__restrict__ dx, ConvGeom g, size_t g_stride, size_t dx_stride) {
-    extern __shared__ __align__(16) float xg_ws[]; // [o][64][CT]
+    extern __shared__ __align__(16) float xg_ws[]; // [o][64][CT], then the other groups' sums [KS - 1][VX CT][128]
     const int c0 = blockIdx.y * CT;
-    for (int e = threadIdx.x; e < g.cout * 64 * CT; e += 128)
+    for (int e = threadIdx.x; e < g.cout * 64 * CT; e += 128 * KS)
         xg_ws[e] = bwd[(size_t)(e / CT) * g.cin + c0 + e % CT];
     __syncthreads();
     const int Xi = g.X >> 1, Yi = g.Y >> 1, Zi = g.Z >> 1;
-    const int idx = blockIdx.x * 128 + threadIdx.x;
-    if (idx >= Xi / VX * Yi * Zi)
+    const int grp = KS > 1 ? threadIdx.x / 128 : 0, lane = threadIdx.x - grp * 128;
+    const int idx = blockIdx.x * 128 + lane;
+    const bool live = idx < Xi / VX * Yi * Zi;
+    if (KS == 1 && !live)
         return;
     const int zi = idx % Zi, yi = idx / Zi % Yi, xi = idx / Zi / Yi * VX;
     const size_t nv = (size_t)g.X * g.Y * g.Z;
@@ -709,7 +732,7 @@ __global__ void __launch_bounds__(128)
         for (int c = 0; c < CT; ++c)
             acc[v][c] = 0.f;
     const bool zl = zi > 0, zr = zi + 1 < Zi;
-    for (int o = 0; o < g.cout; ++o) {
+    for (int o = live ? grp : g.cout; o < g.cout; o += KS) {
 #pragma unroll
         for (int b = 0; b < 4; ++b) {
             const int y = 2 * yi - 1 + b;
@@ -745,6 +768,22 @@ __global__ void __launch_bounds__(128)
                         axpy(acc[v], wc, gv[2 * v + kx][d]);
                 }
         }
+    }
+    if constexpr (KS > 1) {
+        float *red = xg_ws + g.cout * 64 * CT + lane;
+        if (grp) {
+#pragma unroll
+            for (int j = 0; j < VX * CT; ++j)
+                red[((grp - 1) * VX * CT + j) * 128] = acc[j / CT][j % CT];
+        }
+        __syncthreads();
+        if (grp || !live)
+            return;
+#pragma unroll
+        for (int k = 0; k < KS - 1; ++k)
+#pragma unroll
+            for (int j = 0; j < VX * CT; ++j)
+                acc[j / CT][j % CT] += red[(k * VX * CT + j) * 128];
     }
 #pragma unroll
     for (int v = 0; v < VX; ++v)
@@ -969,25 +1008,30 @@ void forward(gpe_warm *W, int B, float *amp, bool training) {
         }
         const int Xi = L.g.X / 2, nvox = Xi * (L.g.Y / 2) * (L.g.Z / 2);
         const size_t n = W->vox((int)l) * L.cout;
-        auto go = [&](auto O, auto V) {
-            constexpr int OT = decltype(O)::value, VX = decltype(V)::value;
-            k_up_fwd<OT, VX><<<dim3((nvox / VX + 127) / 128, 4 * (L.cout / OT), B), 128,
-                               sizeof(float) * L.cin * 16 * OT, s>>>(in, W->fold.p + L.f, wb + L.b,
-                                                                     training ? W->pre[l].p : nullptr, W->act[l].p,
-                                                                     L.g, in_stride, n);
+        auto go = [&](auto O, auto V, auto K) {
+            constexpr int OT = decltype(O)::value, VX = decltype(V)::value, KS = decltype(K)::value;
+            k_up_fwd<OT, VX, KS><<<dim3((nvox / VX + 127) / 128, 4 * (L.cout / OT), B), 128 * KS,
+                                   sizeof(float) * (L.cin * 16 * OT + (KS - 1) * 2 * VX * OT * 128), s>>>(
+                in, W->fold.p + L.f, wb + L.b, training ? W->pre[l].p : nullptr, W->act[l].p, L.g, in_stride, n);
         };
         using I1 = std::integral_constant<int, 1>;
         using I2 = std::integral_constant<int, 2>;
+        using I4 = std::integral_constant<int, 4>;
         // two voxels and eight channels a thread where that still leaves 512 threads
-        // per SM, one voxel and four channels where that does, else two (or one)
+        // per SM, one voxel and four channels where that does, else two (or one); with
+        // the input channels split over four groups where all CTAs are resident at once
+        // (two per SM: 64 CTAs 18.2 -> 8.8 us, 256 CTAs 19.4 -> 11.1, 512 CTAs 19.4 -> 19.9)
+        const size_t small = (size_t)((nvox + 127) / 128) * 4 * (L.cout / 2) * B;
         if (Xi % 2 == 0 && L.cout >= 8 && (size_t)nvox / 2 * 4 * (L.cout / 8) * B >= 148 * 512)
-            go(std::integral_constant<int, 8>{}, I2{});
+            go(std::integral_constant<int, 8>{}, I2{}, I1{});
         else if (L.cout >= 4 && (size_t)nvox * 4 * (L.cout / 4) * B >= 148 * 512)
-            go(std::integral_constant<int, 4>{}, I1{});
+            go(I4{}, I1{}, I1{});
+        else if (L.cout >= 2 && L.cin >= 8 && small <= 148 * 2)
+            go(I2{}, I1{}, I4{});
         else if (L.cout >= 2)
-            go(I2{}, I1{});
+            go(I2{}, I1{}, I1{});
         else
-            go(I1{}, I1{});
+            go(I1{}, I1{}, I1{});
         in        = W->act[l].p;
         in_stride = n;
     }
@@ -1085,23 +1129,30 @@ void conv_xgrad(gpe_warm *W, int l, int B, const float *gy, size_t g_stride, con
         return;
     }
     const int Xi = L.g.X / 2, nvox = Xi * (L.g.Y / 2) * (L.g.Z / 2);
-    auto go = [&](auto C, auto V) {
+    auto go = [&](auto C, auto V, auto K) {
         constexpr int CT = decltype(C)::value, VX = decltype(V)::value;
-        gpe::k_up_xgrad<CT, VX><<<dim3((nvox / VX + 127) / 128, L.cin / CT, B), 128, sizeof(float) * L.cout * 64 * CT,
-                                  s>>>(gy, W->fold.p + W->fold.n / 2 + L.f, pre_in, dx, L.g, g_stride, dx_stride);
+        constexpr int KS = decltype(K)::value;
+        gpe::k_up_xgrad<CT, VX, KS><<<dim3((nvox / VX + 127) / 128, L.cin / CT, B), 128 * KS,
+                                      sizeof(float) * (L.cout * 64 * CT + (KS - 1) * VX * CT * 128), s>>>(
+            gy, W->fold.p + W->fold.n / 2 + L.f, pre_in, dx, L.g, g_stride, dx_stride);
     };
     using I1 = std::integral_constant<int, 1>;
     using I2 = std::integral_constant<int, 2>;
+    using I4 = std::integral_constant<int, 4>;
     // two voxels and eight channels a thread where that still leaves 256 threads
-    // per SM, one voxel and four channels where that does, else two (or one)
+    // per SM, one voxel and four channels where that does, else two (or one); with the
+    // output channels split over four groups where all CTAs are resident at once (two
+    // per SM: 128 CTAs 49.6 -> 25.1 us; 512 CTAs of four channels 52.8 -> 54.3)
     if (Xi % 2 == 0 && L.cin >= 8 && (size_t)nvox / 2 * (L.cin / 8) * B >= 148 * 256)
-        go(std::integral_constant<int, 8>{}, I2{});
+        go(std::integral_constant<int, 8>{}, I2{}, I1{});
     else if (L.cin >= 4 && (size_t)nvox * (L.cin / 4) * B >= 148 * 256)
-        go(std::integral_constant<int, 4>{}, I1{});
+        go(I4{}, I1{}, I1{});
+    else if (L.cin >= 2 && L.cout >= 8 && (size_t)((nvox + 127) / 128) * (L.cin / 2) * B <= 148 * 2)
+        go(I2{}, I1{}, I4{});
     else if (L.cin >= 2)
-        go(I2{}, I1{});
+        go(I2{}, I1{}, I1{});
     else
-        go(I1{}, I1{});
+        go(I1{}, I1{}, I1{});
 }
 
 // gradients of the mean squared amplitude error against `targets` (device,
@@ -1229,7 +1280,7 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
         W->partial.alloc(maxpart);
         W->lpart.alloc(148 * 4);
         // folded weights staged in shared memory, up to 32 channels
-        WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_up_xgrad<8, 2>,
+        WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_up_xgrad<8, 2, 1>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)sizeof(float) * gpe::kMaxCout * 64 * 8));
         for (int ot : {1, 2, 4, 8})
