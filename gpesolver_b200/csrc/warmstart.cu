@@ -1038,7 +1038,15 @@ void forward(gpe_warm *W, int B, float *amp, bool training) {
     WS_CUDA(cudaGetLastError());
 }
 
-// tile of the folded weight gradient for a coarse volume, and its shared memory
+constexpr size_t kWgSmem = 96 * 1024; // the weight-gradient kernel's limit
+int wg_ot(const gpe_warm::Layer &L) { return std::min(L.cout, 8); }
+size_t wg_smem(const gpe::WgTile &w, int ot) {
+    const size_t gs = (size_t)8 * w.tx * w.ty * w.tz * ot;
+    return sizeof(float) * (((size_t)8 * w.cs + 3) / 4 * 4 + std::max<size_t>(gs, (size_t)512 * ot));
+}
+// tile of the folded weight gradient for a coarse volume: at most 128 voxels, fewer along x
+// where the volume is thin (ty tz <= 2: a plane of u then takes 48 floats a channel with its
+// halo, and 128 of them do not fit into shared memory)
 gpe::WgTile wg_tile(const gpe_warm::Layer &L, int B) {
     gpe::WgTile w{};
     const int Xi = L.g.X / 2, Yi = L.g.Y / 2, Zi = L.g.Z / 2;
@@ -1056,7 +1064,12 @@ gpe::WgTile wg_tile(const gpe_warm::Layer &L, int B) {
     };
     w.ys = up(w.tz + 2, 8, 16);
     w.xs = up((w.ty + 2) * w.ys, 16, 32);
-    w.cs = up((w.tx + 2) * w.xs, 1, 32);
+    auto fits = [&] {
+        w.cs = up((w.tx + 2) * w.xs, 1, 32);
+        return wg_smem(w, wg_ot(L)) <= kWgSmem;
+    };
+    while (!fits())
+        w.tx /= 2;
     w.nx = (Xi + w.tx - 1) / w.tx;
     w.ny = (Yi + w.ty - 1) / w.ty;
     w.nz = (Zi + w.tz - 1) / w.tz;
@@ -1064,11 +1077,6 @@ gpe::WgTile wg_tile(const gpe_warm::Layer &L, int B) {
     w.ncg   = (L.cin + 7) / 8;
     return w;
 }
-size_t wg_smem(const gpe::WgTile &w, int ot) {
-    const size_t gs = (size_t)8 * w.tx * w.ty * w.tz * ot;
-    return sizeof(float) * (((size_t)8 * w.cs + 3) / 4 * 4 + std::max<size_t>(gs, (size_t)512 * ot));
-}
-int wg_ot(const gpe_warm::Layer &L) { return std::min(L.cout, 8); }
 // CTAs along the tiles: up to three per SM (all resident) over all channel groups
 int wg_parts(const gpe::WgTile &w, int pairs) { return std::min(w.ntile, std::max(1, 148 * 3 / pairs)); }
 // planes per segment of the last layer's gradient (a multiple of 3) and segments
@@ -1286,7 +1294,7 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
         for (int ot : {1, 2, 4, 8})
             gpe::by_ot(ot, [&](auto O) {
                 WS_CUDA(cudaFuncSetAttribute((const void *)gpe::k_up_wgrad<decltype(O)::value>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024));
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWgSmem));
             });
         *out = W.release();
     });

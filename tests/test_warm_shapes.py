@@ -1,0 +1,20 @@
+"""The warm-start network on volumes far from a cube, against the FP64 restatement
+(oracle/warmnet_ref.py); the tolerances are those of test_warm_kernels.py."""
+import pytest
+
+from . import test_warm_kernels as K
+
+pytestmark = pytest.mark.gpu
+
+
+# coarse volumes of 36 x 1 x 1, 64 x 2 x 1, 33 x 1 x 2, 40 x 2 x 1 and 34 x 1 x 1 voxels: the
+# weight gradient's tiles are cut along x to fit into shared memory
+@pytest.mark.parametrize("dims,levels,channels,batch", [
+    ((72, 2, 2), 1, (8, 8), 2),
+    ((128, 4, 2), 1, (8, 8), 1),
+    ((66, 2, 4), 1, (16, 1), 2),
+    ((80, 4, 2), 1, (4, 32), 1),
+    ((272, 8, 8), 3, (8, 8, 8, 8), 1),
+])
+def test_thin_volumes_match_fp64(dims, levels, channels, batch):
+    K.test_edges_match_fp64(dims, levels, channels, batch)
