@@ -1,8 +1,6 @@
 // Host-side FFT planning and FP64 table construction.
 #pragma once
 
-#include "fft_block.cuh"
-
 #include <cmath>
 #include <stdexcept>
 #include <string>
