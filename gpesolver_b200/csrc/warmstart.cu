@@ -127,15 +127,16 @@ __global__ void k_dense_wgrad(const float *__restrict__ G, const float *__restri
 // dX[b][i] = sum_o W[o][i] G[b][o], times SiLU'(pre[b][i]): the rows o in chunks
 // (blockIdx.y), eight samples at a time, coalesced along i; then the chunks'
 // sums.  (One thread per (b, i) over all rows: 381 us at 4096 x 256, 8 samples,
-// 16 CTAs with one serial chain each.)
-constexpr int kXgRows = 32;
+// 16 CTAs with one serial chain each.)  Chunks of 32 rows, longer ones where that
+// would make more than 4096 (blockIdx.y ends at 65535, and so do the sums).
+int xg_rows(int O) { return std::max(32, (O + 4095) / 4096); }
 __global__ void __launch_bounds__(128)
     k_dense_xgrad_part(const float *__restrict__ G, const __nv_bfloat16 *__restrict__ W, float *__restrict__ part,
-                       int B, int I, int O) {
+                       int B, int I, int O, int rows) {
     const int i = blockIdx.x * 128 + threadIdx.x;
     if (i >= I)
         return;
-    const int o0 = blockIdx.y * kXgRows, o1 = min(o0 + kXgRows, O);
+    const int o0 = blockIdx.y * rows, o1 = min(o0 + rows, O);
     for (int b0 = 0; b0 < B; b0 += 8) {
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 4
@@ -344,10 +345,12 @@ __global__ void __launch_bounds__(128, 8)
     for (int e = threadIdx.x; e < g.cin * 27; e += 128)
         ws[e] = __bfloat162float(W[e]);
     __syncthreads();
-    const int cols = g.Y * g.Z, col = blockIdx.x * 128 + threadIdx.x;
+    // blockIdx.x = column block + column blocks * x block
+    const int cols = g.Y * g.Z, ncb = (cols + 127) / 128, xb = blockIdx.x / ncb;
+    const int col  = (blockIdx.x - xb * ncb) * 128 + threadIdx.x;
     if (col >= cols)
         return;
-    const int y = col / g.Z, z = col - y * g.Z, x0 = blockIdx.y * RX;
+    const int y = col / g.Z, z = col - y * g.Z, x0 = xb * RX;
     const float *inb = in + blockIdx.z * in_stride + col;
     float acc[RX];
 #pragma unroll
@@ -804,14 +807,16 @@ __global__ void __launch_bounds__(128)
                  float *__restrict__ dx, ConvGeom g, size_t g_stride, size_t dx_stride) {
     constexpr int RX = 4;
     __shared__ __align__(16) float ws[27 * CT]; // [tap, mirrored][CT]
-    const int ngrp = g.cin / CT, c0 = (blockIdx.y % ngrp) * CT;
+    // blockIdx.x = column block + column blocks * (channel group + groups * x block)
+    const int cols = g.Y * g.Z, ncb = (cols + 127) / 128, row = blockIdx.x / ncb;
+    const int ngrp = g.cin / CT, c0 = (row % ngrp) * CT;
     for (int e = threadIdx.x; e < 27 * CT; e += 128)
         ws[e] = __bfloat162float(W[(size_t)(c0 + e % CT) * 27 + 26 - e / CT]);
     __syncthreads();
-    const int cols = g.Y * g.Z, col = blockIdx.x * 128 + threadIdx.x;
+    const int col = (blockIdx.x - row * ncb) * 128 + threadIdx.x;
     if (col >= cols)
         return;
-    const int y = col / g.Z, z = col - y * g.Z, x0 = blockIdx.y / ngrp * RX;
+    const int y = col / g.Z, z = col - y * g.Z, x0 = row / ngrp * RX;
     const float *gyb = gy + blockIdx.z * g_stride + col;
     float acc[RX][CT];
 #pragma unroll
@@ -1002,7 +1007,7 @@ void forward(gpe_warm *W, int B, float *amp, bool training) {
     for (const auto &L : W->conv) {
         const size_t l = &L - W->conv.data();
         if (!L.g.up) {
-            k_last_fwd<<<dim3((L.g.Y * L.g.Z + 127) / 128, (L.g.X + 3) / 4, B), 128, 0, s>>>(
+            k_last_fwd<<<dim3((L.g.Y * L.g.Z + 127) / 128 * ((L.g.X + 3) / 4), 1, B), 128, 0, s>>>(
                 in, wb + L.w, wb + L.b, amp, L.g, in_stride);
             break;
         }
@@ -1131,7 +1136,8 @@ void conv_xgrad(gpe_warm *W, int l, int B, const float *gy, size_t g_stride, con
     if (!L.g.up) {
         gpe::by_ot(std::min(L.cin, 8), [&](auto C) {
             constexpr int CT = decltype(C)::value;
-            gpe::k_last_xgrad<CT><<<dim3((L.g.Y * L.g.Z + 127) / 128, (L.g.X + 3) / 4 * (L.cin / CT), B), 128, 0, s>>>(
+            gpe::k_last_xgrad<CT><<<dim3((L.g.Y * L.g.Z + 127) / 128 * ((L.g.X + 3) / 4 * (L.cin / CT)), 1, B), 128, 0,
+                                    s>>>(
                 gy, W->wb.p + L.w, pre_in, dx, L.g, g_stride, dx_stride);
         });
         return;
@@ -1187,10 +1193,11 @@ double backward(gpe_warm *W, int B, const float *targets) {
     // dense 2 and dense 1 (gh2 and gh1 are gradients of the pre-activations)
     k_dense_wgrad<<<(int)(((size_t)W->latent * c.hidden + 255) / 256), 256, 0, s>>>(
         W->gh2.p, W->h1.p, W->grad.p + W->d2w, W->grad.p + W->d2b, B, c.hidden, W->latent);
-    const int rows = (W->latent + kXgRows - 1) / kXgRows;
-    k_dense_xgrad_part<<<dim3((c.hidden + 127) / 128, rows), 128, 0, s>>>(W->gh2.p, wb + W->d2w, W->partial.p, B,
-                                                                          c.hidden, W->latent);
-    k_dense_xgrad_sum<<<(B * c.hidden + 63) / 64, 64, 0, s>>>(W->partial.p, W->h1pre.p, W->gh1.p, B * c.hidden, rows);
+    const int rows = xg_rows(W->latent), chunks = (W->latent + rows - 1) / rows;
+    k_dense_xgrad_part<<<dim3((c.hidden + 127) / 128, chunks), 128, 0, s>>>(W->gh2.p, wb + W->d2w, W->partial.p, B,
+                                                                            c.hidden, W->latent, rows);
+    k_dense_xgrad_sum<<<(B * c.hidden + 63) / 64, 64, 0, s>>>(W->partial.p, W->h1pre.p, W->gh1.p, B * c.hidden,
+                                                              chunks);
     k_dense_wgrad<<<(int)(((size_t)c.hidden * c.n_inputs + 255) / 256), 256, 0, s>>>(
         W->gh1.p, W->x.p, W->grad.p + W->d1w, W->grad.p + W->d1b, B, c.n_inputs, c.hidden);
     WS_CUDA(cudaGetLastError());
@@ -1274,7 +1281,8 @@ int gpe_warm_create(const gpe_warm_config *cfg, int device, gpe_warm **out) {
         W->h2.alloc((size_t)B * W->latent);
         W->gh2.alloc((size_t)B * W->latent);
         // partial sums: the weight gradients' and dense 2's input gradient's
-        size_t maxpart = (size_t)((W->latent + gpe::kXgRows - 1) / gpe::kXgRows) * B * c.hidden;
+        const int xr   = gpe::xg_rows(W->latent);
+        size_t maxpart = (size_t)((W->latent + xr - 1) / xr) * B * c.hidden;
         W->pre.resize(W->conv.size());
         W->act.resize(W->conv.size());
         W->gact.resize(W->conv.size());

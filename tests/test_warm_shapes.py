@@ -18,3 +18,14 @@ pytestmark = pytest.mark.gpu
 ])
 def test_thin_volumes_match_fp64(dims, levels, channels, batch):
     K.test_edges_match_fp64(dims, levels, channels, batch)
+
+
+# more than 65535 chunks or blocks along x in the kernels that had them on a grid's second axis:
+# a latent volume of 2.1 M values, the last convolution forward, its input gradient
+@pytest.mark.parametrize("dims,levels,channels,batch", [
+    ((64, 64, 16), 0, (32,), 1),
+    ((262152, 1, 1), 0, (1,), 1),
+    ((65544, 2, 2), 1, (8, 32), 1),
+])
+def test_long_volumes_match_fp64(dims, levels, channels, batch):
+    K.test_edges_match_fp64(dims, levels, channels, batch)
