@@ -26,7 +26,9 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <memory>
 #include <random>
 #include <type_traits>
@@ -1210,6 +1212,18 @@ double backward(gpe_warm *W, int B, const float *targets) {
     return loss / (double)((size_t)B * N);
 }
 
+// Whether a kernel of W may store floats at p: memory of its own device, aligned.  Memory of
+// another device, the host's, or at an odd address is left to the copy engine, which takes
+// them all or returns an error.
+bool kernel_may_store(const gpe_warm *W, const void *p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == W->device && (uintptr_t)p % alignof(float) == 0;
+}
+
 void upload_inputs(gpe_warm *W, const float *params_host, int B) {
     WS_CUDA(cudaMemcpyAsync(W->x.p, params_host, sizeof(float) * B * W->cfg.n_inputs, cudaMemcpyHostToDevice,
                             W->stream));
@@ -1377,7 +1391,11 @@ int gpe_warm_forward(gpe_warm *W, const float *params_host, int B, float *amp_de
     return wguard([&] {
         WS_CUDA(cudaSetDevice(W->device));
         upload_inputs(W, params_host, B);
-        forward(W, B, amp_dev, false);
+        const bool direct = kernel_may_store(W, amp_dev);
+        forward(W, B, direct ? amp_dev : W->pre.back().p, false);
+        if (!direct)
+            WS_CUDA(cudaMemcpyAsync(amp_dev, W->pre.back().p, sizeof(float) * B * W->vox((int)W->conv.size() - 1),
+                                    cudaMemcpyDeviceToDevice, W->stream));
         WS_CUDA(cudaStreamSynchronize(W->stream));
     });
 }

@@ -1,6 +1,9 @@
 """The warm-start network on volumes far from a cube, against the FP64 restatement
 (oracle/warmnet_ref.py); the tolerances are those of test_warm_kernels.py."""
+import numpy as np
 import pytest
+
+from gpesolver_b200 import warmstart as W
 
 from . import test_warm_kernels as K
 
@@ -29,3 +32,24 @@ def test_thin_volumes_match_fp64(dims, levels, channels, batch):
 ])
 def test_long_volumes_match_fp64(dims, levels, channels, batch):
     K.test_edges_match_fp64(dims, levels, channels, batch)
+
+
+def test_amplitudes_into_any_buffer():
+    """Pinned host memory and an odd device address take the same bytes as a tensor on the device."""
+    import torch
+
+    net = W.WarmStartNet(W.WarmConfig(nx=16, ny=16, nz=8, levels=1, channels=(4, 4), hidden=8, max_batch=2), seed=1)
+    x = np.random.default_rng(2).uniform(-1, 1, (2, 4)).astype(np.float32)
+    n = 2 * net.n_voxels
+    amp = torch.zeros(n, device="cuda")
+    host = torch.zeros(n, pin_memory=True)
+    odd = torch.zeros(4 * n + 8, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    net.forward(x, amp.data_ptr())
+    net.forward(x, host.data_ptr())
+    net.forward(x, odd.data_ptr() + 2)
+    net.close()
+    want = amp.cpu().numpy()
+    assert np.abs(want).max() > 0
+    assert np.array_equal(host.numpy(), want)
+    assert odd[2:2 + 4 * n].cpu().numpy().tobytes() == want.tobytes()
