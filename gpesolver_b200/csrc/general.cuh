@@ -236,7 +236,8 @@ struct GXArgs {
     const void *ex, *ey, *ez;     // exp(i theta) - 1 per axis (kinetic)
     double inv;                   // 1 / N
     const void *vk;               // V_dd(|kx|, |ky|, kz), kz = 1..nz
-    const double *divisor;        // norm the spectrum is still to be divided by, or null
+    const double *divisor;        // [0] norm the spectrum is still to be divided by, [1] its power-of-two
+                                  // scale (g_spectrum_scale); or null
     double dip_scale;
     int nx, ny, nz, tk, lb;
     GPlan k, d;
@@ -314,7 +315,7 @@ template <class R, int MB> __global__ void __launch_bounds__(256, MB) g_x(const 
     const int cnt   = min(1 << a.lb, cols - c0);
     C *p            = (kin ? reinterpret_cast<C *>(a.psi) : reinterpret_cast<C *>(a.S)) + c0;
     const int TS    = 1 << a.lb;
-    const R scale   = (R)(a.divisor && !kin ? a.dip_scale / a.divisor[0] : a.dip_scale);
+    const R scale   = (R)(a.divisor && !kin ? a.dip_scale / (a.divisor[0] * a.divisor[1]) : a.dip_scale);
     unsigned cur = 0, oth = (unsigned)(pl.L * TS);
     auto flip = [&] {
         __syncthreads();
@@ -407,6 +408,16 @@ __device__ __forceinline__ cplx<R> g_turn(cplx<R> v, R V, R phi, R cdd, R hdt, R
     sincos_r<R>(mul_rn(mul_rn((R)-0.5, hdt), total), &s, &c);
     const R wx = mul_rn(mul_rn((R)-2, s), s), wy = mul_rn(mul_rn((R)2, s), c);
     return cplx<R>{add_rn(v.x, fma(v.x, wx, -mul_rn(v.y, wy))), add_rn(v.y, fma(v.x, wy, mul_rn(v.y, wx)))};
+}
+
+// A psi of norm d that is still to be divided by sqrt(d) enters rho as psi 2^-h: |psi|^2 N
+// and its transforms stay in range for any d that psi itself has room for (complex64, 1e13
+// times a normalised state and more: without it 1/d underflows and rho overflows).  Returns h
+// such that d 2^-2h is about 1; 0 for d within 2^+-32, where nothing needs it and every
+// rounding stays as it is.
+template <class R> __device__ __forceinline__ int g_spectrum_scale(double d) {
+    const int e = ((__double2hiint(d) >> 20) & 0x7ff) - 1023, most = sizeof(R) == 4 ? 120 : 500;
+    return abs(e) <= 32 ? 0 : min(max(e >> 1, -most), most);
 }
 
 struct GZArgs {
@@ -536,6 +547,13 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
         const R g3 = cf[0], gw = cf[1], g3n = cf[2], gwn = cf[3];
         const R sc   = (R)(IT ? 1.0 / sqrt(a.norm_state[1]) : 1.0);
         const R wat  = (R)a.w_atoms;
+        R fold       = (R)1;
+        if (MODE == GZ_IT_PRO && a.norm_state) {
+            const int h = g_spectrum_scale<R>(a.norm_state[1]);
+            fold        = (R)scalbn(1.0, -h);
+            if (blockIdx.x == 0 && tid == 0)
+                a.norm_state[2] = scalbn(1.0, -2 * h);
+        }
         const R hdt = (R)a.half_dt, cdd = (R)a.cdd;
         const R cx = (R)a.cx, cy = (R)a.cy, cz = (R)a.cz, dtau = (R)a.dtau;
         const ptrdiff_t plane = (ptrdiff_t)ny * nz;
@@ -574,7 +592,7 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
                     else
                         sm[K + k * TK + row] = v;
                 } else if (MODE == GZ_IT_PRO) {
-                    v = psi[q];
+                    v = cscale(psi[q], fold);
                 } else if (MODE == GZ_NORM) {
                     v = psi[q];
                     acc = add_rn(acc, g_abs2(double2{(double)v.x, (double)v.y}));

@@ -51,7 +51,8 @@ struct ZArgs {
     const void *V;
     void *phi;
     // norms (IT)
-    double *norm_state;  // [0] xnorma, [1] divisor of psi_in (read), both written by the last CTA
+    double *norm_state;  // [0] xnorma, [1] divisor of psi_in (read), [2] power-of-two scale of the
+                         // spectrum of an undivided psi (g_z, read by g_x); written by the last CTA
     double *partial;     // per-CTA partial sums of |psi_out|^2
     unsigned *ticket;    // CTA completion counter (reset by the last CTA)
     int *status;
@@ -67,7 +68,7 @@ extern __shared__ __align__(16) unsigned char g_smem[];
 
 // Norm of the psi an imaginary-time z pass has written, from every thread's sum of
 // |psi|^2: block partials, added in block order by the last block to finish, into
-// norm_state[0] and [1] (status[0] on a non-finite or non-positive one).  At most
+// norm_state[0] and [1], 1 into [2] (status[0] on a non-finite or non-positive one).  At most
 // 1024 threads; all of them call.
 __device__ __forceinline__ void norm_by_last_block(double acc, const ZArgs &a) {
     __shared__ double red[32];
@@ -102,6 +103,7 @@ __device__ __forceinline__ void norm_by_last_block(double acc, const ZArgs &a) {
     if (tid == 0) {
         a.norm_state[0] = x;
         a.norm_state[1] = x;
+        a.norm_state[2] = 1.0;
         if (!(x > 0.0) || !isfinite(x))
             a.status[0] = 1;
         *a.ticket = 0u;
