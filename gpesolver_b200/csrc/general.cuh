@@ -380,17 +380,15 @@ enum {
     GZ_IT_MID,     // dipolar inverse, Euler step and norm, forward
     GZ_DIP_INV,    // spectrum -> phi
     GZ_KIN_FWD, GZ_KIN_INV,
-    GZ_PHASE,      // one half step, psi and phi in memory
-    GZ_IT_STEP,    // the Euler step alone, phi in memory
     GZ_NORM,       // the norm alone
     GZ_MODES
 };
-// The interface's single steps (GZ_DIP_INV and after) run the same code on the same
-// rows as the iterations, so both sequences agree to the last bits.
+// The interface's single steps (GZ_DIP_INV and after, g_half_step, g_euler_step) run the
+// iterations' arithmetic, the norm on their rows too, so both sequences agree to the last
+// bits.
 
 // The pointwise arithmetic with its roundings written out: the compiler then contracts
-// it alike in every mode of g_z, and the iterations and the single steps agree to the
-// last bits.
+// it alike in every kernel.
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
@@ -408,6 +406,26 @@ __device__ __forceinline__ cplx<R> g_turn(cplx<R> v, R V, R phi, R cdd, R hdt, R
     sincos_r<R>(mul_rn(mul_rn((R)-0.5, hdt), total), &s, &c);
     const R wx = mul_rn(mul_rn((R)-2, s), s), wy = mul_rn(mul_rn((R)2, s), c);
     return cplx<R>{add_rn(v.x, fma(v.x, wx, -mul_rn(v.y, wy))), add_rn(v.y, fma(v.x, wy, mul_rn(v.y, wx)))};
+}
+
+// Euler step (cpu_solver.cpp:50-97) of the interior point at psi, held times 1 / sc:
+//   psi' = psi - dtau [cx Lx psi - cy Ly psi - cz Lz psi + (V + cdd phi + g3 |psi|^2 + gw |psi|^3) psi]
+template <class R>
+__device__ __forceinline__ cplx<R> g_euler(const cplx<R> *psi, ptrdiff_t plane, int nz, R sc, R V, R phi, R cdd, R g3,
+                                           R gw, R cx, R cy, R cz, R dtau) {
+    using C    = cplx<R>;
+    const C c0 = cscale(psi[0], sc);
+    const C xm = cscale(psi[-plane], sc), xp = cscale(psi[plane], sc);
+    const C ym = cscale(psi[-nz], sc), yp = cscale(psi[nz], sc);
+    const C zm = cscale(psi[-1], sc), zp = cscale(psi[1], sc);
+    const R dens = g_abs2(c0), am = sqrt(dens);
+    const R h    = add_rn(fma(cdd, phi, V), fma(g3, dens, mul_rn(gw, mul_rn(mul_rn(am, am), am))));
+    auto step    = [&](R c, R xa, R xb, R ya, R yb, R za, R zb) {
+        const R dx = fma((R)-2, c, add_rn(xa, xb)), dy = fma((R)-2, c, add_rn(ya, yb)),
+                dz = fma((R)-2, c, add_rn(za, zb));
+        return fma(-dtau, fma(cx, dx, fma(-cy, dy, fma(-cz, dz, mul_rn(c, h)))), c);
+    };
+    return C{step(c0.x, xm.x, xp.x, ym.x, yp.x, zm.x, zp.x), step(c0.y, xm.y, xp.y, ym.y, yp.y, zm.y, zp.y)};
 }
 
 // A psi of norm d that is still to be divided by sqrt(d) enters rho as psi 2^-h: |psi|^2 N
@@ -462,8 +480,8 @@ __device__ __forceinline__ void g_tiles(const GPlan &pk, unsigned &K, unsigned &
 
 template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 3 : 2) g_z(const __grid_constant__ GZArgs g) {
     using C            = cplx<R>;
-    constexpr bool RT  = MODE <= GZ_RT_EPI || MODE == GZ_PHASE;
-    constexpr bool IT  = MODE == GZ_IT_MID || MODE == GZ_IT_STEP;
+    constexpr bool RT  = MODE <= GZ_RT_EPI;
+    constexpr bool IT  = MODE == GZ_IT_MID;
     constexpr bool KIN_I = MODE == GZ_RT_MID || MODE == GZ_RT_EPI || MODE == GZ_KIN_INV;
     constexpr bool KIN_F = MODE == GZ_RT_PRO || MODE == GZ_RT_MID || MODE == GZ_KIN_FWD;
     constexpr bool DIP_I = MODE == GZ_RT_MID || MODE == GZ_RT_EPI || MODE == GZ_IT_MID || MODE == GZ_DIP_INV;
@@ -570,7 +588,7 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
                     break;
                 const int q = row * nz + k;
                 R f         = h == 0 ? z.y : z.x;
-                if (MODE == GZ_RT_PRO || MODE == GZ_PHASE || MODE == GZ_IT_STEP)
+                if (MODE == GZ_RT_PRO)
                     f = phi[q];
                 if (MODE == GZ_DIP_INV || MODE == GZ_RT_EPI || (MODE == GZ_IT_MID && g.write_phi))
                     phi[q] = f;
@@ -581,13 +599,13 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
                 const bool in = i >= 1 && i < nx - 1 && j >= 1 && j < ny - 1 && k >= 1 && k < nz - 1;
                 C v;
                 if (RT) {
-                    v = MODE == GZ_RT_PRO || MODE == GZ_PHASE ? psi[q] : g_swap(sm[K + k * TK + row], true);
+                    v = MODE == GZ_RT_PRO ? psi[q] : g_swap(sm[K + k * TK + row], true);
                     if (in) {
                         v = g_turn<R>(v, V[q], f, cdd, hdt, g3, gw);
                         if (MODE == GZ_RT_MID) // the next iteration's first half step
                             v = g_turn<R>(v, V[q], f, cdd, hdt, g3n, gwn);
                     }
-                    if (MODE == GZ_RT_EPI || MODE == GZ_PHASE)
+                    if (MODE == GZ_RT_EPI)
                         out[q] = v;
                     else
                         sm[K + k * TK + row] = v;
@@ -600,23 +618,10 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
                     if (!in) {
                         v = reinterpret_cast<const C *>(a.bnd)[base + q];
                     } else {
-                        const C c0 = cscale(psi[q], sc);
-                        const C xm = cscale(psi[q - plane], sc), xp = cscale(psi[q + plane], sc);
-                        const C ym = cscale(psi[q - nz], sc), yp = cscale(psi[q + nz], sc);
-                        const C zm = cscale(psi[q - 1], sc), zp = cscale(psi[q + 1], sc);
-                        const R dens = g_abs2(c0), am = sqrt(dens);
-                        const R h    = add_rn(fma(cdd, f, V[q]), fma(g3, dens, mul_rn(gw, mul_rn(mul_rn(am, am), am))));
-                        auto step    = [&](R c, R xa, R xb, R ya, R yb, R za, R zb) {
-                            const R dx = fma((R)-2, c, add_rn(xa, xb)), dy = fma((R)-2, c, add_rn(ya, yb)),
-                                    dz = fma((R)-2, c, add_rn(za, zb));
-                            return fma(-dtau, fma(cx, dx, fma(-cy, dy, fma(-cz, dz, mul_rn(c, h)))), c);
-                        };
-                        v = C{step(c0.x, xm.x, xp.x, ym.x, yp.x, zm.x, zp.x),
-                              step(c0.y, xm.y, xp.y, ym.y, yp.y, zm.y, zp.y)};
+                        v = g_euler<R>(psi + q, plane, nz, sc, V[q], f, cdd, g3, gw, cx, cy, cz, dtau);
                     }
                     out[q] = v;
-                    if (MODE == GZ_IT_MID)
-                        acc = add_rn(acc, g_abs2(double2{(double)v.x, (double)v.y}));
+                    acc    = add_rn(acc, g_abs2(double2{(double)v.x, (double)v.y}));
                 }
                 rho[h] = mul_rn(wat, g_abs2(v));
             }
@@ -657,6 +662,48 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
     // ---- norm of psi' (imaginary time): deterministic two-level reduction --------
     if (MODE == GZ_IT_MID || MODE == GZ_NORM)
         norm_by_last_block(acc, a);
+}
+
+// ---------------------------------------------------------------------------
+// The interface's pointwise steps
+// ---------------------------------------------------------------------------
+// One potential half step of psi in place, phi in memory: a thread per point.  Bound by DRAM
+// on large grids, by the launch on small ones: 256 x 256 x 64 24.8 us, 4 x 4 x 1600 3.7 (6.4 as
+// a pass over rows, a CTA per 32 of them: long rows leave most SMs idle).
+template <class R>
+__global__ void __launch_bounds__(256)
+    g_half_step(cplx<R> *__restrict__ psi, const __grid_constant__ ZArgs a, int nz) {
+    const unsigned q = blockIdx.x * 256u + threadIdx.x, row = q / (unsigned)nz, i = row / (unsigned)a.ny;
+    const int j = (int)(row - i * a.ny), k = (int)(q - row * nz);
+    if (i < 1 || (int)i >= a.nx - 1 || j < 1 || j >= a.ny - 1 || k < 1 || k >= nz - 1)
+        return;
+    const StepCoef c = a.step.coef[0];
+    psi[q] = g_turn<R>(psi[q], reinterpret_cast<const R *>(a.V)[q], reinterpret_cast<const R *>(a.phi)[q], (R)a.cdd,
+                       (R)a.half_dt, (R)c.g3w, (R)c.gw15);
+}
+
+// The Euler step from psi / sqrt(divisor) into `out`, phi in memory; the boundary takes the
+// values last loaded.  Bound by DRAM on large grids.  Exactly the CTAs that are resident at once
+// (6 an SM, 5 in complex128) walk through the points together, so that a plane's neighbours
+// meet in the L2: 256 x 256 x 64 37.6 us, 47 with 8 an SM, 46 with a thread per point, 64 as a pass
+// over rows; complex128 49, 56, 68 and 82.
+template <class R> constexpr int g_euler_blocks() { return sizeof(R) == 4 ? 6 : 5; }
+template <class R>
+__global__ void __launch_bounds__(256, g_euler_blocks<R>())
+    g_euler_step(const cplx<R> *__restrict__ psi, cplx<R> *__restrict__ out, const cplx<R> *__restrict__ bnd,
+                 const R *__restrict__ V, const R *__restrict__ phi, const __grid_constant__ ZArgs a, int nz) {
+    const StepCoef c      = a.step.coef[0];
+    const R sc            = (R)(1.0 / sqrt(a.norm_state[1]));
+    const ptrdiff_t plane = (ptrdiff_t)a.ny * nz;
+    const unsigned n      = (unsigned)a.nx * a.ny * nz;
+    for (unsigned q = blockIdx.x * 256u + threadIdx.x; q < n; q += gridDim.x * 256u) {
+        const unsigned row = q / (unsigned)nz, i = row / (unsigned)a.ny;
+        const int j = (int)(row - i * a.ny), k = (int)(q - row * nz);
+        const bool in = i >= 1 && (int)i < a.nx - 1 && j >= 1 && j < a.ny - 1 && k >= 1 && k < nz - 1;
+        out[q] = in ? g_euler<R>(psi + q, plane, nz, sc, V[q], phi[q], (R)a.cdd, (R)c.g3w, (R)c.gw15, (R)a.cx,
+                                 (R)a.cy, (R)a.cz, (R)a.dtau)
+                    : bnd[q];
+    }
 }
 
 } // namespace gpe

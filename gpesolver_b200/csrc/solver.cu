@@ -176,7 +176,6 @@ template <class R> class Solver final : public SolverBase {
         staging.alloc(2 * N);
         norm_state.alloc(4);
         status.alloc(4);
-        iter_zero.alloc(1);
         iter_base.alloc(1);
         cur_coef.alloc(1);
         eout.alloc(8);
@@ -393,7 +392,7 @@ template <class R> class Solver final : public SolverBase {
 
     // cpu_solver.cpp:50-97, linear and nonlinear part fused: psi' of the interior from
     // psi / sqrt(divisor), the boundary takes the values last loaded
-    void imag_linear() override { gen_z<GZ_IT_STEP>(cur, psi.p, psii.p, cur_coef.p, 0, 0); }
+    void imag_linear() override { enqueue_euler(cur); }
 
     void imag_nonlinear() override {
         std::swap(psi.p, psii.p);
@@ -425,7 +424,7 @@ template <class R> class Solver final : public SolverBase {
 
     void potential_half_step() override {
         materialize();
-        gen_z<GZ_PHASE>(cur, psi.p, psi.p, cur_coef.p, 0, 0, iter_zero.p);
+        enqueue_half_step(cur);
     }
 
     void kinetic_step() override {
@@ -596,7 +595,7 @@ template <class R> class Solver final : public SolverBase {
                 b = 2 * F;
                 break;
             case GPE_K_PHASE:
-                gen_z<GZ_PHASE>(cur, psi.p, psi.p, cur_coef.p, 0, 0, iter_zero.p);
+                enqueue_half_step(cur);
                 b = 2 * F + 2 * Rb;
                 break;
             case GPE_K_F_X:
@@ -641,7 +640,7 @@ template <class R> class Solver final : public SolverBase {
                 break;
             }
             default:
-                gen_z<GZ_IT_STEP>(cur, psi.p, psii.p, cur_coef.p, 0, 0);
+                enqueue_euler(cur);
                 b = 2 * F + 2 * Rb;
                 break;
             }
@@ -1206,17 +1205,14 @@ template <class R> class Solver final : public SolverBase {
         });
     }
     template <int MODE>
-    void gen_z(cudaStream_t s, C *pin, C *pout, const StepCoef *coef, int local, int write_phi,
-               const int *base = nullptr) {
+    void gen_z(cudaStream_t s, C *pin, C *pout, const StepCoef *coef, int local, int write_phi) {
         GZArgs a{};
         a.z = zargs(pin, pout, coef, local);
-        if (base)
-            a.z.step.base = base;
         a.write_phi = write_phi;
         a.nz = nz, a.mz = g_magic(nz), a.lb = shape.lbz, a.buf = shape.buf;
         a.k = kz.plan, a.d = dz.plan;
-        // the single steps without a transform take no tile
-        constexpr bool tile = MODE < GZ_PHASE;
+        // the norm takes no tile
+        constexpr bool tile = MODE != GZ_NORM;
         launch(g_z<R, MODE>, (nx * ny + (1 << a.lb) - 1) >> a.lb, shape.ntz, tile ? shape.smz : 0, s, a);
     }
     void capture_general(int kind, int count) {
@@ -1364,7 +1360,7 @@ template <class R> class Solver final : public SolverBase {
     MappedBuf<double> ehist;   // energy history of imag_steps_energies
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t ev_widened = nullptr, ev_copied = nullptr;
-    DevBuf<int> iter_zero, iter_base;
+    DevBuf<int> iter_base;
     MappedBuf<int> status;
     // fused pipeline (compile-time line lengths; complex64 only)
     bool fused = false;
@@ -1562,6 +1558,16 @@ template <class R> class Solver final : public SolverBase {
         gen_x(s, false, true, norm_state.p + 1, 1.0 / (8.0 * (double)N));
         gen_y(s, true, false, true);
         gen_z<GZ_DIP_INV>(s, p, p, cur_coef.p, 0, 1);
+    }
+
+    void enqueue_half_step(cudaStream_t s) {
+        launch(g_half_step<R>, (int)((N + 255) / 256), 256, 0, s, psi.p, zargs(psi.p, psi.p, cur_coef.p, 0), nz);
+    }
+
+    void enqueue_euler(cudaStream_t s) {
+        const size_t most = 148 * g_euler_blocks<R>();
+        launch(g_euler_step<R>, (int)std::min<size_t>((N + 255) / 256, most), 256, 0, s, (const C *)psi.p, psii.p,
+               (const C *)bnd.p, (const R *)V.p, (const R *)phi.p, zargs(psi.p, psii.p, cur_coef.p, 0), nz);
     }
 
     void enqueue_kinetic(cudaStream_t s) {
@@ -2106,7 +2112,7 @@ int gpe_time_kernel(gpe_handle *h, int which, int reps, double *ms, double *byte
 const char *gpe_kernel_name(int which) {
     static const char *names[] = {"g_z", "g_y", "g_x", "g_y", "g_z",
                                   "g_z", "g_y", "g_x", "g_y", "g_z",
-                                  "g_z", "g_z", "k3_x", "k3_y", "k2_z", "k3_y",
+                                  "g_half_step", "g_euler_step", "k3_x", "k3_y", "k2_z", "k3_y",
                                   "k3_x_kin", "k3_x_dip", "k4_yz"};
     if (which < 0 || which >= GPE_K_COUNT)
         return "";
