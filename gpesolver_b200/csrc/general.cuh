@@ -380,12 +380,11 @@ enum {
     GZ_IT_MID,     // dipolar inverse, Euler step and norm, forward
     GZ_DIP_INV,    // spectrum -> phi
     GZ_KIN_FWD, GZ_KIN_INV,
-    GZ_NORM,       // the norm alone
     GZ_MODES
 };
-// The interface's single steps (GZ_DIP_INV and after, g_half_step, g_euler_step) run the
-// iterations' arithmetic, the norm on their rows too, so both sequences agree to the last
-// bits.
+// The interface's single steps (GZ_DIP_INV and after, g_half_step, g_euler_step, g_norm) run
+// the iterations' arithmetic, the norm in their order too, so both sequences agree to the
+// last bits.
 
 // The pointwise arithmetic with its roundings written out: the compiler then contracts
 // it alike in every kernel.
@@ -611,9 +610,6 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
                         sm[K + k * TK + row] = v;
                 } else if (MODE == GZ_IT_PRO) {
                     v = cscale(psi[q], fold);
-                } else if (MODE == GZ_NORM) {
-                    v = psi[q];
-                    acc = add_rn(acc, g_abs2(double2{(double)v.x, (double)v.y}));
                 } else { // the Euler step of psi_in / sqrt(divisor)
                     if (!in) {
                         v = reinterpret_cast<const C *>(a.bnd)[base + q];
@@ -628,15 +624,14 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
             if (DIP_F)
                 sm[D + k * TD + p] = C{rho[0], rho[1]};
         }
-        if (!DIP_F && MODE != GZ_NORM)
+        if (!DIP_F)
             return;
         if (KIN_F) // rows beyond the grid's last
             for (int e = cnt * nz + tid; e < RW * nz; e += nt) {
                 const int row = g_div(e, nz, g.mz), k = e - row * nz;
                 sm[K + k * TK + row] = C{(R)0, (R)0};
             }
-        if (MODE != GZ_NORM)
-            __syncthreads();
+        __syncthreads();
     }
 
     // ---- out: kinetic spectrum, then bins 1..nz of the row pairs -----------------
@@ -660,7 +655,7 @@ template <class R, int MODE> __global__ void __launch_bounds__(256, sizeof(R) ==
     }
 
     // ---- norm of psi' (imaginary time): deterministic two-level reduction --------
-    if (MODE == GZ_IT_MID || MODE == GZ_NORM)
+    if (MODE == GZ_IT_MID)
         norm_by_last_block(acc, a);
 }
 
@@ -703,6 +698,50 @@ __global__ void __launch_bounds__(256, g_euler_blocks<R>())
         out[q] = in ? g_euler<R>(psi + q, plane, nz, sc, V[q], phi[q], (R)a.cdd, (R)c.g3w, (R)c.gw15, (R)a.cx,
                                  (R)a.cy, (R)a.cz, (R)a.dtau)
                     : bnd[q];
+    }
+}
+
+// The norm of psi, summed in the order of g_z's imaginary-time step (parts of 2^lb rows, row
+// pairs, the same threads).  Bound by DRAM, and by the parts' sums where they are small; so a
+// resident CTA takes several parts and one fence and ticket for all of them: 300 x 300 x 100
+// 22.1 us, 512 x 512 x 8 16.6 (27.1 and 31.0 with a CTA and a ticket per part).
+template <class R> constexpr int g_norm_blocks() { return sizeof(R) == 4 ? 6 : 5; }
+template <class R>
+__global__ void __launch_bounds__(256, g_norm_blocks<R>())
+    g_norm(const cplx<R> *__restrict__ psi, const __grid_constant__ ZArgs a, int nz, unsigned mz, int lb) {
+    using C         = cplx<R>;
+    constexpr int U = 2; // pairs of loads in flight
+    __shared__ double red[2][32];
+    const int nt = blockDim.x, rows = a.nx * a.ny, parts = (rows + (1 << lb) - 1) >> lb;
+    const int dp = g_div(nt, nz, mz), dk = nt - dp * nz; // items nt apart: row pairs, elements
+    const int p0 = g_div(threadIdx.x, nz, mz);
+    for (int part = blockIdx.x, odd = 0;; part += gridDim.x, odd ^= 1) {
+        const int r0 = part << lb, cnt = min(1 << lb, rows - r0), n = ((cnt + 1) >> 1) * nz;
+        const C *src = psi + (size_t)r0 * nz;
+        double acc   = 0.0;
+        int p = p0, k = threadIdx.x - p0 * nz; // row 2p and 2p + 1, element k
+        while (p * nz + k < n) {
+            C v[U][2];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const C *x = src + 2 * p * nz + k;
+                v[u][0]    = 2 * p < cnt ? x[0] : C{(R)0, (R)0};
+                v[u][1]    = 2 * p + 1 < cnt ? x[nz] : C{(R)0, (R)0};
+                p += dp, k += dk;
+                if (k >= nz)
+                    k -= nz, ++p;
+            }
+#pragma unroll
+            for (int u = 0; u < 2 * U; ++u) // (zeros change nothing)
+                acc = add_rn(acc, g_abs2(double2{(double)v[u >> 1][u & 1].x, (double)v[u >> 1][u & 1].y}));
+        }
+        if (part + (int)gridDim.x >= parts) {
+            norm_by_last_block(acc, a, part, parts);
+            return;
+        }
+        const double sum = block_sum(acc, red[odd]);
+        if (threadIdx.x == 0)
+            a.partial[part] = sum;
     }
 }
 

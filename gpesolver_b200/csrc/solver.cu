@@ -247,7 +247,7 @@ template <class R> class Solver final : public SolverBase {
         GPE_CUDA(cudaMemcpyAsync(psii.p, psi.p, sizeof(C) * N, cudaMemcpyDeviceToDevice, cur));
         GPE_CUDA(cudaMemcpyAsync(bnd.p, psi.p, sizeof(C) * N, cudaMemcpyDeviceToDevice, cur));
         // calc_norm + normalize: the normalisation is held as the lazy divisor.
-        gen_z<GZ_NORM>(cur, psi.p, psi.p, cur_coef.p, 0, 0);
+        enqueue_norm(cur);
         lazy = true;
         check_status();
     }
@@ -405,7 +405,7 @@ template <class R> class Solver final : public SolverBase {
     // and load_psi report them.
     double calc_norm(bool to_host) override {
         materialize();
-        gen_z<GZ_NORM>(cur, psi.p, psi.p, cur_coef.p, 0, 0);
+        enqueue_norm(cur);
         set_divisor_one();
         if (!to_host)
             return 0.0;
@@ -1211,9 +1211,7 @@ template <class R> class Solver final : public SolverBase {
         a.write_phi = write_phi;
         a.nz = nz, a.mz = g_magic(nz), a.lb = shape.lbz, a.buf = shape.buf;
         a.k = kz.plan, a.d = dz.plan;
-        // the norm takes no tile
-        constexpr bool tile = MODE != GZ_NORM;
-        launch(g_z<R, MODE>, (nx * ny + (1 << a.lb) - 1) >> a.lb, shape.ntz, tile ? shape.smz : 0, s, a);
+        launch(g_z<R, MODE>, (nx * ny + (1 << a.lb) - 1) >> a.lb, shape.ntz, shape.smz, s, a);
     }
     void capture_general(int kind, int count) {
         cudaStream_t s      = cap_stream;
@@ -1558,6 +1556,12 @@ template <class R> class Solver final : public SolverBase {
         gen_x(s, false, true, norm_state.p + 1, 1.0 / (8.0 * (double)N));
         gen_y(s, true, false, true);
         gen_z<GZ_DIP_INV>(s, p, p, cur_coef.p, 0, 1);
+    }
+
+    void enqueue_norm(cudaStream_t s) {
+        const int parts = (nx * ny + (1 << shape.lbz) - 1) >> shape.lbz;
+        launch(g_norm<R>, std::min(parts, 148 * g_norm_blocks<R>() * (256 / shape.ntz)), shape.ntz, 0, s,
+               (const C *)psi.p, zargs(psi.p, psi.p, cur_coef.p, 0), nz, g_magic(nz), shape.lbz);
     }
 
     void enqueue_half_step(cudaStream_t s) {

@@ -46,3 +46,21 @@ def test_steps_match_numpy(dims, prec, tol):
         want = want + sign * (-0.5 if axis == 0 else 0.5) / (p.m * d * d) * lap
     want = np.where(inside, psi - p.imag_time_dt * want, psi)
     assert rel_l2(euler, want) < tol
+
+
+@pytest.mark.parametrize("prec", ["c128", "c64"])
+@pytest.mark.parametrize("dims", [(3, 3, 3), (1, 1, 1), (5, 7, 3), (4, 3, 1600), (300, 12, 8), (96, 90, 50), (384, 384, 9)])
+def test_norm_matches_numpy(dims, prec):
+    """Sums of squares in FP64 over parts of rows: 1e-13 from numpy's, on psi as the precision holds it; the
+    last grid has several parts per CTA.  The same to the bit when asked again."""
+    p = gparams(O.default_config(nx=dims[0], ny=dims[1], nz=dims[2]))
+    rng = np.random.default_rng(sum(dims))
+    psi = rng.normal(size=dims) + 1j * rng.normal(size=dims)
+    if prec == "c64":
+        psi = psi.astype(np.complex64).astype(np.complex128)
+    with G.B200GrossPitaevskiSolver(p, precision=prec, schedule="split") as s:
+        s.import_data(psi)
+        got = [s.calc_norm() for _ in range(3)]
+    want = (np.abs(psi) ** 2).sum() * p.dx * p.dy * p.dz
+    assert abs(got[0] - want) < 1e-13 * want
+    assert got[1:] == got[:1] * 2
