@@ -9,7 +9,7 @@
 // first stage, inputs brought in by cp.async behind the transforms, twiddles staged in
 // shared memory.
 //
-// Bound by instruction issue, then DRAM (235 MB an iteration at 256 x 256 x 64, 36
+// Bound by instruction issue, then DRAM (218 MB an iteration at 256 x 256 x 64, 33
 // us).  With a pass of its own over the tiles for the pair lines, phi, the phase and rho, and
 // every bin of the spectrum read twice, it executed 472 instructions a point there: 90 us.
 #pragma once

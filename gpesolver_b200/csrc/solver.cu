@@ -634,8 +634,9 @@ template <class R> class Solver final : public SolverBase {
                     b = 2 * F + S2h + S2b;
                 } else {
                     f_z<ZM_RT_MID>(cur, psi.p, psi.p, coef_dev.p, 0);
-                    // increment R+W, real-space psi R+W, spectrum R+W, V read, phi write
-                    b = 4 * F + 2 * S2h + Rb + Rb;
+                    // increment R+W, real-space psi R+W, spectrum R+W, V read (phi is
+                    // written only by the last iteration of a call)
+                    b = 4 * F + 2 * S2h + Rb;
                 }
                 break;
             }
