@@ -10,10 +10,11 @@
 // else is allocated, on the device or in pinned host memory.
 //
 // Limits and sharing:
-//  * scratch holds the pruned dipolar spectrum (nx * 2ny * (nz+1) complex64),
-//    the V_dd(k) table ((nx+1) * (ny+1) * (nz+1) floats) and three twiddle
-//    tables with their rounding remainders; grids needing more than GPE_NOALLOC_SCRATCH_BYTES are rejected
-//    with GPE_ERR_SIZE (128 x 128 x 32 needs about 10.9 MB);
+//  * scratch holds the pruned dipolar spectrum (nx * 2ny * nz complex64, room for
+//    nz+1 bins), the V_dd(k) table ((nx+1) * (ny+1) * nz floats, likewise) and three
+//    twiddle tables with their rounding remainders; grids whose room exceeds
+//    GPE_NOALLOC_SCRATCH_BYTES are rejected with GPE_ERR_SIZE (128 x 128 x 32 takes about
+//    10.9 MB).  The kz = 0 bin is not stored; its room keeps the limit where callers know it;
 //   * the array lives on every GPU that loads the library until the process
 //    exits, and every call on a GPU shares it: calls that overlap on that GPU
 //    (other streams, other threads) race.  Every call rebuilds the twiddle and
@@ -83,12 +84,12 @@ __global__ void k_na_tables(float4 *twx, float4 *twy, float4 *twz, float *vk, in
 
 struct Layout {
     size_t a_off, vk_off, twx_off, twy_off, twz_off, total;
-    // each twiddle region holds the table followed by its remainder table
+    // twiddle regions: (hi, lo) pairs
 };
 
 Layout layout(int nx, int ny, int nz) {
     Layout l{};
-    const int H = nz + 1;
+    const int H = nz + 1; // the limit's count of bins, one more than is stored
     size_t off = 0;
     l.a_off    = off;
     off += align256(sizeof(float2) * (size_t)nx * 2 * ny * H);
@@ -102,13 +103,6 @@ Layout layout(int nx, int ny, int nz) {
     off += align256(sizeof(float2) * 2 * 2 * (size_t)nz);
     l.total = off;
     return l;
-}
-
-int tile_for(int L, int pad) {
-    int TB = 32;
-    while (TB > 1 && 2 * sizeof(float2) * (size_t)(TB + pad) * L > 64 * 1024)
-        TB >>= 1;
-    return TB;
 }
 
 int fail(int code, const std::string &msg) {
@@ -153,11 +147,6 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
     if (dev < 0 || dev >= kMaxDevices)
         return fail(GPE_ERR_ARG, "gpe_calc_fi3d_noalloc: device ordinal out of range");
     cudaStream_t s = (cudaStream_t)cuda_stream;
-    const int TBx = tile_for(lx.L, 0), TBy = tile_for(ly.L, 0), TBz = tile_for(lz.L, 1);
-    // the limits on line lengths
-    const size_t smx = 2 * sizeof(float2) * (size_t)TBx * lx.L;
-    const size_t smy = 2 * sizeof(float2) * (size_t)TBy * ly.L;
-    const size_t smz = 2 * sizeof(float2) * (size_t)(TBz + 1) * lz.L; // z tiles: odd stride TB + 1
 
     NoallocSlot &slot = g_noalloc_slots[dev];
     {
@@ -176,6 +165,7 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
             const void *kern[] = {(const void *)g_z<float, GZ_IT_PRO>, (const void *)g_z<float, GZ_DIP_INV>,
                                   (const void *)g_y<float, 2>, (const void *)g_y<float, 3>,
                                   (const void *)g_x<float, 2>, (const void *)g_x<float, 3>};
+            int fixed = 0; // the most that a kernel holds statically
             for (const void *f : kern) {
                 cudaFuncAttributes fa{};
                 err = cudaFuncGetAttributes(&fa, f);
@@ -184,14 +174,14 @@ extern "C" int gpe_calc_fi3d_noalloc(const void *psi_c64_dev, float *fi3d_dev, i
                                                optin - (int)fa.sharedSizeBytes);
                 if (err != cudaSuccess)
                     return fail(GPE_ERR_CUDA, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(err));
+                fixed = std::max(fixed, (int)fa.sharedSizeBytes);
             }
             slot.base     = static_cast<unsigned char *>(p);
-            slot.smem_max = (size_t)optin;
+            slot.smem_max = (size_t)(optin - fixed);
             slot.ready    = true;
         }
     }
-    const size_t most = std::max({smx, smy, smz, sh.smx, sh.smy, sh.smz});
-    if (most > slot.smem_max)
+    if (std::max({sh.smx, sh.smy, sh.smz}) > slot.smem_max)
         return fail(GPE_ERR_SIZE, "gpe_calc_fi3d_noalloc: the line tiles of this grid need more shared memory "
                                   "than the device allows per block");
     // An error left by earlier, unrelated work would be reported as this call's:
