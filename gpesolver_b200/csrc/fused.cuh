@@ -30,16 +30,6 @@
 
 namespace gpe {
 
-// Tile widths (lines per CTA) for a pass of line length L in precision R:
-// CNT*L complex within 32 KiB (one in-place tile buffer per CTA).
-template <class R, int L> constexpr int tile_lines() {
-    int c = (int)(32768 / (int)sizeof(cplx<R>) / L);
-    int p = 1;
-    while (p * 2 <= c && p * 2 <= 32)
-        p *= 2;
-    return p;
-}
-
 struct Twid {
     const void *tw;
     const void *lo;

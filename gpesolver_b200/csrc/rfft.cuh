@@ -153,7 +153,7 @@ struct LinePass {
     template <int S>
     static __device__ __forceinline__ void middle(C *buf, const C *tw, const C *twlo, int tid) {
         if constexpr (S < NSTG - 1) {
-            ct_stage_ip<SIGN, R, L, RAD.r[S], ns_before(S), COUNT, TS, NT, CMP, false, false>(buf, tw, twlo, tid);
+            ct_stage_ip<SIGN, R, L, RAD.r[S], ns_before(S), COUNT, TS, NT, CMP>(buf, tw, twlo, tid);
             middle<S + 1>(buf, tw, twlo, tid);
         }
     }
