@@ -267,16 +267,13 @@ __device__ __forceinline__ void g_xmid_r(const GXArgs &a, const GPlan &pl, bool 
             const C *ex = reinterpret_cast<const C *>(a.ex);
             const C wy = __ldg(reinterpret_cast<const C *>(a.ey) + y), wz = __ldg(reinterpret_cast<const C *>(a.ez) + z);
             const C wyz = cadd(cadd(wy, wz), cmul(wy, wz)); // (1+wy)(1+wz) - 1
-            const R ih = (R)a.inv, il = (R)(a.inv - (double)ih); // 1/N, and its rounding in complex64
+            const R ih  = (R)a.inv;
 #pragma unroll
             for (int q = 0; q < RAD; ++q) {
                 const C wx = __ldg(&ex[j + q * st.nr]);
                 const C w  = cadd(cadd(wx, wyz), cmul(wx, wyz)); // exp(i theta) - 1
                 const C u  = sizeof(R) == 4 ? cmul(v[q], w) : apply_wm1(v[q], w);
-                if constexpr (sizeof(R) == 4)
-                    v[q] = C{fma(u.y, ih, u.y * il), fma(u.x, ih, u.x * il)}; // swapped: inverse
-                else
-                    v[q] = C{u.y * ih, u.x * ih};
+                v[q]       = C{u.y * ih, u.x * ih}; // swapped: inverse
             }
         } else {
             const int iy = y <= a.ny ? y : 2 * a.ny - y;
