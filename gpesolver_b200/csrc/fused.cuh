@@ -247,12 +247,14 @@ __global__ void __launch_bounds__(NT, NX >= 256 ? 2 : 3) // 512-point lines: two
 // Dipolar x pencils of 2nx = 512 points as two transforms of nx = 256 each: the even
 // bins are FFT_nx(S), the odd ones FFT_nx(S w^x), w = exp(-2 pi i / 2nx), and the kept
 // half of the inverse is iFFT_nx(even) + w^-x iFFT_nx(odd).  256 points are two stages of
-// radix 16 where 512 were three of radix 8 (a third fewer trips through shared memory
-// and synchronisations, no arithmetic on the padding), and one butterfly a thread
-// needs 32 registers for its points instead of 64.  A tile holds CNT even and CNT odd lines; both
-// of a column lie in one warp, read the same addresses and are added by a shuffle.
+// radix 16 where 512 were three of radix 8: fewer synchronisations, and one butterfly a
+// thread needs 32 registers for its points instead of 64.  The instructions stay (46.4 ->
+// 46.1 M): the second half's twiddles and the sums take what the third stage gave back.  A
+// tile holds CNT even and CNT odd lines; both of a column lie in one warp, read the same
+// addresses and are added by a shuffle.
 // Bound by instruction issue (62%).  256 x 256 x 64: 79 -> 72 us, the iteration 253 ->
-// 248 us against k3_x_dip with 8 lines, 267 against its 16 (spilled).
+// 248 us (2%) against k3_x_dip with 8 lines, 267 against its 16 (spilled).  16 lines spill here
+// too (248 bytes); the autotuner times both widths.
 template <class R, int NX, int CNT> constexpr size_t x_dip_eo_smem() {
     return sizeof(cplx<R>) * (2 * CNT * NX + 3 * NX) + sizeof(R) * (NX + 1) * CNT;
 }

@@ -20,16 +20,16 @@
 // kz^2/k^2, zero on the kz = 0 plane, which is not stored
 // (fftw_poisson_solver.cpp:39-45).
 //
-// A line transform is two (up to 256 points), three or more Stockham stages of
-// radix <= 16 between two shared-memory buffers; the first stage of a line along x or y
-// reads global memory and the last one stores there, so a two-stage transform crosses shared
-// memory once.  All transforms run forward: an inverse one swaps re and im at both ends.
+// A line transform is as few Stockham stages of radix <= 16 as its factors allow (two for
+// most lengths up to 256, three for 125, 200, 216, 250 and the like) between two shared-memory
+// buffers; the first stage of a line along x or y reads global memory and the last one stores
+// there, so a two-stage transform crosses shared memory once.  All transforms run forward: an inverse one swaps re and im at both ends.
 // Twiddles are those of plan.hpp, in complex64 hi + lo (compensated).
 //
 // Bound by the chain of dependent instructions on small grids (one or two warps per
 // scheduler; 30 x 20 x 12: 20 us an iteration, 5 a launch), by instruction issue on large ones
 // (100 x 90 x 30: 44-54% of the slots).  Real time, us an iteration, one kernel per
-// axis pass -> now: 100 x 90 x 30 149 -> 45; complex128 128 x 128 x 32 220 -> 80; imaginary
+// axis pass -> now: 100 x 90 x 30 145 -> 46; complex128 128 x 128 x 32 213 -> 80; imaginary
 // time, complex128 64 x 64 x 16: 37 -> 28.
 #pragma once
 
@@ -160,8 +160,8 @@ __device__ __forceinline__ void g_last_r(const GStage &st, const void *tw, cplx<
     }
 }
 
-// Whole transform of the columns p -> p.  buf: two tiles of `ts` elements each at
-// 0 and ts; the second one only for three stages and more.
+// Whole transform of the columns p -> p, with tiles at elements 0 and L << lb of shared
+// memory; the second one only for three stages and more.
 template <class R>
 __device__ __forceinline__ void g_lines(const GPlan &pl, cplx<R> *p, size_t rs, int nin, int nout, int cnt, bool swap,
                                         int lb, int tid, int nt) {
@@ -267,7 +267,7 @@ __device__ __forceinline__ void g_xmid_r(const GXArgs &a, const GPlan &pl, bool 
             const C *ex = reinterpret_cast<const C *>(a.ex);
             const C wy = __ldg(reinterpret_cast<const C *>(a.ey) + y), wz = __ldg(reinterpret_cast<const C *>(a.ez) + z);
             const C wyz = cadd(cadd(wy, wz), cmul(wy, wz)); // (1+wy)(1+wz) - 1
-            const R ih  = (R)a.inv;
+            const R ih  = (R)a.inv; // one word: a common factor of up to 6e-8 on the increment alone
 #pragma unroll
             for (int q = 0; q < RAD; ++q) {
                 const C wx = __ldg(&ex[j + q * st.nr]);

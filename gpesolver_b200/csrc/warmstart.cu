@@ -249,7 +249,7 @@ __global__ void k_fold(const __nv_bfloat16 *__restrict__ wb, float *__restrict__
 // channels over KS groups of 128 threads, summed in order through shared memory: there a
 // thread's chain of loads is the time.  pre may be null (prediction).
 // Measured: 32 -> 32 channels to 16 x 16 x 4, 1 sample, 190 -> 18 (KS = 1) -> 8.8 us; 8 -> 8 to
-// 128 x 128 x 32, 8 samples, 747 -> 195 us.
+// 128 x 128 x 32, 8 samples, 747 -> 176 us.
 template <int OT, int VX, int KS>
 __global__ void __launch_bounds__(128 * KS)
     k_up_fwd(const float *__restrict__ in, const float *__restrict__ fwd, const __nv_bfloat16 *__restrict__ bias,
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(128 * KS)
 
 // The last convolution (cin -> 1, no upsampling, linear).  One thread: 4 voxels
 // along x, whose windows share their loads (L1); lanes take neighbouring (y, z)
-// columns.  Bound by the L1 reads (54 per 108 multiply-adds): 448 -> 182 us at 8
+// columns.  Bound by the L1 reads (54 per 108 multiply-adds): 448 -> 145 us at 8
 // channels, 128 x 128 x 32, 8 samples (one voxel a thread, staged tiles, before).
 __global__ void __launch_bounds__(128, 8)
     k_last_fwd(const float *__restrict__ in, const __nv_bfloat16 *__restrict__ W,
@@ -406,7 +406,7 @@ __global__ void __launch_bounds__(128, 8)
 // u values in 32 banks.  Two halves of the warps split a tile's rows and are
 // added in shared memory at the end.
 // Measured at 8 -> 8 channels, 128 x 128 x 32, 8 samples: 30.8 ms (one thread per
-// tap over 2048 voxels) -> 390 us.
+// tap over 2048 voxels) -> 212 us.
 constexpr int kWgVox = 128; // coarse voxels per tile, at most
 
 struct WgTile {
@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(64 * OT * up_reduce_slices<OT>())
 // Lanes take neighbouring (y, z) columns and walk along x over a segment of sx
 // planes, holding the 3 x 9 window of one input channel (blockIdx.y) and the 27
 // sums in registers: 9 loads (L1) and 27 multiply-adds per voxel.  The block's
-// sums meet in shared memory.  8 channels, 128 x 128 x 32, 8 samples: 4.2 ms -> 250 us.
+// sums meet in shared memory.  8 channels, 128 x 128 x 32, 8 samples: 4.2 ms -> 143 us.
 //  blockIdx.x = column block x segment, z = sample.
 __global__ void __launch_bounds__(256, 3)
     k_last_wgrad(const float *__restrict__ in, const float *__restrict__ gy, float *__restrict__ partial,
@@ -711,7 +711,7 @@ __global__ void __launch_bounds__(256)
 // Bound by FP32 issue and the shared-memory weight reads (VX = 2 halves them);
 // small volumes take CT = 2, VX = 1 so that the layer fills the SMs, the smallest with
 // the output channels over KS groups of 128 threads.  8 -> 8
-// channels at 128 x 128 x 32, 8 samples: 1086 + 2 x 70 (SiLU' pass) -> 200 us.
+// channels at 128 x 128 x 32, 8 samples: 1086 + 2 x 70 (SiLU' pass) -> 170 us.
 template <int CT, int VX, int KS>
 __global__ void __launch_bounds__(128 * KS)
     k_up_xgrad(const float *__restrict__ gy, const float *__restrict__ bwd, const float *__restrict__ pre_in,
